@@ -84,12 +84,12 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restri
     const int tab_f4 = LUT_SMEM ? (bins + 1) / 2 : 0;
     unsigned char *s_state = reinterpret_cast<unsigned char *>(smem4 + tab_f4);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t q = lane / G, j = lane % G;
+    const uint32_t q = Lanes<G>::chain_of(lane), j = Lanes<G>::lane_of(lane);
     constexpr int CPW = 32 / G;
     using Lay = Layout<G, SPL>;
     unsigned char *wb = s_state + (size_t)warp * Lay::WARP_BYTES;
     float *s_len = reinterpret_cast<float *>(s_state + (size_t)(blockDim.x >> 5) * Lay::WARP_BYTES);
-    const Planes st{reinterpret_cast<float2 *>(wb), reinterpret_cast<float *>(wb + Lay::XY_BYTES), s_len};
+    const Planes st{reinterpret_cast<float *>(wb), s_len};
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
         __syncthreads();
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restri
         ma.lin = e.lin;
         const uint32_t chain = it.y + warp * CPW + q;
         chain_body<G, SPL, EXACT, CLAMP, false, kModeForward, false, STEEP, !LUT_SMEM>(e.spec, e.kc, e.init_seg, tab, st,
-                                                                                       q * G, j,
+                                                                                       Lanes<G>::base_of(lane), j,
                                                                             chain, chain < e.spec.n_chains,
                                                                             out + e.out_offset, ma);
         __syncthreads();
@@ -132,12 +132,12 @@ __global__ void __launch_bounds__(MAXT, 1) batch_adjoint_kernel(const BatchExp *
     const int tab_f4 = (bins + 1) / 2;
     unsigned char *s_state = reinterpret_cast<unsigned char *>(smem4 + tab_f4);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t q = lane / G, j = lane % G;
+    const uint32_t q = Lanes<G>::chain_of(lane), j = Lanes<G>::lane_of(lane);
     constexpr int CPW = 32 / G;
     using Lay = Layout<G, SPL>;
     unsigned char *wb = s_state + (size_t)warp * Lay::WARP_BYTES;
     float *s_len = reinterpret_cast<float *>(s_state + (size_t)(blockDim.x >> 5) * Lay::WARP_BYTES);
-    const Planes st{reinterpret_cast<float2 *>(wb), reinterpret_cast<float *>(wb + Lay::XY_BYTES), s_len};
+    const Planes st{reinterpret_cast<float *>(wb), s_len};
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
         __syncthreads();
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(MAXT, 1) batch_adjoint_kernel(const BatchExp *
         ma.grad = grad + (size_t)e.out_offset * 6;
         const uint32_t chain = it.y + warp * CPW + q;
         chain_body<G, SPL, true, true, false, kModeAdjoint>(e.spec, e.kc, e.init_seg,
-                                                            reinterpret_cast<const float2 *>(smem4), st, q * G, j,
+                                                            reinterpret_cast<const float2 *>(smem4), st, Lanes<G>::base_of(lane), j,
                                                             chain, chain < e.spec.n_chains, nullptr, ma);
         __syncthreads();
     }

@@ -6,6 +6,34 @@
 namespace twisty {
 namespace {
 
+// The tangents of a path's points (lane j's segments), normalised here to length kscale.
+template <int SPL>
+struct PosLoad {
+    const float *pp;
+    uint32_t j, N;
+    float kscale;
+    __device__ __forceinline__ void one(int m, float &x, float &y, float &z) const
+    {
+        const uint32_t s = j * SPL + m;
+        x = y = z = 0.f;
+        if (s < N) {
+            x = pp[3 * s + 3] - pp[3 * s];
+            y = pp[3 * s + 4] - pp[3 * s + 1];
+            z = pp[3 * s + 5] - pp[3 * s + 2];
+            const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kscale;
+            x *= r; y *= r; z *= r;
+        }
+    }
+    __device__ __forceinline__ Tan2 pair(int h) const
+    {
+        constexpr int H = (SPL + 1) / 2;
+        float x0, y0, z0, x1 = 0.f, y1 = 0.f, z1 = 0.f;
+        one(h, x0, y0, z0);
+        if (h + H < SPL) one(h + H, x1, y1, z1);
+        return Tan2{pack2(x0, x1), pack2(y0, y1), pack2(z0, z1)};
+    }
+};
+
 // Compensated weigher of given paths: one group of 32 lanes per path; tangents from the
 // positions, normalised here.
 template <int SPL, bool EXACT>
@@ -19,27 +47,16 @@ __global__ void __launch_bounds__(256) weigh_comp_kernel(const float *__restrict
     const uint32_t j = threadIdx.x & 31;
     if (p >= n_paths) return;  // whole warps exit together
     const float *pp = pos + p * 3 * (uint64_t)(N + 1);
-    auto tan = [&](int m, float &x, float &y, float &z) {
-        const uint32_t s = j * SPL + m;
-        if (s < N) {
-            x = pp[3 * s + 3] - pp[3 * s];
-            y = pp[3 * s + 4] - pp[3 * s + 1];
-            z = pp[3 * s + 5] - pp[3 * s + 2];
-            const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kc.kscale;   // tangents at length kscale
-            x *= r; y *= r; z *= r;
-        } else {
-            x = y = z = 0.f;
-        }
-    };
+    const PosLoad<SPL> load{pp, j, N, kc.kscale};
     int32_t *brow = bins ? bins + p * (N - 1) : nullptr;
     auto sink = [&](uint32_t i, int32_t b) {
         if (brow) brow[i] = b;
     };
     uint32_t clamped = 0;
-    double w = path_log10<32, SPL, EXACT, true, true>(j, N, tab, kc, tan, ShflNext<32>{}, sink, clamped);
+    double w = path_log10<32, SPL, EXACT, true, true>(j, N, tab, kc, load, ShflNext<32>{}, sink, clamped);
     if (!EXACT && isnan(w)) {
         // a steep bin (NaN slope) or a NaN curvature: the exact blend through the linear table
-        w = path_log10<32, SPL, true, true, true>(j, N, lin, kc, tan, ShflNext<32>{}, sink, clamped);
+        w = path_log10<32, SPL, true, true, true>(j, N, lin, kc, load, ShflNext<32>{}, sink, clamped);
     }
     if (j == 0) {
         const bool ok = !isnan(w);
@@ -185,7 +202,7 @@ bool comp_table_needs_clamp(float inv_ds, const LutMetaF &m)
 // the cost per weighted step (both fitted to those runs), so they win once a pass's paths reach
 // about 58000 and 125000 times its burn-in steps per chain; the thresholds below round those up.
 // (At 2^24 paths and 256 burn-in steps: 1 x 16 +5 % at N = 16, 1 x 24 4-10 % slower.)
-// With unpadded one-lane rows (comp_pitch_xy), 1 x 16 at 24 warps carries 1.5x the chains of
+// With one-lane rows in their own banks (Layout), 1 x 16 at 24 warps carries 1.5x the chains of
 // 16 warps at 0.883 of the cost per step: +9.6 % at N = 16 on passes of 2^32 path-segments,
 // +4 % at 2^26 paths, 7 % slower at 2^24; it takes over at paths >= 210000 x burn-in.
 // 4 x 12, which also turns the shorter side, serves N = 37..48 with less padding than 4 x 16:

@@ -15,15 +15,14 @@
 //    (the chord is the axis and stays fixed) and leaves the lengths alone; each rotated
 //    tangent is renormalised by one Newton step, so |t_i| = 1 to an ulp and the full
 //    recompute needs no normalisation: kappa_i = |t_{i+1} - t_i| N/S.
-//  * Three planes per warp: (t.x, t.y) as float2, t.z, and l. Segment s = j*SPL + m of the
-//    chain in lanes q*G..q*G+G-1 sits in row m, column q*G + j of each plane; a lane's own
-//    segments are a base register plus immediate offsets, so a tangent is one 8-byte and
-//    one 4-byte LDS (12 bytes, the shared-memory bandwidth the full recompute needs; the
-//    full recompute reads consecutive columns of one row: conflict-free). Row pitches
-//    (32 + 16/SPL float2, 32 + G/SPL floats) shift successive rows by distinct banks so
-//    the k consecutive segments of a rotation fall in distinct banks (at most 2-way
-//    conflicts); one-lane shapes keep rows of 32 (comp_pitch_xy). The next lane's first
-//    tangent comes by shuffle.
+//  * What bounds the step at 8 and 16 lanes per chain is the shared-memory pipe (16 x 16 at
+//    N = 256: 90 % of its wavefronts, 83 % of the issue slots): 12 bytes per tangent
+//    of the full recompute and 8 per table gather, then the shuffles. So a proposal takes three
+//    shuffles (k and left in one word, sine and 1 - cosine ready), a chord's three sums travel
+//    together (group_sum3), and four paths' totals are summed together (batch_step): N = 256
+//    10.18 -> 9.55 ms per 2^25 paths. With 32 lanes the issue slots bind: those shapes keep pairs of
+//    segments and compute on them with the packed FP32 instructions (Layout, for_curvatures):
+//    N = 512 3.84 -> 3.40 ms per 2^23 paths.
 //  * Rotation: the chord is summed across the group (for full-warp groups as 32-bit fixed
 //    point with the warp reduction instruction, scaled by the chain's longest segment so
 //    that 64 segments cannot overflow; otherwise by float shuffles), normalised, and each
@@ -36,7 +35,7 @@
 //    the blend across the bin (secant): a segment costs one 8-byte LDS, one integer add
 //    (exact) and one FMA (the interpolation correction). Each lane rounds its correction
 //    sum to the same fixed point, the group adds the lanes' totals with integer shuffles
-//    (exact), and the chain's running log-sum-exp keeps its reference exponent as an
+//    (exact, four paths together), and the chain's running log-sum-exp keeps its reference exponent as an
 //    integer path total, so a path's weight relative to the running maximum is exp2 of an
 //    exact integer difference. The host scales the table so that N+1 entries stay below
 //    2^31; when that leaves fewer than 22 fraction bits, or the secant would lose more
@@ -117,23 +116,100 @@ __device__ __forceinline__ float ex2_approx(float x)
     return r;
 }
 
-template <int G>
-__device__ __forceinline__ void group_sum3(float &x, float &y, float &z)
+// Two floats in one 64-bit register: the packed FP32 instructions of sm_100 round each half as
+// the scalar instruction does and take one issue slot for two operations (measured: 1.95
+// packed FMAs per clock and SM against 3.8 scalar ones -- the same arithmetic rate from half
+// the issue slots, which the loads, conversions and integer work beside it then use).
+struct F2 {
+    uint64_t v;
+    __device__ __forceinline__ float lo() const { return __uint_as_float((uint32_t)v); }
+    __device__ __forceinline__ float hi() const { return __uint_as_float((uint32_t)(v >> 32)); }
+};
+
+__device__ __forceinline__ F2 pack2(float lo, float hi)
 {
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-        x += __shfl_xor_sync(FULL, x, o);
-        y += __shfl_xor_sync(FULL, y, o);
-        z += __shfl_xor_sync(FULL, z, o);
-    }
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
 }
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2_rd(F2 a, F2 b)   // rounded toward -infinity
+{
+    F2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, pack2(-1.0f, -1.0f), a); }   // a - b, exactly rounded
+
+// The lanes of a chain, from the chain's base lane qb. Lane j of it is lane qb + j; with 4 lanes per chain
+// lane qb + 8j, so that the chains sit side by side in a row of shared memory (Layout).
+template <int G>
+struct Lanes {
+    static constexpr int CPW = 32 / G;
+    static constexpr int STRIDE = G == 4 ? CPW : 1;   // from one lane of a chain to the next
+    static constexpr uint32_t MASK = G == 4 ? 0x01010101u : G == 32 ? FULL : (1u << (G & 31)) - 1u;   // ballot bits from qb on
+    __device__ __forceinline__ static uint32_t base_of(uint32_t lane) { return G == 4 ? lane % CPW : lane / G * G; }
+    __device__ __forceinline__ static uint32_t chain_of(uint32_t lane) { return G == 4 ? lane % CPW : lane / G; }
+    __device__ __forceinline__ static uint32_t lane_of(uint32_t lane) { return G == 4 ? lane / CPW : lane % G; }
+    // the value of the chain's lane j
+    template <class T>
+    __device__ __forceinline__ static T from(T v, uint32_t j, uint32_t qb)
+    {
+        return G == 4 ? __shfl_sync(FULL, v, j * CPW + qb) : __shfl_sync(FULL, v, j, G);
+    }
+};
 
 template <int G, class T>
 __device__ __forceinline__ T group_sum(T v)
 {
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(FULL, v, o * Lanes<G>::STRIDE);
     return v;
+}
+
+// The sums of three values over the chain's lanes, in every lane. From 8 lanes on the three
+// travel together: the first exchange takes x and y (each lane keeps one and sends the other),
+// the second adds z to them, the rest move one value each, and three broadcasts end it: 8
+// shuffles for 16 lanes instead of 12 (the shuffles share the shared-memory pipe that bounds
+// the step). The additions pair the same lanes in the same order as three butterflies do.
+template <int G>
+__device__ __forceinline__ void group_sum3(float &x, float &y, float &z, uint32_t j, uint32_t qb)
+{
+    constexpr int S = Lanes<G>::STRIDE;
+    if constexpr (G < 8) {
+        x = group_sum<G>(x);
+        y = group_sum<G>(y);
+        z = group_sum<G>(z);
+    } else {
+        const bool b0 = j & 1u, b1 = j & 2u;
+        float p = b0 ? y : x;
+        p += __shfl_xor_sync(FULL, b0 ? x : y, S);
+        z += __shfl_xor_sync(FULL, z, S);
+        float r = b1 ? z : p;
+        r += __shfl_xor_sync(FULL, b1 ? p : z, 2 * S);
+#pragma unroll
+        for (int o = 4; o < G; o <<= 1) r += __shfl_xor_sync(FULL, r, o * S);
+        x = Lanes<G>::from(r, 0, qb);
+        y = Lanes<G>::from(r, 1, qb);
+        z = Lanes<G>::from(r, 2, qb);
+    }
 }
 
 // TwoSum-combine the lanes' Kahan pairs (hi, lo) of one group.
@@ -142,8 +218,8 @@ __device__ __forceinline__ void group_sum_pair(float &hi, float &lo)
 {
 #pragma unroll
     for (int o = 1; o < G; o <<= 1) {
-        const float oh = __shfl_xor_sync(FULL, hi, o);
-        const float ol = __shfl_xor_sync(FULL, lo, o);
+        const float oh = __shfl_xor_sync(FULL, hi, o * Lanes<G>::STRIDE);
+        const float ol = __shfl_xor_sync(FULL, lo, o * Lanes<G>::STRIDE);
         const float s = hi + oh;
         const float bp = s - hi;
         const float e = (hi - (s - bp)) + (oh - bp);
@@ -190,34 +266,97 @@ __device__ __forceinline__ float bin_of(float qq, const CompConsts &k, bool vali
     return r - (fl - 8388608.0f);
 }
 
-// Walk the curvatures this lane owns: seg(i, qq, valid) for curvature i = base+m-1 (between
-// segments base+m-1 and base+m), the last one with the next lane's first tangent.
-// tan(m, x, y, z) gives the unit tangent of segment j*SPL+m (zero past the last segment);
-// next(t0, n) the next lane's first tangent given this lane's (t0). Every slot is evaluated,
-// with valid = false past curvature N-2, so no table load hides behind a branch (padding
-// tangents are zero: their |t_{i+1}-t_i|^2 is 0 or 1, a bin in the table). FULLN: N == G*SPL,
-// only the group's last boundary is invalid.
-template <int G, int SPL, bool FULLN, class TanFn, class NextFn, class SegFn>
-__device__ __forceinline__ void for_curvatures(uint32_t j, uint32_t N, TanFn tan, NextFn next, SegFn seg)
+// The bins of two squared lengths at once, for tables that need no clamping: bin_of<false> with
+// its additions packed. Returns both fractions.
+__device__ __forceinline__ F2 bins_of(F2 qq, const CompConsts &k, int32_t &L0, int32_t &L1)
 {
-    float t0x = 0.f, t0y = 0.f, t0z = 0.f, px = 0.f, py = 0.f, pz = 0.f;
+    const F2 r = pack2(sqrt_approx(qq.lo()), sqrt_approx(qq.hi()));
+    const F2 fl = add2_rd(r, pack2(8388608.0f, 8388608.0f));
+    L0 = (int32_t)min((uint32_t)fl.v - 0x4B000000u, (uint32_t)k.bins - 1u);
+    L1 = (int32_t)min((uint32_t)(fl.v >> 32) - 0x4B000000u, (uint32_t)k.bins - 1u);
+    return sub2(r, add2(fl, pack2(-8388608.0f, -8388608.0f)));
+}
+
+// How a warp's tangents lie in shared memory (Layout, below). Measured against XYZ with the walk in
+// order (precision geometry, the batched log-sum-exp in both): PAIRS at 32 lanes N = 512 +6 %,
+// 701 +5 %, but 16 x 16 -5 % (more bank conflicts in the rotation, which that shape's
+// shared-memory pipe at 90 % of its wavefronts pays for) and 8 x 16 -8 % (spills); PLANES
+// at 4 lanes N = 64 +17 %, 66 +13 %, at one lane N = 16 +2 %, but under the 64 registers of the 4-lane
+// shapes below 12 segments per lane -4 to -7 % (N = 18, 30, 34).
+enum { kPairs = 0, kXyz = 1, kPlanes = 2 };
+__host__ __device__ constexpr int comp_layout(int G, int SPL)
+{
+    return G == 32 ? kPairs : G == 1 || (G == 4 && SPL >= 12) ? kPlanes : kXyz;
+}
+// Whether the recompute works on pairs of segments with packed arithmetic.
+__host__ __device__ constexpr bool comp_packed(int G, int SPL) { return comp_layout(G, SPL) != kXyz; }
+
+// Three pairs: the tangents of a lane's segments h and h + H, H = (SPL + 1) / 2.
+struct Tan2 {
+    F2 x, y, z;
+};
+
+// Walk the curvatures this lane owns (curvature i lies between segments i and i + 1; the last one
+// with the next lane's first tangent). load.one(m, x, y, z) gives the tangent of segment j*SPL + m,
+// zero past the last segment; next(t0, n) the next lane's first tangent given this lane's (t0).
+// Every slot is evaluated, with valid = false past curvature N-2, so no table load hides behind a
+// branch (padding tangents are zero: their |t_{i+1}-t_i|^2 is 0 or 1, a bin in the table). FULLN:
+// N == G*SPL, only the group's last boundary is invalid.
+// In the layouts with packed arithmetic, seg2(i, i', qq, valid, valid') takes two curvatures at a
+// time, H = (SPL + 1) / 2 apart, and seg1(i, qq, valid) the one left over when SPL is odd: pairs
+// H apart keep every difference of neighbours a difference of two register pairs,
+// P_{h+1} - P_h, with load.pair(h) = the tangents of segments j*SPL + h and j*SPL + h + H (the upper
+// half of the last pair of an odd SPL is not read). The others walk their segments in order.
+template <int G, int SPL, bool FULLN, class Load, class NextFn, class Seg2Fn, class Seg1Fn>
+__device__ __forceinline__ void for_curvatures(uint32_t j, uint32_t N, const Load &load, NextFn next, Seg2Fn seg2, Seg1Fn seg1)
+{
+    constexpr int H = (SPL + 1) / 2;
+    constexpr bool ODD = SPL & 1;
     const uint32_t base = j * SPL;
-#pragma unroll
-    for (int m = 0; m < SPL; ++m) {
-        float tx, ty, tz;
-        tan(m, tx, ty, tz);
-        if (m == 0) {
-            t0x = tx; t0y = ty; t0z = tz;
-        } else {
-            const float dx = tx - px, dy = ty - py, dz = tz - pz;
-            seg(base + m - 1, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), FULLN || base + m <= N - 1);
-        }
-        px = tx; py = ty; pz = tz;
-    }
     float nx, ny, nz;
-    next(t0x, t0y, t0z, nx, ny, nz);
-    const float dx = nx - px, dy = ny - py, dz = nz - pz;
-    seg(base + SPL - 1, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), base + SPL <= N - 1);
+    if constexpr (!comp_packed(G, SPL)) {
+        float t0x = 0.f, t0y = 0.f, t0z = 0.f, px = 0.f, py = 0.f, pz = 0.f;
+#pragma unroll
+        for (int m = 0; m < SPL; ++m) {
+            float tx, ty, tz;
+            load.one(m, tx, ty, tz);
+            if (m == 0) {
+                t0x = tx; t0y = ty; t0z = tz;
+            } else {
+                const float dx = tx - px, dy = ty - py, dz = tz - pz;
+                seg1(base + m - 1, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), FULLN || base + m <= N - 1);
+            }
+            px = tx; py = ty; pz = tz;
+        }
+        next(t0x, t0y, t0z, nx, ny, nz);
+        const float dx = nx - px, dy = ny - py, dz = nz - pz;
+        seg1(base + SPL - 1, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), base + SPL <= N - 1);
+    } else {
+        auto sq2 = [](const Tan2 &b, const Tan2 &a) {
+            const F2 dx = sub2(b.x, a.x), dy = sub2(b.y, a.y), dz = sub2(b.z, a.z);
+            return fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        };
+        Tan2 first = load.pair(0);
+        next(first.x.lo(), first.y.lo(), first.z.lo(), nx, ny, nz);
+        if (ODD && H == 1) first = Tan2{pack2(first.x.lo(), nx), pack2(first.y.lo(), ny), pack2(first.z.lo(), nz)};
+        Tan2 prev = first;
+#pragma unroll
+        for (int h = 1; h < H; ++h) {
+            Tan2 cur = load.pair(h);
+            if (ODD && h == H - 1) cur = Tan2{pack2(cur.x.lo(), nx), pack2(cur.y.lo(), ny), pack2(cur.z.lo(), nz)};
+            // the upper curvature, j*SPL + h + H - 1, is the group's last boundary only for odd SPL
+            seg2(base + h - 1, base + h + H - 1, sq2(cur, prev), FULLN || base + h <= N - 1,
+                 (FULLN && !(ODD && h == H - 1)) || base + h + H <= N - 1);
+            prev = cur;
+        }
+        if constexpr (ODD) {
+            const float dx = first.x.hi() - prev.x.lo(), dy = first.y.hi() - prev.y.lo(), dz = first.z.hi() - prev.z.lo();
+            seg1(base + H - 1, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), (FULLN && SPL > 1) || base + H <= N - 1);
+        } else {
+            const Tan2 cur{pack2(first.x.hi(), nx), pack2(first.y.hi(), ny), pack2(first.z.hi(), nz)};
+            seg2(base + H - 1, base + SPL - 1, sq2(cur, prev), FULLN || base + H <= N - 1, base + SPL <= N - 1);
+        }
+    }
 }
 
 // next() for tangents held in registers: the next lane's t0 by shuffle.
@@ -228,9 +367,9 @@ struct ShflNext {
         if constexpr (G == 1) {   // a one-lane chain has no next lane: its last slot is padding
             nx = t0x; ny = t0y; nz = t0z;
         } else {
-            nx = __shfl_down_sync(FULL, t0x, 1, G);
-            ny = __shfl_down_sync(FULL, t0y, 1, G);
-            nz = __shfl_down_sync(FULL, t0z, 1, G);
+            nx = __shfl_down_sync(FULL, t0x, Lanes<G>::STRIDE);
+            ny = __shfl_down_sync(FULL, t0y, Lanes<G>::STRIDE);
+            nz = __shfl_down_sync(FULL, t0z, Lanes<G>::STRIDE);
         }
     }
 };
@@ -253,9 +392,9 @@ __device__ __forceinline__ float2 tab_load(const float2 *__restrict__ tab, int32
 // Generic full recompute of one path's log10 weight (absorption excluded), for the exact
 // table or, with 64-bit lane sums, for the fixed-point table at any lane width. bin_sink(i,
 // bin) receives every curvature's bin (-1 for NaN).
-template <int G, int SPL, bool EXACT, bool CLAMP, bool GLOBAL = false, class TanFn, class NextFn, class BinFn>
+template <int G, int SPL, bool EXACT, bool CLAMP, bool GLOBAL = false, class Load, class NextFn, class BinFn>
 __device__ __forceinline__ double path_log10(uint32_t j, uint32_t N, const float2 *__restrict__ tab,
-                                             const CompConsts &k, TanFn tan, NextFn next, BinFn bin_sink,
+                                             const CompConsts &k, const Load &load, NextFn next, BinFn bin_sink,
                                              uint32_t &clamped)
 {
     unsigned long long isum = 0;
@@ -274,11 +413,15 @@ __device__ __forceinline__ double path_log10(uint32_t j, uint32_t N, const float
             csum = valid ? c2 : csum;
         }
     };
+    auto seg2 = [&](uint32_t i0, uint32_t i1, F2 qq, bool v0, bool v1) {
+        seg(i0, qq.lo(), v0);
+        seg(i1, qq.hi(), v1);
+    };
     // a chain that fills its group's slots: slot validity known at compile time
     if (N == (uint32_t)(G * SPL))
-        for_curvatures<G, SPL, true>(j, N, tan, next, seg);
+        for_curvatures<G, SPL, true>(j, N, load, next, seg2, seg);
     else
-        for_curvatures<G, SPL, false>(j, N, tan, next, seg);
+        for_curvatures<G, SPL, false>(j, N, load, next, seg2, seg);
     if (EXACT) {
         float hi = ks, lo = -kc;
         group_sum_pair<G>(hi, lo);
@@ -289,45 +432,55 @@ __device__ __forceinline__ double path_log10(uint32_t j, uint32_t N, const float
     return k.lw_offset + (double)is * k.inv_scale + (double)cs;
 }
 
-// Fixed-point full recompute for chains: the group's total of table entries plus rounded
-// interpolation corrections, in units of 2^-s. Each lane's sum is exact in 32 bits (its true
-// value lies in [0, 2^32) by the table's scale); the group total is added in 32 bits for a
-// narrow table, in 64 bits for a wide one (both exact). *bad is set when any curvature of
-// the path is NaN.
-template <int G, int SPL, bool CLAMP, bool GLOBAL, class TanFn, class NextFn>
-__device__ __forceinline__ unsigned long long path_fixed(uint32_t j, uint32_t gbase, uint32_t N, const float2 *__restrict__ tab,
-                                               const CompConsts &k, TanFn tan, NextFn next, bool &bad,
+// Fixed-point full recompute for chains: this lane's share of the path total, table entries plus
+// the rounded interpolation correction, in units of 2^-s. Each lane's sum is exact in 32 bits
+// (its true value lies in [0, 2^32) by the table's scale); the group total is added in 32 bits
+// for a narrow table, in 64 bits for a wide one (both exact). nan is set when one of the lane's
+// curvatures is NaN or in a steep bin.
+template <int G, int SPL, bool CLAMP, bool GLOBAL, class Load, class NextFn>
+__device__ __forceinline__ uint32_t path_fixed(uint32_t j, uint32_t N, const float2 *__restrict__ tab,
+                                               const CompConsts &k, const Load &load, NextFn next, bool &nan,
                                                uint32_t &clamped)
 {
     uint32_t isum = 0;
-    float csum = 0.f;
-    auto seg = [&](uint32_t, float qq, bool valid) {
-        int32_t L;
-        const float frac = bin_of<CLAMP>(qq, k, valid, clamped, L);
+    float c0 = 0.f, c1 = 0.f;
+    // a padding slot leaves the sum alone even where the slope is NaN (a steep bin)
+    auto entry = [&](int32_t L, float frac, bool valid, float &c) {
         const float2 e = tab_load<GLOBAL>(tab, L);
         isum += valid ? __float_as_uint(e.x) : 0u;
-        // a padding slot leaves the sum alone even where the slope is NaN (a steep bin)
-        const float c2 = fmaf(frac, e.y, csum);
-        csum = valid ? c2 : csum;
+        const float c2 = fmaf(frac, e.y, c);
+        c = valid ? c2 : c;
+    };
+    auto seg1 = [&](uint32_t, float qq, bool valid) {
+        int32_t L;
+        const float frac = bin_of<CLAMP>(qq, k, valid, clamped, L);
+        entry(L, frac, valid, c0);
+    };
+    auto seg2 = [&](uint32_t i0, uint32_t i1, F2 qq, bool v0, bool v1) {
+        if constexpr (CLAMP) {
+            int32_t L0, L1;
+            const float f0 = bin_of<true>(qq.lo(), k, v0, clamped, L0), f1 = bin_of<true>(qq.hi(), k, v1, clamped, L1);
+            entry(L0, f0, v0, c0);
+            entry(L1, f1, v1, c1);
+        } else {
+            int32_t L0, L1;
+            const F2 f = bins_of(qq, k, L0, L1);
+            entry(L0, f.lo(), v0, c0);
+            entry(L1, f.hi(), v1, c1);
+        }
     };
     if (N == (uint32_t)(G * SPL))
-        for_curvatures<G, SPL, true>(j, N, tan, next, seg);
+        for_curvatures<G, SPL, true>(j, N, load, next, seg2, seg1);
     else
-        for_curvatures<G, SPL, false>(j, N, tan, next, seg);
-    const uint32_t nan_lanes = __ballot_sync(FULL, isnan(csum));
-    constexpr uint32_t gmask = (G == 32) ? FULL : ((1u << G) - 1u);
-    bad = ((nan_lanes >> gbase) & gmask) != 0u;
-    isum += (uint32_t)__float2int_rn(csum * k.fscale);
-    if (k.wide) return group_sum<G>((unsigned long long)isum);
-    return (unsigned long long)group_sum<G>(isum);
+        for_curvatures<G, SPL, false>(j, N, load, next, seg2, seg1);
+    const float csum = comp_packed(G, SPL) ? c0 + c1 : c0;
+    nan = isnan(csum);
+    return isum + (uint32_t)__float2int_rn(csum * k.fscale);
 }
 
-// Row pitches of a warp's planes (float2 and float elements). With several lanes per chain
-// the rows are padded so that the consecutive segments of one rotation, spread over lanes and
-// rows, fall in distinct banks. With one lane per chain every lane is its own chain: a rotation
-// has the lanes at unrelated rows, and an unpadded row of 32 puts lane i in bank (pair) i mod
-// 16 (32) whatever its row, so no access conflicts (the padded pitch measured the one-lane
-// kernel bound by shared-memory wavefronts at 92 % of their peak).
+// Row pitches of the XYZ layout (float2 and float elements), and with them the bytes of shared
+// memory per warp that hold its chains' tangents whatever the layout: the chain count of a pass
+// with num_chains 0 follows from how many warps fit, so the size is the same for all three.
 __host__ __device__ constexpr int comp_pitch_xy(int G, int SPL)
 {
     return G == 1 ? 32 : 32 + ((16 / SPL) > 1 ? (16 / SPL) : 1);
@@ -336,24 +489,82 @@ __host__ __device__ constexpr int comp_pitch_z(int G, int SPL)
 {
     return G == 1 ? 32 : 32 + ((G / SPL) > 1 ? (G / SPL) : 1);
 }
+__host__ __device__ constexpr int warp_state_bytes(int G, int SPL)
+{
+    return (SPL * (comp_pitch_xy(G, SPL) * 8 + comp_pitch_z(G, SPL) * 4) + 15) / 16 * 16;
+}
 
-template <int G, int SPL>
-struct Layout {
-    static constexpr int PXY = comp_pitch_xy(G, SPL);  // float2 plane pitch
-    static constexpr int PZ = comp_pitch_z(G, SPL);    // float plane pitch
-    static constexpr int XY_BYTES = SPL * PXY * 8;
-    static constexpr int Z_BYTES = SPL * PZ * 4;
-    // xy, z planes; rounded to 16 bytes so that every warp's float2 plane (and what follows the
-    // last warp) stays aligned when SPL * PZ is odd
-    static constexpr int WARP_BYTES = (XY_BYTES + Z_BYTES + 15) / 16 * 16;
-    __device__ __forceinline__ static uint32_t xy(uint32_t col, uint32_t m) { return m * (uint32_t)PXY + col; }
-    __device__ __forceinline__ static uint32_t z(uint32_t col, uint32_t m) { return m * (uint32_t)PZ + col; }
+// Where segment m of lane o of a chain lies (qb: the chain's base lane): a for x (XYZ: for (x, y), in
+// float2), b for z in XYZ.
+struct Slot {
+    uint32_t a, b;
 };
 
-constexpr size_t warp_state_bytes(int G, int SPL)
-{
-    return ((size_t)SPL * comp_pitch_xy(G, SPL) * 8 + (size_t)SPL * comp_pitch_z(G, SPL) * 4 + 15) / 16 * 16;
-}
+// The layout of a warp's tangents in shared memory:
+//  * PAIRS: three planes (x, y, z); row h of each holds, per lane, the pair of segments
+//    h and h + H, H = (SPL + 1) / 2, as one float2: the recompute reads a pair of tangents by three
+//    8-byte loads (consecutive columns of one row, no bank conflicts) straight into the register
+//    pairs that its packed arithmetic works on. Of an odd SPL's last row only the lower half
+//    exists, as one float per lane. Rows are padded to PP pairs, as many as the bytes allow.
+//  * XYZ: (x, y) as float2 and z in planes of one row per segment, at immediate offsets from a
+//    lane's base: 12 bytes per tangent too, in an 8-byte and a 4-byte load. The row pitches
+//    (32 + 16/SPL float2, 32 + G/SPL floats) put the consecutive segments of a rotation in distinct
+//    banks (at most 2-way conflicts).
+//  * PLANES: x, y and z in rows of 32 floats, the column rotated by the row: 4 consecutive
+//    segments of a 4-lane chain lie in the chain's own 4 banks where SPL = 1 mod 4 (and mostly so for
+//    other SPL), and every access of a one-lane chain in its own bank.
+template <int G, int SPL>
+struct Layout {
+    static constexpr int KIND = comp_layout(G, SPL);
+    static constexpr int H = (SPL + 1) / 2;
+    static constexpr bool ODD = SPL & 1;
+    static constexpr int CPW = 32 / G;
+    static constexpr int PXY = comp_pitch_xy(G, SPL), PZ = comp_pitch_z(G, SPL);
+    static constexpr int WARP_BYTES = warp_state_bytes(G, SPL);
+    static constexpr int PP = (WARP_BYTES / 12 - (ODD ? 32 : 0)) / (SPL / 2) / 2;
+    static constexpr int PLANE = KIND == kPairs ? (SPL / 2) * 2 * PP + (ODD ? 32 : 0) : SPL * 32;   // floats
+    static_assert(KIND == kXyz || (PP >= 32 && 3 * PLANE * 4 <= WARP_BYTES && PLANE % 2 == 0), "the planes fit");
+    __device__ __forceinline__ static Slot slot(uint32_t o, uint32_t m, uint32_t qb)
+    {
+        if constexpr (KIND == kPlanes) {
+            const uint32_t w = m * 32u + ((CPW * (o + m) + qb) & 31u);
+            return Slot{w, w};
+        } else if constexpr (KIND == kXyz) {
+            const uint32_t col = G == 4 ? o * CPW + qb : qb + o;
+            return Slot{m * PXY + col, m * PZ + col};
+        } else {
+            const uint32_t col = qb + o;
+            const uint32_t up = m >= (uint32_t)H ? 1u : 0u;
+            uint32_t w = (m - up * H) * (2u * PP) + 2u * col + up;
+            if (ODD && m == (uint32_t)(H - 1)) w = (H - 1) * 2u * PP + col;
+            return Slot{w, w};
+        }
+    }
+    __device__ __forceinline__ static void get(const float *t, Slot s, float &x, float &y, float &z)
+    {
+        if constexpr (KIND == kXyz) {
+            const float2 v = reinterpret_cast<const float2 *>(t)[s.a];
+            x = v.x;
+            y = v.y;
+            z = (t + SPL * PXY * 2)[s.b];
+        } else {
+            x = t[s.a];
+            y = t[s.a + PLANE];
+            z = t[s.a + 2 * PLANE];
+        }
+    }
+    __device__ __forceinline__ static void put(float *t, Slot s, float x, float y, float z)
+    {
+        if constexpr (KIND == kXyz) {
+            reinterpret_cast<float2 *>(t)[s.a] = make_float2(x, y);
+            (t + SPL * PXY * 2)[s.b] = z;
+        } else {
+            t[s.a] = x;
+            t[s.a + PLANE] = y;
+            t[s.a + 2 * PLANE] = z;
+        }
+    }
+};
 
 // Threads per CTA the chain kernel of a shape is compiled for (its register budget: 65536 /
 // threads). With 12 or more segments per lane every shape fits 768 threads (24 warps) in 80
@@ -369,11 +580,50 @@ __host__ __device__ constexpr int comp_max_threads(int G, int SPL)
 // padding segments 1).
 __host__ __device__ constexpr size_t cta_len_bytes(int G, int SPL) { return ((size_t)G * SPL * 4 + 15) / 16 * 16; }
 
-// The planes of one warp's chains (tangents) and the CTA's segment lengths.
+// One warp's tangents and the CTA's segment lengths.
 struct Planes {
-    float2 *xy;
-    float *z;
+    float *t;    // Layout
     float *l;    // CTA-wide, by segment index
+};
+
+// The tangents of lane j of the chain in slot q, for for_curvatures. SHIFT: the weights see the
+// receiver moved by `shift`: v_{N-2} = l t + shift, renormalised.
+template <int G, int SPL, bool SHIFT = false>
+struct SmemLoad {
+    using Lay = Layout<G, SPL>;
+    const Planes &st;
+    uint32_t qb, j;
+    uint32_t moved;       // SHIFT: segment N - 2
+    const float *shift;
+    float kscale, inv_ks;
+    __device__ __forceinline__ void one(int m, float &x, float &y, float &z) const
+    {
+        Lay::get(st.t, Lay::slot(j, m, qb), x, y, z);
+        if (SHIFT && j * SPL + m == moved) {
+            const float l = st.l[j * SPL + m] * inv_ks;
+            x = fmaf(l, x, shift[0]);
+            y = fmaf(l, y, shift[1]);
+            z = fmaf(l, z, shift[2]);
+            const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kscale;
+            x *= r; y *= r; z *= r;
+        }
+    }
+    __device__ __forceinline__ Tan2 pair(int h) const
+    {
+        constexpr int H = Lay::H;
+        const bool both = !(Lay::ODD && h == H - 1);
+        if constexpr (Lay::KIND == kPairs && !SHIFT) {
+            if (both) {
+                const float2 *p = reinterpret_cast<const float2 *>(st.t) + (qb + j) + h * Lay::PP;
+                const float2 x = p[0], y = p[Lay::PLANE / 2], z = p[Lay::PLANE];
+                return Tan2{pack2(x.x, x.y), pack2(y.x, y.y), pack2(z.x, z.y)};
+            }
+        }
+        float x0, y0, z0, x1 = 0.f, y1 = 0.f, z1 = 0.f;
+        one(h, x0, y0, z0);
+        if (both) one(h + H, x1, y1, z1);
+        return Tan2{pack2(x0, x1), pack2(y0, y1), pack2(z0, z1)};
+    }
 };
 
 enum { kModeForward = 0, kModeExport = 1, kModeAdjoint = 2 };
@@ -443,19 +693,12 @@ __device__ __forceinline__ void stage_table(float4 *smem4, const float2 *__restr
 // fixed-point table that cross a steep bin. Not inlined: it runs rarely, and inlined its
 // registers would count against the hot loop's.
 template <int G, int SPL, bool CLAMP>
-__device__ __noinline__ double steep_fallback(Planes st, uint32_t gbase, uint32_t j, uint32_t N,
+__device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j, uint32_t N,
                                               const float2 *__restrict__ lin, CompConsts kc)
 {
-    using Lay = Layout<G, SPL>;
-    const uint32_t own = gbase + j;
-    auto tan = [&](int m, float &x, float &y, float &z) {
-        const float2 a = st.xy[Lay::xy(own, m)];
-        x = a.x;
-        y = a.y;
-        z = st.z[Lay::z(own, m)];
-    };
+    const SmemLoad<G, SPL> load{st, qb, j, 0, nullptr, 0.f, 0.f};
     uint32_t unused = 0;
-    return path_log10<G, SPL, true, CLAMP, true>(j, N, lin, kc, tan, ShflNext<G>{}, [](uint32_t, int32_t) {}, unused);
+    return path_log10<G, SPL, true, CLAMP, true>(j, N, lin, kc, load, ShflNext<G>{}, [](uint32_t, int32_t) {}, unused);
 }
 
 // One Markov chain run by the G lanes of one group on its own records st (tangent, length;
@@ -468,7 +711,7 @@ template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INC
           bool TAB_GLOBAL = false>
 __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConsts &kc,
                                              const float *__restrict__ init_seg, const float2 *s_tab, Planes st,
-                                             uint32_t gbase, uint32_t j, uint32_t chain, bool real_chain,
+                                             uint32_t qb, uint32_t j, uint32_t chain, bool real_chain,
                                              ChainOut *__restrict__ out, const ModeArgs &ma)
 {
     constexpr bool FIX = !EXACT && MODE != kModeAdjoint;
@@ -478,8 +721,9 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
     // the tangents are stored at length kscale; records handed to export and the adjoint are unit
     const float inv_ks = 1.0f / kc.kscale;
     auto load_rec = [&](uint32_t owner, uint32_t m) {
-        const float2 a = st.xy[Lay::xy(gbase + owner, m)];
-        return make_float4(a.x * inv_ks, a.y * inv_ks, st.z[Lay::z(gbase + owner, m)] * inv_ks, st.l[owner * SPL + m]);
+        float x, y, z;
+        Lay::get(st.t, Lay::slot(owner, m, qb), x, y, z);
+        return make_float4(x * inv_ks, y * inv_ks, z * inv_ks, st.l[owner * SPL + m]);
     };
 
     float max_len = 0.f;
@@ -499,11 +743,10 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
             x *= h * kc.kscale; y *= h * kc.kscale; z *= h * kc.kscale;       // stored at length kscale
             max_len = fmaxf(max_len, len);
         }
-        st.xy[Lay::xy(gbase + j, m)] = make_float2(x, y);
-        st.z[Lay::z(gbase + j, m)] = z;
+        Lay::put(st.t, Lay::slot(j, m, qb), x, y, z);
     }
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) max_len = fmaxf(max_len, __shfl_xor_sync(FULL, max_len, o));
+    for (int o = 1; o < G; o <<= 1) max_len = fmaxf(max_len, __shfl_xor_sync(FULL, max_len, o * Lanes<G>::STRIDE));
     // fixed-point chord scale: a segment is at most 2^24 units, 64 of them at most 2^30
     const float chord_scale = 16777216.0f / (max_len * kc.kscale);   // the tangents have length kscale
     const float renorm = -0.5f * inv_ks * inv_ks;   // Newton step to |t'| = kscale: 1.5 + renorm |t'|^2
@@ -544,10 +787,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
     // tangent of segment s (any lane's) and the fixed-point term of the curvature between two
     // tangents, with its interpolation correction rounded on its own
     auto tan_at = [&](uint32_t s, float &x, float &y, float &z) {
-        const float2 a = st.xy[Lay::xy(gbase + s / SPL, s % SPL)];
-        x = a.x;
-        y = a.y;
-        z = st.z[Lay::z(gbase + s / SPL, s % SPL)];
+        Lay::get(st.t, Lay::slot(s / SPL, s % SPL, qb), x, y, z);
     };
     auto term = [&](float ax, float ay, float az, float bx, float by, float bz, bool &nan) -> uint32_t {
         const float dx = bx - ax, dy = by - ay, dz = bz - az;
@@ -560,36 +800,83 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
         return __float_as_uint(e.x) + (uint32_t)__float2int_rn(cor * kc.fscale);
     };
 
-    const uint32_t own = gbase + j;
-    // tangent of this lane's segment m; with SHIFT the weights see the receiver moved:
-    // v_{N-2} = l t + shift, renormalised
-    auto tan_smem = [&](int m, float &x, float &y, float &z) {
-        const float2 a = st.xy[Lay::xy(own, m)];
-        x = a.x;
-        y = a.y;
-        z = st.z[Lay::z(own, m)];
-        if (SHIFT && j * SPL + m == N - 2) {
-            const float l = st.l[j * SPL + m] * inv_ks;
-            x = fmaf(l, x, c.eval_shift[0]);
-            y = fmaf(l, y, c.eval_shift[1]);
-            z = fmaf(l, z, c.eval_shift[2]);
-            const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kc.kscale;
-            x *= r; y *= r; z *= r;
+    const SmemLoad<G, SPL, SHIFT> load_smem{st, qb, j, N - 2, c.eval_shift, kc.kscale, inv_ks};
+    const ShflNext<G> next_smem{};
+    // The chain's running log-sum-exp (fixed-point form). It starts from the total 0 with an empty
+    // sum: the first path's total is its new maximum.
+    auto lse_add = [&](unsigned long long tot) {
+        // exact integer difference: narrow totals stay below 2^31, wide ones are 64-bit
+        const float dt = kc.wide ? (float)(long long)(tot - lse_t) : (float)(int32_t)((uint32_t)tot - (uint32_t)lse_t);
+        const float x = dt * kc.l2s;
+        float term = 1.f;
+        if (x > 0.f) {
+            const float f = ex2_approx(-x);
+            lse_s *= f;
+            lse_c *= f;
+            lse_t = tot;
+        } else {
+            term = ex2_approx(x);
+        }
+        kahan_add(lse_s, lse_c, term);
+    };
+    // Forward passes of groups of 4 lanes and more sum the lanes' shares of four path totals together:
+    // exchanges after every second and fourth weighted step leave one step's shares in each lane (step
+    // j mod 4), the other levels add as a butterfly does, and each lane runs the log-sum-exp of
+    // its own steps: 5 shuffles for four paths of 16 lanes instead of 16, and one log-sum-exp
+    // update for four paths instead of one for each in every lane.
+    constexpr bool BATCH = FIX && MODE == kModeForward && !INCR && G >= 4;
+    constexpr int LS = Lanes<G>::STRIDE;
+    uint32_t even = 0, flags = 0;       // the even step's share; steps 0..3 met (bits 0..3) and weighed (bits 4..7)
+    unsigned long long pair01 = 0;
+    // the lower lane (by bit `up` of j) keeps x0 and sends x1, the upper one the other way round
+    auto exchange = [&](unsigned long long x0, unsigned long long x1, bool up, int off) -> unsigned long long {
+        if (kc.wide) return (up ? x1 : x0) + __shfl_xor_sync(FULL, up ? x0 : x1, off);
+        return (uint32_t)(up ? x1 : x0) + __shfl_xor_sync(FULL, (uint32_t)(up ? x0 : x1), off);
+    };
+    auto exchange32 = [&](uint32_t x0, uint32_t x1, bool up, int off) -> unsigned long long {
+        const uint32_t got = __shfl_xor_sync(FULL, up ? x0 : x1, off);
+        return kc.wide ? (unsigned long long)(up ? x1 : x0) + got : (unsigned long long)((up ? x1 : x0) + got);
+    };
+    auto batch_step = [&](uint32_t slot, bool end, uint32_t part) {
+        if (slot & 1u) {
+            const unsigned long long two = exchange32(even, part, j & 1u, LS);
+            if (slot == 1u) pair01 = two;
+            if (slot == 3u || end) {
+                unsigned long long tot = exchange(pair01, slot == 3u ? two : 0ull, j & 2u, 2 * LS);
+                if (kc.wide) {
+#pragma unroll
+                    for (int o = 4; o < G; o <<= 1) tot += __shfl_xor_sync(FULL, tot, o * LS);
+                } else {
+                    uint32_t t32 = (uint32_t)tot;
+#pragma unroll
+                    for (int o = 4; o < G; o <<= 1) t32 += __shfl_xor_sync(FULL, t32, o * LS);
+                    tot = t32;
+                }
+                if ((flags >> (4u + (j & 3u))) & 1u) lse_add(tot);
+                valid += __popc(flags >> 4);
+                failed += __popc(flags & 15u) - __popc(flags >> 4);
+                flags = 0;
+            }
+        } else {
+            even = part;
         }
     };
-    const ShflNext<G> next_smem{};
     auto no_bins = [](uint32_t, int32_t) {};
 
     for (uint32_t base = 0; base < total; base += G) {
         const dev::Proposal pr = dev::draw_step(c.seed, c.experiment, gchain, base + j, N, c.k_eff, c.max_angle);
+        // sin = 2 s c and 1 - cos = 2 s^2 of the turn (half angle s, c); k and left in one word, so
+        // that three shuffles broadcast a proposal
         float psn, pcs;
         dev::sincos_half(pr.angle, psn, pcs);
+        const float psth = 2.f * psn * pcs, pomc = 2.f * psn * psn;
+        const uint32_t pkl = pr.k | (pr.left << 8);   // k <= 64, left < 1024
         const uint32_t nstep = min((uint32_t)G, total - base);
         for (uint32_t jj = 0; jj < nstep; ++jj) {
-            const uint32_t k = __shfl_sync(FULL, pr.k, jj, G);
-            const uint32_t left = __shfl_sync(FULL, pr.left, jj, G);
-            const float sn = __shfl_sync(FULL, psn, jj, G);
-            const float cs = __shfl_sync(FULL, pcs, jj, G);
+            const uint32_t kl = Lanes<G>::from(pkl, jj, qb);
+            const uint32_t k = kl & 255u, left = kl >> 8;
+            const float sth0 = Lanes<G>::from(psth, jj, qb);
+            const float omc = Lanes<G>::from(pomc, jj, qb);
             const uint32_t right = left + k;
             // the segments this chain turns: the sub-chain, or its complement where that is
             // shorter, on the steps where that takes two or more rounds off the warp's rotation
@@ -602,13 +889,14 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     dX = 0.f; dY = 0.f; dZ = 0.f;
 #pragma unroll
                     for (int m = 0; m < SPL; ++m) {   // padding slots hold zero tangents
-                        const float2 a = st.xy[Lay::xy(own, m)];
+                        float x, y, z;
+                        Lay::get(st.t, Lay::slot(j, m, qb), x, y, z);
                         const float l = st.l[j * SPL + m];
-                        dX = fmaf(l, a.x, dX);
-                        dY = fmaf(l, a.y, dY);
-                        dZ = fmaf(l, st.z[Lay::z(own, m)], dZ);
+                        dX = fmaf(l, x, dX);
+                        dY = fmaf(l, y, dY);
+                        dZ = fmaf(l, z, dZ);
                     }
-                    group_sum3<G>(dX, dY, dZ);
+                    group_sum3<G>(dX, dY, dZ, j, qb);
                 }
                 // whole-warp reductions: every chain of a warp belongs to one experiment (a CTA
                 // runs one experiment's work item at a time), so cmpl_on is the same in every lane
@@ -624,7 +912,8 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
             } else {
                 kmax = k;
 #pragma unroll
-                for (int o = G; o < 32; o <<= 1) kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
+                for (int o = 1; o < Lanes<G>::CPW; o <<= 1)   // over the warp's chains
+                    kmax = max(kmax, __shfl_xor_sync(FULL, kmax, G == 4 ? o : o * G));
             }
             const uint32_t rounds = min((kmax + G - 1) / G, max_rounds);
             // incremental form: the two end curvatures before the rotation (kappa_{left-1} and
@@ -652,6 +941,15 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
             // round's in registers (measured: no spills, N <= 64 up to 27 % faster)
             constexpr bool RELOAD = R > 4 && (SPL < 16 || G < 8);
             constexpr int RK = RELOAD ? 1 : R;
+            // PLANES shapes turn the segments of two rounds at once with the packed instructions (16
+            // for two segments instead of 32; the same roundings). Their 4-lane shapes keep the
+            // chord pass's slots, two to a register, instead of finding each again. Together
+            // N = 66 +11 % over PLANES without them, N = 24 on one lane +8 %, and 13 % off a burn-in step.
+            // Under the 64 registers of the 4-lane shapes below 12 segments per lane the pairs spill
+            // (N = 16..36 -10 to -25 %), and the Rodrigues form packed lost 6-18 % at 8 lanes.
+            constexpr bool PACK_ROT = Lay::KIND == kPlanes;
+            constexpr bool KEEP_SLOTS = PACK_ROT && G == 4;
+            static_assert(!PACK_ROT || RELOAD, "the packed rotation reads its tangents again");
             // The move: the chord of the turned segments, the axis, the rotation. WRAP: the warp
             // turns complements this step (the chains with cm), which wrap past segment N-1 to 0,
             // turn by -theta and carry d; a step that turns none runs the plain code.
@@ -666,7 +964,8 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     return s;
                 };
                 float vx[RK], vy[RK], vz[RK];
-                uint32_t va[RK], vb[RK];
+                Slot va[RK];
+                [[maybe_unused]] uint32_t slots2[(R + 1) / 2];   // KEEP_SLOTS: below 2^16 each
                 float cx = 0.f, cy = 0.f, cz = 0.f;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -674,13 +973,10 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     const uint32_t idx = j + r * G;
                     const uint32_t s = seg_of(idx);
                     const int ri = RELOAD ? 0 : r;
-                    va[ri] = Lay::xy(gbase + s / SPL, s % SPL);
-                    vb[ri] = Lay::z(gbase + s / SPL, s % SPL);
+                    va[ri] = Lay::slot(s / SPL, s % SPL, qb);
+                    if constexpr (KEEP_SLOTS) slots2[r / 2] = (r & 1) ? slots2[r / 2] + (va[0].a << 16) : va[0].a;
                     if (WRAP ? idx < cnt : s < right) {
-                        const float2 a = st.xy[va[ri]];
-                        vx[ri] = a.x;
-                        vy[ri] = a.y;
-                        vz[ri] = st.z[vb[ri]];
+                        Lay::get(st.t, va[ri], vx[ri], vy[ri], vz[ri]);
                         const float l = st.l[s];
                         cx = fmaf(l, vx[ri], cx);
                         cy = fmaf(l, vy[ri], cy);
@@ -698,70 +994,94 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     cy = (float)iy;
                     cz = (float)iz;
                 } else {
-                    group_sum3<G>(cx, cy, cz);
+                    group_sum3<G>(cx, cy, cz, j, qb);
                 }
                 if (cmw) { cx = dX - cx; cy = dY - cy; cz = dZ - cz; }   // the sub-chain's chord
                 // Rodrigues by +theta about the unit chord a -- the rotation the reference's
                 // quaternion sandwich q^-1 p q applies with its product convention:
-                // v cos + (a x v) sin + a (a.v)(1 - cos), sin = 2 s c, 1 - cos = 2 s^2 (half angle s, c)
+                // v cos + (a x v) sin + a (a.v)(1 - cos)
                 const float inv = rsqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
                 const float ax = cx * inv, ay = cy * inv, az = cz * inv;
-                const float sth = (cmw ? -2.f : 2.f) * sn * cs, omc = 2.f * sn * sn;
+                const float sth = cmw ? -sth0 : sth0;
                 // Groups of 1 or 4 lanes (up to 32 or 8 rounds): the rotation as v + M v with
                 // M = R - I = sin(theta) [a]x + (1 - cos(theta)) (a a^T - I), built once per step,
                 // 9 FMAs per segment against 19 for the Rodrigues form (the correction is added
                 // to v, so it rounds like the Rodrigues terms do). Measured +4.6-5.5 % at
                 // N = 8..24 and +1-2 % at N = 32..96; with 8-lane groups (4 rounds) 1.9 % slower
                 // at N = 128, so those keep the Rodrigues form.
-                constexpr bool RMAT = G <= 4;
-                float m00 = 0.f, m01 = 0.f, m02 = 0.f, m10 = 0.f, m11 = 0.f, m12 = 0.f, m20 = 0.f, m21 = 0.f, m22 = 0.f;
-                if constexpr (RMAT) {
-                    const float oax = omc * ax, oay = omc * ay, oaz = omc * az;
-                    const float sax = sth * ax, say = sth * ay, saz = sth * az;
-                    m00 = fmaf(oax, ax, -omc);
-                    m11 = fmaf(oay, ay, -omc);
-                    m22 = fmaf(oaz, az, -omc);
-                    m01 = fmaf(oax, ay, -saz);
-                    m10 = fmaf(oax, ay, saz);
-                    m02 = fmaf(oax, az, say);
-                    m20 = fmaf(oax, az, -say);
-                    m12 = fmaf(oay, az, -sax);
-                    m21 = fmaf(oay, az, sax);
-                }
-                __syncwarp();
+                [[maybe_unused]] constexpr bool RMAT = G <= 4;
+                if constexpr (PACK_ROT) {
+                    const F2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+                    const F2 omc2 = pack2(omc, omc), nomc2 = pack2(-omc, -omc), sth2 = pack2(sth, sth), nsth2 = pack2(-sth, -sth);
+                    const F2 oax = mul2(omc2, ax2), oay = mul2(omc2, ay2), oaz = mul2(omc2, az2);
+                    const F2 m00 = fma2(oax, ax2, nomc2), m11 = fma2(oay, ay2, nomc2), m22 = fma2(oaz, az2, nomc2);
+                    const F2 m01 = fma2(oax, ay2, mul2(nsth2, az2)), m10 = fma2(oax, ay2, mul2(sth2, az2));
+                    const F2 m02 = fma2(oax, az2, mul2(sth2, ay2)), m20 = fma2(oax, az2, mul2(nsth2, ay2));
+                    const F2 m12 = fma2(oay, az2, mul2(nsth2, ax2)), m21 = fma2(oay, az2, mul2(sth2, ax2));
+                    const F2 renorm2 = pack2(renorm, renorm), c15 = pack2(1.5f, 1.5f);
+                    __syncwarp();
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (r > 0 && (uint32_t)r >= rounds) break;
-                    const uint32_t idx = j + r * G;
-                    const uint32_t s = seg_of(idx);
-                    const int ri = RELOAD ? 0 : r;
-                    if (RELOAD) {
-                        va[0] = Lay::xy(gbase + s / SPL, s % SPL);
-                        vb[0] = Lay::z(gbase + s / SPL, s % SPL);
+                    for (int r = 0; r < R; r += 2) {
+                        if (r > 0 && (uint32_t)r >= rounds) break;
+                        const uint32_t i0 = j + r * G, i1 = i0 + G;
+                        const uint32_t s0 = seg_of(i0), s1 = seg_of(i1);
+                        const bool p0 = WRAP ? i0 < cnt : s0 < right;
+                        const bool p1 = r + 1 < R && (WRAP ? i1 < cnt : s1 < right);
+                        const Slot a0 = KEEP_SLOTS ? Slot{slots2[r / 2] & 0xFFFFu, 0} : Lay::slot(s0 / SPL, s0 % SPL, qb);
+                        const Slot a1 = KEEP_SLOTS ? Slot{slots2[r / 2] >> 16, 0} : Lay::slot(s1 / SPL, s1 % SPL, qb);
+                        float x0 = 0.f, y0 = 0.f, z0 = 0.f, x1 = 0.f, y1 = 0.f, z1 = 0.f;
+                        if (p0) Lay::get(st.t, a0, x0, y0, z0);
+                        if (p1) Lay::get(st.t, a1, x1, y1, z1);
+                        const F2 x = pack2(x0, x1), y = pack2(y0, y1), z = pack2(z0, z1);
+                        const F2 nx = fma2(m00, x, fma2(m01, y, fma2(m02, z, x)));
+                        const F2 ny = fma2(m10, x, fma2(m11, y, fma2(m12, z, y)));
+                        const F2 nz = fma2(m20, x, fma2(m21, y, fma2(m22, z, z)));
+                        const F2 h = fma2(renorm2, fma2(nx, nx, fma2(ny, ny, mul2(nz, nz))), c15);
+                        const F2 rx = mul2(nx, h), ry = mul2(ny, h), rz = mul2(nz, h);
+                        if (p0) Lay::put(st.t, a0, rx.lo(), ry.lo(), rz.lo());
+                        if (p1) Lay::put(st.t, a1, rx.hi(), ry.hi(), rz.hi());
                     }
-                    if (WRAP ? idx < cnt : s < right) {
-                        if (RELOAD) {
-                            const float2 a = st.xy[va[0]];
-                            vx[0] = a.x;
-                            vy[0] = a.y;
-                            vz[0] = st.z[vb[0]];
+                } else {
+                    [[maybe_unused]] float m00 = 0.f, m01 = 0.f, m02 = 0.f, m10 = 0.f, m11 = 0.f, m12 = 0.f, m20 = 0.f, m21 = 0.f, m22 = 0.f;
+                    if constexpr (RMAT) {
+                        const float oax = omc * ax, oay = omc * ay, oaz = omc * az;
+                        const float sax = sth * ax, say = sth * ay, saz = sth * az;
+                        m00 = fmaf(oax, ax, -omc);
+                        m11 = fmaf(oay, ay, -omc);
+                        m22 = fmaf(oaz, az, -omc);
+                        m01 = fmaf(oax, ay, -saz);
+                        m10 = fmaf(oax, ay, saz);
+                        m02 = fmaf(oax, az, say);
+                        m20 = fmaf(oax, az, -say);
+                        m12 = fmaf(oay, az, -sax);
+                        m21 = fmaf(oay, az, sax);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        if (r > 0 && (uint32_t)r >= rounds) break;
+                        const uint32_t idx = j + r * G;
+                        const uint32_t s = seg_of(idx);
+                        const int ri = RELOAD ? 0 : r;
+                        if (RELOAD) va[0] = Lay::slot(s / SPL, s % SPL, qb);
+                        if (WRAP ? idx < cnt : s < right) {
+                            if (RELOAD) Lay::get(st.t, va[0], vx[0], vy[0], vz[0]);
+                            const float x = vx[ri], y = vy[ri], z = vz[ri];
+                            float nx, ny, nz;
+                            if constexpr (RMAT) {
+                                nx = fmaf(m00, x, fmaf(m01, y, fmaf(m02, z, x)));
+                                ny = fmaf(m10, x, fmaf(m11, y, fmaf(m12, z, y)));
+                                nz = fmaf(m20, x, fmaf(m21, y, fmaf(m22, z, z)));
+                            } else {
+                                const float crx = ay * z - az * y, cry = az * x - ax * z, crz = ax * y - ay * x;
+                                const float ad = (ax * x + ay * y + az * z) * omc;
+                                nx = fmaf(ax, ad, fmaf(sth, crx, fmaf(-omc, x, x)));
+                                ny = fmaf(ay, ad, fmaf(sth, cry, fmaf(-omc, y, y)));
+                                nz = fmaf(az, ad, fmaf(sth, crz, fmaf(-omc, z, z)));
+                            }
+                            const float h = fmaf(renorm, fmaf(nx, nx, fmaf(ny, ny, nz * nz)), 1.5f);
+                            Lay::put(st.t, va[ri], nx * h, ny * h, nz * h);
                         }
-                        const float x = vx[ri], y = vy[ri], z = vz[ri];
-                        float nx, ny, nz;
-                        if constexpr (RMAT) {
-                            nx = fmaf(m00, x, fmaf(m01, y, fmaf(m02, z, x)));
-                            ny = fmaf(m10, x, fmaf(m11, y, fmaf(m12, z, y)));
-                            nz = fmaf(m20, x, fmaf(m21, y, fmaf(m22, z, z)));
-                        } else {
-                            const float crx = ay * z - az * y, cry = az * x - ax * z, crz = ax * y - ay * x;
-                            const float ad = (ax * x + ay * y + az * z) * omc;
-                            nx = fmaf(ax, ad, fmaf(sth, crx, fmaf(-omc, x, x)));
-                            ny = fmaf(ay, ad, fmaf(sth, cry, fmaf(-omc, y, y)));
-                            nz = fmaf(az, ad, fmaf(sth, crz, fmaf(-omc, z, z)));
-                        }
-                        const float h = fmaf(renorm, fmaf(nx, nx, fmaf(ny, ny, nz * nz)), 1.5f);
-                        st.xy[va[ri]] = make_float2(nx * h, ny * h);
-                        st.z[vb[ri]] = nz * h;
                     }
                 }
                 if constexpr (WRAP) {
@@ -815,19 +1135,33 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     tot = inc_tot;
                     ++inc_since_full;
                 } else {
-                    tot = path_fixed<G, SPL, CLAMP, TAB_GLOBAL>(j, gbase, N, s_tab, kc, tan_smem, next_smem, bad, clamped);
+                    bool nan;
+                    uint32_t part = path_fixed<G, SPL, CLAMP, TAB_GLOBAL>(j, N, s_tab, kc, load_smem, next_smem, nan, clamped);
+                    bad = ((__ballot_sync(FULL, nan) >> qb) & Lanes<G>::MASK) != 0u;
                     // a NaN slope marks a steep bin, where the secant would err by more than
                     // 1e-7: weigh such paths (rare) with the exact blend through the linear
                     // table; only a NaN curvature leaves a path invalid
                     if constexpr (STEEP) {
                         if (__any_sync(FULL, bad)) {
-                            const double wx = steep_fallback<G, SPL, CLAMP>(st, gbase, j, N, ma.lin, kc);
+                            const double wx = steep_fallback<G, SPL, CLAMP>(st, qb, j, N, ma.lin, kc);
                             if (bad && !isnan(wx)) {
                                 bad = false;
-                                tot = (unsigned long long)llrint(fmax(0.0, (wx - kc.lw_offset) * (double)kc.fscale));
+                                // the total in shares of at most 32 bits, one per lane
+                                const unsigned long long t =
+                                      (unsigned long long)llrint(fmax(0.0, (wx - kc.lw_offset) * (double)kc.fscale));
+                                part = (uint32_t)(t / G) + (j < (uint32_t)(t % G) ? 1u : 0u);
                             }
                         }
                     }
+                    if constexpr (BATCH) {
+                        const uint32_t slot = wstep & 3u;
+                        flags |= active ? (bad ? 1u : 17u) << slot : 0u;
+                        const bool end = wstep + 1u == c.steps;
+                        batch_step(slot, end, part);
+                        if (end && !(slot & 1u)) batch_step(slot + 1u, true, 0u);
+                        continue;
+                    }
+                    tot = kc.wide ? group_sum<G>((unsigned long long)part) : (unsigned long long)group_sum<G>(part);
                     inc_tot = tot;
                     inc_bad = bad;
                     inc_since_full = 0;
@@ -857,8 +1191,8 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     double ex = px, ey = py, ez = pz;  // inclusive scan of lane totals
 #pragma unroll
                     for (int o = 1; o < G; o <<= 1) {
-                        const double ux = __shfl_up_sync(FULL, ex, o, G), uy = __shfl_up_sync(FULL, ey, o, G),
-                                     uz = __shfl_up_sync(FULL, ez, o, G);
+                        const double ux = __shfl_up_sync(FULL, ex, o * Lanes<G>::STRIDE), uy = __shfl_up_sync(FULL, ey, o * Lanes<G>::STRIDE),
+                                     uz = __shfl_up_sync(FULL, ez, o * Lanes<G>::STRIDE);
                         if ((int)j >= o) { ex += ux; ey += uy; ez += uz; }
                     }
                     ex -= px; ey -= py; ez -= pz;  // exclusive
@@ -882,26 +1216,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     ++failed;
                     continue;
                 }
-                if (valid == 0) {
-                    lse_t = tot;
-                    lse_s = 1.f;
-                    lse_c = 0.f;
-                } else {
-                    // exact integer difference: narrow totals stay below 2^31, wide ones are 64-bit
-                    const float dt = kc.wide ? (float)(long long)(tot - lse_t)
-                                             : (float)(int32_t)((uint32_t)tot - (uint32_t)lse_t);
-                    const float x = dt * kc.l2s;
-                    float term = 1.f;
-                    if (x > 0.f) {
-                        const float f = ex2_approx(-x);
-                        lse_s *= f;
-                        lse_c *= f;
-                        lse_t = tot;
-                    } else {
-                        term = ex2_approx(x);
-                    }
-                    kahan_add(lse_s, lse_c, term);
-                }
+                lse_add(tot);
                 ++valid;
                 continue;
             }
@@ -931,10 +1246,14 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                 };
                 // a chain that fills its group's slots walks them with validity known at compile
                 // time (every curvature but the group's last boundary), as the forward recompute does
+                auto adj_seg2 = [&](uint32_t i0, uint32_t i1, F2 qq, bool v0, bool v1) {
+                    adj_seg(i0, qq.lo(), v0);
+                    adj_seg(i1, qq.hi(), v1);
+                };
                 if (N == (uint32_t)(G * SPL))
-                    for_curvatures<G, SPL, true>(j, N, tan_smem, next_smem, adj_seg);
+                    for_curvatures<G, SPL, true>(j, N, load_smem, next_smem, adj_seg2, adj_seg);
                 else
-                    for_curvatures<G, SPL, false>(j, N, tan_smem, next_smem, adj_seg);
+                    for_curvatures<G, SPL, false>(j, N, load_smem, next_smem, adj_seg2, adj_seg);
                 float hi = s, lo = -cc;
                 group_sum_pair<G>(hi, lo);
                 w = (double)hi + (double)lo;
@@ -956,7 +1275,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     if (j == 0) acc[5] += wt;
                 }
             } else {
-                w = path_log10<G, SPL, true, CLAMP, TAB_GLOBAL>(j, N, s_tab, kc, tan_smem, next_smem, no_bins, clamped);
+                w = path_log10<G, SPL, true, CLAMP, TAB_GLOBAL>(j, N, s_tab, kc, load_smem, next_smem, no_bins, clamped);
             }
             if (MODE == kModeExport && !ma.exp_pos && active && j == 0)   // weights-only replay
                 ma.exp_w[(size_t)chain * c.steps + wstep] = isnan(w) ? NAN : w + (N - 1) * ma.log10_abs;
@@ -975,8 +1294,8 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                 double ex = px, ey = py, ez = pz;
 #pragma unroll
                 for (int o = 1; o < G; o <<= 1) {
-                    const double ux = __shfl_up_sync(FULL, ex, o, G), uy = __shfl_up_sync(FULL, ey, o, G),
-                                 uz = __shfl_up_sync(FULL, ez, o, G);
+                    const double ux = __shfl_up_sync(FULL, ex, o * Lanes<G>::STRIDE), uy = __shfl_up_sync(FULL, ey, o * Lanes<G>::STRIDE),
+                                 uz = __shfl_up_sync(FULL, ez, o * Lanes<G>::STRIDE);
                     if ((int)j >= o) { ex += ux; ey += uy; ez += uz; }
                 }
                 ex -= px; ey -= py; ez -= pz;
@@ -1035,8 +1354,19 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
     double chain_log10 = -INFINITY;
     if (valid) {
         const double head = FIX ? kc.lw_offset + (double)lse_t * kc.inv_scale : (double)lse_m;
-        chain_log10 = head + log10((double)lse_s - (double)lse_c) + (double)(N - 1) * ma.log10_abs;
+        chain_log10 = head + log10((double)lse_s - (double)lse_c);   // -inf in a lane that met no path
     }
+    if constexpr (BATCH) {
+        // the chain's four interleaved sums, lanes j mod 4
+        double m = chain_log10;
+        m = fmax(m, __shfl_xor_sync(FULL, m, LS));
+        m = fmax(m, __shfl_xor_sync(FULL, m, 2 * LS));
+        double x = chain_log10 > -INFINITY ? exp10(chain_log10 - m) : 0.0;
+        x += __shfl_xor_sync(FULL, x, LS);
+        x += __shfl_xor_sync(FULL, x, 2 * LS);
+        chain_log10 = m > -INFINITY ? m + log10(x) : -INFINITY;
+    }
+    if (valid) chain_log10 += (double)(N - 1) * ma.log10_abs;
     if (j == 0 && real_chain && out) {
         ChainOut o;
         o.log10_sum = chain_log10;

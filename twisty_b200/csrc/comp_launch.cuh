@@ -59,12 +59,12 @@ __global__ void __launch_bounds__(MAXT, 1) comp_chain_kernel(ChainSpec c, CompCo
     __syncthreads();
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t q = lane / G, j = lane % G;
+    const uint32_t q = Lanes<G>::chain_of(lane), j = Lanes<G>::lane_of(lane);
     constexpr int CPW = 32 / G;
     const uint32_t chain = (blockIdx.x * warps + warp) * CPW + q;
     unsigned char *wb = s_state + (size_t)warp * Lay::WARP_BYTES;
-    const Planes pl{reinterpret_cast<float2 *>(wb), reinterpret_cast<float *>(wb + Lay::XY_BYTES), s_len};
-    const double cl = chain_body<G, SPL, EXACT, CLAMP, SHIFT, MODE, INCR, STEEP, LUTG>(c, kc, init_seg, s_tab, pl, q * G,
+    const Planes pl{reinterpret_cast<float *>(wb), s_len};
+    const double cl = chain_body<G, SPL, EXACT, CLAMP, SHIFT, MODE, INCR, STEEP, LUTG>(c, kc, init_seg, s_tab, pl, Lanes<G>::base_of(lane),
                                                                                        j, chain, chain < c.n_chains, out,
                                                                                        ma);
     if (j == 0) s_res[warp * CPW + q] = cl;
