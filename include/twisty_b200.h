@@ -48,9 +48,9 @@ typedef enum twisty_status {
 
 /* Arithmetic form of the Markov-chain kernel. */
 typedef enum twisty_form {
-    /* The reference GPU kernel's design (FullExperimentRunnerOptimalPerturbOptimized_GPU.cu:
-     * 689-918): one chain per thread, chain state in global memory, FP32 IEEE
-     * rotate/tangent/curvature, FP64 log10 per segment, CombinedWeightValues_C partials. */
+    /* The reference GPU kernel's arithmetic (FullExperimentRunnerOptimalPerturbOptimized_GPU.cu:
+     * 689-918): FP32 IEEE rotate/tangent/curvature/blend, bit-identical per chain, FP64 path
+     * weights, CombinedWeightValues_C partials; 8 to 32 lanes per chain. */
     TWISTY_FORM_PLAIN_FP32 = 0,
     /* The B200 form: warp-cooperative chains held in shared memory as segment vectors,
      * FP32 tables staged in shared memory, Kahan-compensated FP32 log-weights, log-sum-exp

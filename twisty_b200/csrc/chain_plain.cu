@@ -1,16 +1,14 @@
 // chain_plain.cu -- the plain FP32 drop-in form, the FP64 yardstick form, the FP64 global
 // reduction over chains, and the reference-semantics weigher of given paths.
 //
-// Plain form: the design of the reference's GPU kernel
-// (Twisty/FullExperimentRunnerOptimalPerturbOptimized_GPU.cu:689-918) -- one Markov chain
-// per thread with its positions, tangents and curvatures in global memory (one
-// contiguous block per chain), every tangent and curvature recomputed each step, FP64
-// log10 per segment and a CombinedWeightValues_C accumulator per chain -- with the grid
-// sized for 148 SMs instead of the reference's fixed 128x64 threads, Philox in place of
-// cuRAND, and the reference CPU runner's proposal ranges
-// (Twisty/FullExperimentRunnerOptimalPerturb.cpp:483-519). All FP32 arithmetic is
-// spelled with round-to-nearest intrinsics in the reference's operation order, so a chain
-// here is bit-identical to the same chain run by the CPU oracle.
+// Plain form: the arithmetic of the reference's GPU kernel
+// (Twisty/FullExperimentRunnerOptimalPerturbOptimized_GPU.cu:689-918) -- positions rotated,
+// every tangent and curvature recomputed each step, the float table blended, FP64 log weights and
+// CombinedWeightValues_C accumulators -- with Philox in place of cuRAND and the reference CPU
+// runner's proposal ranges (Twisty/FullExperimentRunnerOptimalPerturb.cpp:483-519). All FP32
+// arithmetic is spelled with round-to-nearest intrinsics in the reference's operation order, so
+// every position, tangent, curvature, bin and blend here is bit-identical to the same chain run
+// by the CPU oracle; only the FP64 sums over segments and paths associate differently.
 #include "kernels.h"
 
 #include <algorithm>
@@ -25,98 +23,249 @@ using dev::CombinedWeight;
 
 constexpr int kPlainThreads = 128;
 
-__global__ void __launch_bounds__(kPlainThreads) plain_chain_kernel(ChainSpec c, const float *__restrict__ init_pos,
-                                                                     float *__restrict__ state,
-                                                                     const float *__restrict__ lut, LutMetaF mf,
-                                                                     ChainOut *__restrict__ out,
-                                                                     float *__restrict__ exp_pos,
-                                                                     double *__restrict__ exp_w)
+// log10 weight of the path at x (planes of stride n_segments + 1), segment by segment in the
+// reference's order and stopping where it stops: for the paths with a segment weight that is not a
+// positive normal number (NaN curvatures, zero or negative table entries), which are rare.
+__device__ __noinline__ bool plain_path_in_order(const float *x, const ChainSpec &c, const float *__restrict__ lut,
+                                                 const dev::LutMeta &m, double &running, uint32_t &clamped)
 {
-    const uint32_t chain = blockIdx.x * blockDim.x + threadIdx.x;
-    if (chain >= c.n_chains) return;
     const uint32_t N = c.n_segments;
-    const size_t stride = plain_state_floats_per_chain(N);
-    float *pos = state + (size_t)chain * stride;  // (N+1)*3
-    float *tan = pos + 3 * (N + 1);               // N*3
-    float *curv = tan + 3 * N;                    // N-1
-    for (uint32_t i = 0; i < 3 * (N + 1); ++i) pos[i] = init_pos[i];
-    const dev::LutMeta m{mf.min_k, mf.max_k, mf.step, mf.bins};
-
-    CombinedWeight cw;
-    dev::cw_reset(cw);
-    uint32_t failed = 0, clamped = 0;
-    const uint32_t steps = (chain == c.n_chains - 1) ? c.last_steps : c.steps;
-    const uint32_t total = c.burn_in + steps;
-    for (uint32_t s = 0; s < total; ++s) {
-        const dev::Proposal pr = dev::draw_step(c.seed, c.experiment, c.chain0 + chain, s, N, c.k_eff, c.max_angle);
-        const uint32_t left = pr.left, right = pr.left + pr.k;
-        const float lx = pos[3 * left], ly = pos[3 * left + 1], lz = pos[3 * left + 2];
-        const float dx = __fsub_rn(pos[3 * right], lx), dy = __fsub_rn(pos[3 * right + 1], ly),
-                    dz = __fsub_rn(pos[3 * right + 2], lz);
-        const float inv = dev::rinvnorm(dx, dy, dz);
-        const float ax = __fmul_rn(dx, inv), ay = __fmul_rn(dy, inv), az = __fmul_rn(dz, inv);
-        float sn, cs;
-        dev::sincos_half(pr.angle, sn, cs);
-        const float q[4] = {cs, __fmul_rn(ax, sn), __fmul_rn(ay, sn), __fmul_rn(az, sn)};
-        for (uint32_t i = left + 1; i < right; ++i) {
-            float x = __fsub_rn(pos[3 * i], lx), y = __fsub_rn(pos[3 * i + 1], ly), z = __fsub_rn(pos[3 * i + 2], lz);
-            dev::rrotate(q, x, y, z);
-            pos[3 * i] = __fadd_rn(x, lx);
-            pos[3 * i + 1] = __fadd_rn(y, ly);
-            pos[3 * i + 2] = __fadd_rn(z, lz);
+    const float *y = x + (N + 1), *z = y + (N + 1);
+    float px = 0.f, py = 0.f, pz = 0.f;
+    running = 0.0;
+    for (uint32_t i = 0; i < N; ++i) {
+        float vx = __fsub_rn(x[i + 1], x[i]), vy = __fsub_rn(y[i + 1], y[i]), vz = __fsub_rn(z[i + 1], z[i]);
+        if (c.has_eval_shift && i == N - 2) {
+            vx = __fadd_rn(vx, c.eval_shift[0]);
+            vy = __fadd_rn(vy, c.eval_shift[1]);
+            vz = __fadd_rn(vz, c.eval_shift[2]);
         }
-        if (s < c.burn_in) continue;
-        // UpdateTangentsFromPos (CurvePerturbUtils.cpp:147-154)
-        for (uint32_t i = 0; i < N; ++i) {
-            float x = __fsub_rn(pos[3 * i + 3], pos[3 * i]), y = __fsub_rn(pos[3 * i + 4], pos[3 * i + 1]),
-                  z = __fsub_rn(pos[3 * i + 5], pos[3 * i + 2]);
-            if (c.has_eval_shift && i == N - 2) {
-                x = __fadd_rn(x, c.eval_shift[0]);
-                y = __fadd_rn(y, c.eval_shift[1]);
-                z = __fadd_rn(z, c.eval_shift[2]);
-            }
-            const float r = dev::rinvnorm(x, y, z);
-            tan[3 * i] = __fmul_rn(x, r);
-            tan[3 * i + 1] = __fmul_rn(y, r);
-            tan[3 * i + 2] = __fmul_rn(z, r);
-        }
-        // UpdateCurvaturesFromTangents_RadiativeTransfer (CurvePerturbUtils.cpp:157-166, bound N-1)
-        for (uint32_t i = 0; i + 1 < N; ++i) {
-            const float x = __fmul_rn(__fsub_rn(tan[3 * i + 3], tan[3 * i]), c.inv_ds);
-            const float y = __fmul_rn(__fsub_rn(tan[3 * i + 4], tan[3 * i + 1]), c.inv_ds);
-            const float z = __fmul_rn(__fsub_rn(tan[3 * i + 5], tan[3 * i + 2]), c.inv_ds);
-            curv[i] = __fsqrt_rn(dev::rdot3(x, y, z));
-        }
-        // WeightCurveViaCurvatureLog10_CudaSafe (PathWeighters.cpp:27-104)
-        double running = 0.0;
-        bool ok = true;
-        for (uint32_t i = 0; i + 1 < N; ++i) {
+        const float r = dev::rinvnorm(vx, vy, vz);
+        const float tx = __fmul_rn(vx, r), ty = __fmul_rn(vy, r), tz = __fmul_rn(vz, r);
+        if (i > 0) {
+            const float kappa = __fsqrt_rn(dev::rdot3(__fmul_rn(__fsub_rn(tx, px), c.inv_ds), __fmul_rn(__fsub_rn(ty, py), c.inv_ds),
+                                                      __fmul_rn(__fsub_rn(tz, pz), c.inv_ds)));
             double blend;
-            if (dev::rbin_blend(curv[i], lut, m, blend, clamped) < 0) { ok = false; break; }
+            if (dev::rbin_blend(kappa, lut, m, blend, clamped) < 0) return false;
             const double lg = log10(blend * c.absorption_factor);
-            if (isnan(lg)) { ok = false; break; }
+            if (isnan(lg)) return false;
             running += lg;
         }
-        if (ok && !isnan(running)) dev::cw_add(cw, running);
-        else ++failed;
-        if (exp_w) {
-            // export replay: every weighted path of this chain, in step order (a weights-only
-            // replay passes no position buffer)
-            const size_t pidx = (size_t)chain * c.steps + (s - c.burn_in);
-            if (exp_pos) {
-                float *dst = exp_pos + pidx * 3 * (size_t)(N + 1);
-                for (uint32_t i = 0; i < 3 * (N + 1); ++i) dst[i] = pos[i];
+        px = tx; py = ty; pz = tz;
+    }
+    return !isnan(running);
+}
+
+// G lanes run one chain, its positions in shared memory as three planes (in `state` in global
+// memory for chains too long for that, SMEM false, G = 32). Lane j takes the points and segments
+// j, j + G, ... of a rotation and of the recompute, so neighbouring lanes read neighbouring points;
+// the previous segment's tangent comes from the lane before by shuffle.
+//  * The path weight is the product of the segment weights: each lane multiplies its
+//    segments' mantissas and adds their exponents, the group combines them, and one FP64 log10 per path
+//    replaces one per segment (a product of n FP64 factors errs by n 2^-53 relative, less than a sum of n logs).
+//  * Lane j finishes the paths of steps j mod G: the log10 and the accumulator's power of ten
+//    run once per G paths in each lane, not once per path in all of them.
+// The first form of this kernel, one thread per chain with its state in global memory, was bound by
+// its strided state traffic and the log10 per segment: the whole experiment of N = 64, 2^20 paths on
+// 16384 chains took 7.20 ms, and takes 0.91 ms with this one.
+template <int G, bool SMEM>
+__global__ void __launch_bounds__(kPlainThreads, 1024 / kPlainThreads)
+plain_chain_kernel(ChainSpec c, const float *__restrict__ init_pos, float *__restrict__ state, uint32_t stride,
+                   const float *__restrict__ lut, LutMetaF mf, ChainOut *__restrict__ out, float *__restrict__ exp_pos,
+                   double *__restrict__ exp_w)
+{
+    extern __shared__ float plain_smem[];
+    const uint32_t j = threadIdx.x % G, slot = threadIdx.x / G;
+    const uint32_t chain = blockIdx.x * (kPlainThreads / G) + slot;
+    const bool real = chain < c.n_chains;
+    if (!SMEM && !real) return;   // a whole warp
+    const uint32_t N = c.n_segments;
+    float *x = SMEM ? plain_smem + (size_t)slot * stride : state + (size_t)chain * stride;
+    float *y = x + (N + 1), *z = y + (N + 1);
+    for (uint32_t i = j; i <= N; i += G) {
+        x[i] = init_pos[3 * i];
+        y[i] = init_pos[3 * i + 1];
+        z[i] = init_pos[3 * i + 2];
+    }
+    const dev::LutMeta m{mf.min_k, mf.max_k, mf.step, mf.bins};
+    const uint32_t gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31u) / G * G);
+    __syncwarp();
+
+    // this lane's paths: the steps j mod G
+    CombinedWeight cw;
+    dev::cw_reset(cw);
+    uint32_t valid = 0, failed = 0, clamped = 0;
+    bool poisoned = false;
+    enum : uint32_t { kNone, kProduct, kSum, kFailed, kZeroFirst, kZero };
+    uint32_t kept = kNone;
+    double kept_w = 0.0;      // kProduct: the mantissas' product, else log10 of the weight
+    int kept_e = 0;
+    bool met = false;         // the chain has met a valid path
+
+    const uint32_t steps = !real ? 0 : (chain == c.n_chains - 1) ? c.last_steps : c.steps;
+    const uint32_t total = c.burn_in + c.steps;
+    for (uint32_t base = 0; base < total; base += G) {
+        const dev::Proposal pr = dev::draw_step(c.seed, c.experiment, c.chain0 + chain, base + j, N, c.k_eff, c.max_angle);
+        float psn, pcs;
+        dev::sincos_half(pr.angle, psn, pcs);
+        const uint32_t nstep = min((uint32_t)G, total - base);
+        for (uint32_t jj = 0; jj < nstep; ++jj) {
+            const uint32_t left = __shfl_sync(0xffffffffu, pr.left, jj, G);
+            const uint32_t right = left + __shfl_sync(0xffffffffu, pr.k, jj, G);
+            const float sn = __shfl_sync(0xffffffffu, psn, jj, G), cs = __shfl_sync(0xffffffffu, pcs, jj, G);
+            const float lx = x[left], ly = y[left], lz = z[left];
+            const float dx = __fsub_rn(x[right], lx), dy = __fsub_rn(y[right], ly), dz = __fsub_rn(z[right], lz);
+            const float inv = dev::rinvnorm(dx, dy, dz);
+            const float ax = __fmul_rn(dx, inv), ay = __fmul_rn(dy, inv), az = __fmul_rn(dz, inv);
+            const float q[4] = {cs, __fmul_rn(ax, sn), __fmul_rn(ay, sn), __fmul_rn(az, sn)};
+            for (uint32_t i = left + 1 + j; i < right; i += G) {
+                float vx = __fsub_rn(x[i], lx), vy = __fsub_rn(y[i], ly), vz = __fsub_rn(z[i], lz);
+                dev::rrotate(q, vx, vy, vz);
+                x[i] = __fadd_rn(vx, lx);
+                y[i] = __fadd_rn(vy, ly);
+                z[i] = __fadd_rn(vz, lz);
             }
-            exp_w[pidx] = (ok && !isnan(running)) ? running : NAN;
+            __syncwarp();
+            if (base + jj < c.burn_in) continue;
+            const uint32_t wstep = base + jj - c.burn_in;
+            const bool active = wstep < steps;
+
+            double prod = 1.0;
+            int esum = 0;
+            bool odd = false;
+            uint32_t cl = 0;
+            float ptx = 0.f, pty = 0.f, ptz = 0.f;   // the tangent of this lane's previous round
+            for (uint32_t r = 0; r * G < N; ++r) {
+                const uint32_t i = r * G + j;
+                const uint32_t at = min(i, N - 1);
+                // UpdateTangentsFromPos (CurvePerturbUtils.cpp:147-154)
+                float vx = __fsub_rn(x[at + 1], x[at]), vy = __fsub_rn(y[at + 1], y[at]), vz = __fsub_rn(z[at + 1], z[at]);
+                if (c.has_eval_shift && at == N - 2) {
+                    vx = __fadd_rn(vx, c.eval_shift[0]);
+                    vy = __fadd_rn(vy, c.eval_shift[1]);
+                    vz = __fadd_rn(vz, c.eval_shift[2]);
+                }
+                const float rn = dev::rinvnorm(vx, vy, vz);
+                const float tx = __fmul_rn(vx, rn), ty = __fmul_rn(vy, rn), tz = __fmul_rn(vz, rn);
+                // tangent i-1: of the lane before, of the last lane's previous round for lane 0
+                const bool last = j == G - 1;
+                const float bx = __shfl_sync(0xffffffffu, last ? ptx : tx, j + G - 1, G);
+                const float by = __shfl_sync(0xffffffffu, last ? pty : ty, j + G - 1, G);
+                const float bz = __shfl_sync(0xffffffffu, last ? ptz : tz, j + G - 1, G);
+                if (i > 0 && i < N) {
+                    // UpdateCurvaturesFromTangents_RadiativeTransfer (CurvePerturbUtils.cpp:157-166, bound N-1)
+                    const float kappa = __fsqrt_rn(dev::rdot3(__fmul_rn(__fsub_rn(tx, bx), c.inv_ds), __fmul_rn(__fsub_rn(ty, by), c.inv_ds),
+                                                              __fmul_rn(__fsub_rn(tz, bz), c.inv_ds)));
+                    // WeightCurveViaCurvatureLog10_CudaSafe (PathWeighters.cpp:27-104)
+                    double blend = 0.0;
+                    const bool nan = dev::rbin_blend(kappa, lut, m, blend, cl) < 0;
+                    const double v = blend * c.absorption_factor;
+                    const int hi = __double2hiint(v);   // sign, exponent, high mantissa bits
+                    odd |= nan || hi < 0x00100000 || hi >= 0x7ff00000;
+                    esum += (hi >> 20) - 1023;
+                    prod *= __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(v));
+                }
+                ptx = tx; pty = ty; ptz = tz;
+                if ((r & 511u) == 511u) {   // 512 mantissas stay below 2^512
+                    esum += (__double2hiint(prod) >> 20) - 1023;
+                    prod = __hiloint2double((__double2hiint(prod) & 0x000fffff) | 0x3ff00000, __double2loint(prod));
+                }
+            }
+            esum += (__double2hiint(prod) >> 20) - 1023;
+            prod = __hiloint2double((__double2hiint(prod) & 0x000fffff) | 0x3ff00000, __double2loint(prod));
+#pragma unroll
+            for (int o = 1; o < G; o <<= 1) {
+                prod *= __shfl_xor_sync(0xffffffffu, prod, o);
+                esum += __shfl_xor_sync(0xffffffffu, esum, o);
+            }
+            uint32_t how = kProduct;
+            if (__ballot_sync(0xffffffffu, odd) & gmask) {
+                double running;
+                cl = 0;
+                const bool ok = plain_path_in_order(x, c, lut, m, running, cl);
+                if (j > 0) cl = 0;   // every lane of the group weighed the same path
+                how = !ok ? kFailed : running > -INFINITY ? kSum : met ? kZero : kZeroFirst;
+                prod = running;
+            }
+            if (active) {
+                clamped += cl;
+                met |= how != kFailed;
+                if (wstep % G == j) {
+                    kept = how;
+                    kept_w = prod;
+                    kept_e = esum;
+                }
+            }
+            if (wstep % G == G - 1 || wstep + 1 == c.steps) {
+                if (kept != kNone) {
+                    const double running = kept == kProduct ? log10(kept_w) + (double)kept_e * 0.30102999566398119521
+                                           : kept == kFailed ? NAN : kept_w;
+                    // a zero weight adds nothing, unless it is the accumulator's first: the
+                    // reference's CombinedWeightValues_C then scales by 10^inf and stays NaN
+                    if (kept == kProduct || kept == kSum) dev::cw_add(cw, running);
+                    if (kept == kFailed) ++failed;
+                    else ++valid;
+                    poisoned |= kept == kZeroFirst;
+                    if (exp_w) exp_w[(size_t)chain * c.steps + (wstep - wstep % G + j)] = running;
+                    kept = kNone;
+                }
+            }
+            if (exp_pos && active) {
+                // export replay: every weighted path of this chain, in step order (a weights-only
+                // replay passes no position buffer)
+                float *dst = exp_pos + ((size_t)chain * c.steps + wstep) * 3 * (size_t)(N + 1);
+                for (uint32_t e = j; e < 3 * (N + 1); e += G) dst[e] = x[(e % 3) * (N + 1) + e / 3];
+            }
+            __syncwarp();
         }
     }
-    ChainOut o;
-    o.log10_sum = dev::cw_log10(cw);
-    o.valid = cw.n;
-    o.failed = failed;
-    o.clamped = clamped;
-    o.pad = 0;
-    out[chain] = o;
+    double part = dev::cw_log10(cw), mx = part;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    double sum = part > -INFINITY ? exp10(part - mx) : 0.0;
+    if (poisoned || isnan(part)) sum = NAN;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        valid += __shfl_xor_sync(0xffffffffu, valid, o);
+        failed += __shfl_xor_sync(0xffffffffu, failed, o);
+        clamped += __shfl_xor_sync(0xffffffffu, clamped, o);
+    }
+    if (j == 0 && real) {
+        ChainOut o;
+        o.log10_sum = mx > -INFINITY || isnan(sum) ? mx + log10(sum) : -INFINITY;
+        o.valid = valid;
+        o.failed = failed;
+        o.clamped = clamped;
+        o.pad = 0;
+        out[chain] = o;
+    }
+}
+
+// Floats of shared memory per chain: three planes of N + 1, padded so that the chains of a warp
+// start G banks apart (G lanes read G consecutive points).
+uint32_t plain_smem_stride(uint32_t n, int G)
+{
+    const uint32_t f = 3 * (n + 1);
+    if (G == 32) return f;
+    return f + ((uint32_t)G + 32u - f % 32u) % 32u;
+}
+
+template <int G, bool SMEM>
+cudaError_t launch_plain_t(const ChainSpec &c, const float *init_pos, float *state, const float *lut, LutMetaF m, ChainOut *out,
+                           cudaStream_t st, float *exp_pos, double *exp_w)
+{
+    constexpr uint32_t per_block = kPlainThreads / G;
+    const uint32_t blocks = (c.n_chains + per_block - 1) / per_block;
+    const uint32_t stride = SMEM ? plain_smem_stride(c.n_segments, G) : (uint32_t)plain_state_floats_per_chain(c.n_segments);
+    const size_t smem = SMEM ? sizeof(float) * (size_t)stride * per_block : 0;
+    auto kern = plain_chain_kernel<G, SMEM>;
+    if (SMEM) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<blocks, kPlainThreads, smem, st>>>(c, init_pos, state, stride, lut, m, out, exp_pos, exp_w);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------
@@ -364,13 +513,23 @@ __global__ void __launch_bounds__(128) weigh_plain_kernel(const float *__restric
 
 }  // namespace
 
+// Lanes per chain: the fewest of 8, 16 and 32 that give an SM at least 768 threads, from the chains
+// of the pass and from those that fit in its shared memory (fewer lanes spend less on the work that
+// every lane of a chain repeats; below 768 threads the latency of a step shows).
 cudaError_t launch_plain_chains(const ChainSpec &c, const float *init_pos, float *state, const float *lut,
                                 LutMetaF m, ChainOut *out, cudaStream_t st, float *exp_pos, double *exp_w)
 {
     if (c.n_chains == 0) return cudaSuccess;
-    const uint32_t blocks = (c.n_chains + kPlainThreads - 1) / kPlainThreads;
-    plain_chain_kernel<<<blocks, kPlainThreads, 0, st>>>(c, init_pos, state, lut, m, out, exp_pos, exp_w);
-    return cudaGetLastError();
+    if (plain_state_floats_per_chain(c.n_segments) > 0)
+        return launch_plain_t<32, false>(c, init_pos, state, lut, m, out, st, exp_pos, exp_w);
+    constexpr uint64_t kSms = 148, kSmem = 227 * 1024;
+    auto threads_per_sm = [&](int G) {
+        const uint64_t fit = kSmem / (sizeof(float) * plain_smem_stride(c.n_segments, G));
+        return std::min<uint64_t>(fit, (c.n_chains + kSms - 1) / kSms) * (uint64_t)G;
+    };
+    if (threads_per_sm(8) >= 768) return launch_plain_t<8, true>(c, init_pos, state, lut, m, out, st, exp_pos, exp_w);
+    if (threads_per_sm(16) >= 768) return launch_plain_t<16, true>(c, init_pos, state, lut, m, out, st, exp_pos, exp_w);
+    return launch_plain_t<32, true>(c, init_pos, state, lut, m, out, st, exp_pos, exp_w);
 }
 
 cudaError_t launch_fp64_chains(const ChainSpec &c, const float *init_pos, double *state, const double *lut,

@@ -89,12 +89,11 @@ cudaError_t launch_comp_tables_batch(uint32_t n, uint32_t bins, const float *lut
 cudaError_t launch_plain_chains(const ChainSpec &c, const float *init_pos, float *state,
                                 const float *lut, LutMetaF m, ChainOut *out, cudaStream_t st,
                                 float *exp_pos = nullptr, double *exp_w = nullptr);
-// Plain-form state of one chain: positions (N+1)*3, tangents N*3, curvatures N-1,
-// padded to a multiple of 4 floats.
+// Floats of global memory per chain of the plain form: none while four chains' positions fit in
+// a CTA's shared memory (N <= 4800), else the positions, (N+1)*3.
 __host__ __device__ inline size_t plain_state_floats_per_chain(uint32_t n)
 {
-    const size_t f = 3 * (size_t)(n + 1) + 3 * (size_t)n + (n - 1);
-    return (f + 3) & ~(size_t)3;
+    return n <= 4800 ? 0 : 3 * ((size_t)n + 1);
 }
 
 cudaError_t launch_fp64_chains(const ChainSpec &c, const float *init_pos, double *state,
