@@ -240,13 +240,25 @@ cudaError_t launch_weigh_comp(const float *pos, uint64_t n_paths, uint32_t n_seg
                               cudaStream_t st, LogFixed lf = LogFixed{0.0, 0.0});
 
 // --------------------------------------------- independent-sample paths (msegment.cu)
+// How the paths are weighed: with the plain weigher's arithmetic and the float table, or the compensated
+// weigher's with the fixed-point table (exact 0) or the linear one.
+struct MSegWeigh {
+    int plain, exact;
+    float inv_ds;
+    double absorption_factor, log10_absorption;
+    LutMetaF meta;
+    LogFixed lf;
+    const float *lut;
+    const float2 *fix, *lin;
+};
+// Threads of a launch; its scratch holds 3 (N+1) floats for each.
+uint32_t msegment_threads(uint32_t n_segments, uint64_t n_paths);
 // n_paths fresh random curves (the reference's recursive bootstrapper, Philox draws keyed by
-// seed and path0 + i) into pos[n_paths][N+1][3]; N - 2 must be resolvable (4, 6, 8, 12, ...).
-cudaError_t launch_msegment_paths(uint32_t n_segments, float ds, const float p0[3], const float p1[3],
-                                  const float pm1[3], const float pm[3], uint64_t seed, uint32_t experiment,
-                                  uint64_t path0, uint64_t n_paths, float *pos, cudaStream_t st);
-// Per-path weights as one ChainOut each (invalid paths: -inf, failed = 1).
-cudaError_t launch_pack_paths(const double *w, const uint8_t *valid, uint64_t n, ChainOut *out, cudaStream_t st);
+// seed and path0 + i), weighed as they are built: one ChainOut each (invalid paths: -inf,
+// failed = 1). N - 2 must be resolvable (4, 6, 8, 12, ...).
+cudaError_t launch_msegment(uint32_t n_segments, float ds, const float p0[3], const float p1[3], const float pm1[3],
+                            const float pm[3], uint64_t seed, uint32_t experiment, uint64_t path0, uint64_t n_paths,
+                            uint32_t threads, const MSegWeigh &wg, float *scratch, ChainOut *out, cudaStream_t st);
 
 // ------------------------------------------------------------ normaliser (norm.cu)
 uint32_t norm_partial_blocks();

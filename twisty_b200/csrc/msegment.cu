@@ -5,17 +5,26 @@
 // (ResolveEvenNumberOfSegments, Twisty/PathGeneration.cpp:47-414) between the fixed points
 // 0, 1, N-1, N, weighed like the Markov-chain paths; the estimate is the mean weight.
 //
-// One thread builds one path, writing its points straight into the path batch in global
-// memory (each point is written once and read back by at most three later placements, through
-// L1). The recursion runs on a small explicit stack in the reference's order (centre point,
-// then the left half, then the right half). The arithmetic follows the reference's mix of float
+// One thread builds and weighs one path at a time. The arithmetic follows the reference's mix of float
 // vectors and double scalars; the random draws come from Philox-4x32-10, counter (draw index,
 // path id lo, path id hi, experiment ^ 'MSEG'), key = seed, one 32-bit output per float draw and
 // two per double draw -- the reference's std::mt19937_64 stream is not reproduced (its
 // threads' interleaving makes it unreproducible anyway). A placement the reference would
-// abort on (spheres that do not intersect, a NaN extent) marks the path invalid (NaN point).
+// abort on (spheres that do not intersect, a NaN extent) marks the path invalid.
+//  * The recursion (centre point, then the left half, then the right half) walks the leaves of a
+//    perfect binary tree: before leaf t come the centres of the spans that begin at it, the largest
+//    first, so the walk needs no stack and every thread of a warp places the same span.
+//  * The reference draws an angle phi = acos(1 - 2u) and uses its sine and cosine only, and the
+//    largest u from cos(asin(a / r)): in double those are 1 - 2u, 2 sqrt(u (1 - u)) and
+//    d / (2r), so a centre costs one sincospi, one cube root, one square root and one
+//    division in FP64 where the angles took two arc functions, three of sine and cosine, a power and four divisions.
+//  * Points go to a scratch column per thread, element by element side by side, so that a warp's
+//    stores and loads are whole lines, and the thread that placed a path weighs it. (Before, each
+//    path's points were 12-byte pieces of its own row in a 1 GB batch, read again by a weigher of its
+//    own: N = 66, 2^21 paths 5.7 ms on the device against 4.2, N = 258, 2^19 paths 6.9 against 4.4.)
 #include "kernels.h"
 #include "device_common.cuh"
+#include "comp_body.cuh"
 
 namespace twisty {
 namespace {
@@ -36,15 +45,43 @@ __device__ __forceinline__ F3 fcross(F3 a, F3 b)
 __device__ __forceinline__ float fmag(F3 a) { return sqrtf(fdot(a, a)); }
 __device__ __forceinline__ F3 funit(F3 a) { return a * (1.0f / sqrtf(fdot(a, a))); }
 
-// Uniform draws from a per-path Philox stream.
+// Uniform draws from a per-path Philox stream. Only the draw index changes between the draws of a path:
+// the half of the first round and the quarter of the second that do not depend on it are kept.
 struct Draws {
-    uint64_t seed;
-    uint32_t path_lo, path_hi, tag;
+    uint32_t k0, k1, tag;
+    uint32_t x0, x1, y2, y3;   // round 1: words 0 and 1; round 2: the products of word 0
     uint32_t n = 0;
-    __device__ uint32_t word()
+    __device__ Draws(uint64_t seed, uint32_t path_lo, uint32_t path_hi, uint32_t t)
+        : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)), tag(t)
     {
-        uint32_t c0 = n++, c1 = path_lo, c2 = path_hi, c3 = tag;
-        dev::philox4x32_10(c0, c1, c2, c3, (uint32_t)seed, (uint32_t)(seed >> 32));
+        const uint64_t a = (uint64_t)0xCD9E8D57u * path_hi;
+        x0 = (uint32_t)(a >> 32) ^ path_lo ^ k0;
+        x1 = (uint32_t)a;
+        const uint64_t b = (uint64_t)0xD2511F53u * x0;
+        y2 = (uint32_t)(b >> 32);
+        y3 = (uint32_t)b;
+    }
+    // the next word: word 0 of the block with counter (n, path lo, path hi, tag)
+    __device__ __forceinline__ uint32_t word()
+    {
+        const uint32_t i = n++;
+        uint32_t a = k0, b = k1;
+        const uint64_t m = (uint64_t)0xD2511F53u * i;
+        const uint32_t z2 = (uint32_t)(m >> 32) ^ tag ^ b, z3 = (uint32_t)m;
+        a += 0x9E3779B9u;
+        b += 0xBB67AE85u;
+        const uint64_t w = (uint64_t)0xCD9E8D57u * z2;
+        uint32_t c0 = (uint32_t)(w >> 32) ^ x1 ^ a, c1 = (uint32_t)w, c2 = y2 ^ z3 ^ b, c3 = y3;
+#pragma unroll
+        for (int r = 2; r < 10; ++r) {
+            a += 0x9E3779B9u;
+            b += 0xBB67AE85u;
+            const uint64_t p = (uint64_t)0xD2511F53u * c0, q = (uint64_t)0xCD9E8D57u * c2;
+            c0 = (uint32_t)(q >> 32) ^ c1 ^ a;
+            c1 = (uint32_t)q;
+            c2 = (uint32_t)(p >> 32) ^ c3 ^ b;
+            c3 = (uint32_t)p;
+        }
         return c0;
     }
     __device__ float uf(float a, float b) { return a + (float)(word() >> 8) * (1.0f / 16777216.0f) * (b - a); }
@@ -57,14 +94,21 @@ struct Draws {
     __device__ int coin() { return (int)(word() & 1u); }
 };
 
+// The path's points: element e = 3 i + k of this thread's column.
 struct PathPts {
-    float *p;  // [N+1][3]
-    __device__ F3 get(uint32_t i) const { return F3{p[3 * i], p[3 * i + 1], p[3 * i + 2]}; }
+    float *p;
+    size_t pitch;   // threads of the launch
+    __device__ F3 get(uint32_t i) const
+    {
+        const float *q = p + 3 * (size_t)i * pitch;
+        return F3{q[0], q[pitch], q[2 * pitch]};
+    }
     __device__ void set(uint32_t i, F3 v) const
     {
-        p[3 * i] = v.x;
-        p[3 * i + 1] = v.y;
-        p[3 * i + 2] = v.z;
+        float *q = p + 3 * (size_t)i * pitch;
+        q[0] = v.x;
+        q[pitch] = v.y;
+        q[2 * pitch] = v.z;
     }
 };
 
@@ -169,8 +213,8 @@ __device__ bool resolve_three(const PathPts &P, uint32_t l, uint32_t r, double d
 }
 
 // The centre point of m segments between l and r (ResolveEvenNumberOfSegments' placement);
-// the halves are handled by the caller.
-__device__ bool place_centre(const PathPts &P, int m, uint32_t l, uint32_t r, double ds, Draws &g)
+// the halves are handled by the caller. inv_h = 2 / m.
+__device__ bool place_centre(const PathPts &P, int m, double inv_h, uint32_t l, uint32_t r, double ds, double inv_ds, Draws &g)
 {
     const int h = m / 2;
     const uint32_t c = l + (uint32_t)h;
@@ -186,32 +230,33 @@ __device__ bool place_centre(const PathPts &P, int m, uint32_t l, uint32_t r, do
     if (d < 0.001f) {
         const double phi = acos(1.0 - 2.0 * g.ud(0.0, 1.0));
         const double theta = g.ud(0.0, (double)(2.0f * kPiF));
-        const double sr = rad * pow((double)g.uf(0.0f, 1.0f), 1.0 / 3.0);
+        const double sr = rad * cbrt((double)g.uf(0.0f, 1.0f));
         frame(a, b, xa, ya, za);
         F3 off = xa * (float)sin(phi) * (float)cos(theta) + ya * (float)sin(phi) * (float)sin(theta) + za * (float)cos(phi);
         P.set(c, a + off * (float)sr);
         return true;
     }
-    const double d2 = d * d;
     const F3 mid = (b + a) * 0.5f;
     const double to_mid = fmag(mid - a);
-    const double aa = sqrt(rad * rad - (0.25 * d2));
-    const double extent = asin(aa / rad);
-    const float umax = (float)(0.5f - cos(extent) * 0.5f);
-    const double phi = acos(1.0 - 2.0 * g.ud(0.0, (double)umax));
+    // cos(asin(sqrt(rad^2 - d^2 / 4) / rad)) = d / (2 rad)
+    const float umax = (float)(0.5 - 0.25 * d * (inv_ds * inv_h));
+    const double u = g.ud(0.0, (double)umax);
+    const double cphi = 1.0 - 2.0 * u, sphi = 2.0 * sqrt(u * (1.0 - u));
     const double theta = g.ud(0.0, (double)(2.0f * kPiF));
     const bool flip = g.coin() != 0;
-    const double hyp = to_mid / cos(phi);
     const double maxr = h * ds;
-    const double minp = hyp / maxr;
-    const double sr = maxr * pow(minp + (1.0f - minp) * (double)g.uf(0.0f, 1.0f), 1.0 / 3.0);
+    const double minp = to_mid / (cphi * maxr);
+    const double sr = maxr * cbrt(minp + (1.0f - minp) * (double)g.uf(0.0f, 1.0f));
     frame(a, b, xa, ya, za);
-    F3 off = xa * (float)sin(phi) * (float)cos(theta) + ya * (float)sin(phi) * (float)sin(theta);
+    double st, ct;
+    sincospi(theta * 0.31830988618379067154, &st, &ct);
+    const float sp = (float)sphi;
+    F3 off = xa * sp * (float)ct + ya * sp * (float)st;
     if (!flip) {
-        off = off + za * (float)cos(phi);
+        off = off + za * (float)cphi;
         P.set(c, a + off * (float)sr);
     } else {
-        off = off + za * (float)cos(phi) * -1.0f;
+        off = off + za * (float)cphi * -1.0f;
         P.set(c, b + off * (float)sr);
     }
     return true;
@@ -227,76 +272,176 @@ struct MSegSpec {
     uint64_t n_paths;
 };
 
-__global__ void __launch_bounds__(128) msegment_paths_kernel(MSegSpec s, float *__restrict__ pos)
+// Places the points of one path; false when the reference would abort.
+__device__ bool build_path(const MSegSpec &s, const PathPts &P, uint64_t path)
 {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= s.n_paths) return;
     const uint32_t N = s.n_segments;
-    const PathPts P{pos + i * 3 * (uint64_t)(N + 1)};
+    Draws g(s.seed, (uint32_t)path, (uint32_t)(path >> 32), s.experiment ^ 0x4D534547u);
+    const double ds = s.ds, inv_ds = 1.0 / ds;
+    // N - 2 = leaf << depth, leaf 4 or 6 (the host validated N - 2 as resolvable)
+    const uint32_t M = N - 2;
+    uint32_t leaf = M, depth = 0;
+    while (leaf > 6) {
+        leaf >>= 1;
+        ++depth;
+    }
+    const double inv_leaf = 2.0 / (double)leaf;
+    for (uint32_t t = 0; t < (1u << depth); ++t) {
+        const uint32_t l = 1 + t * leaf;
+        const int top = t ? __ffs((int)t) - 1 : (int)depth;
+        for (int k = top; k >= 0; --k) {
+            const uint32_t m = leaf << k;
+            // 2 / m = 2 / leaf scaled by 2^-k
+            const double inv_h = __hiloint2double(__double2hiint(inv_leaf) - (k << 20), __double2loint(inv_leaf));
+            if (!place_centre(P, (int)m, inv_h, l, l + m, ds, inv_ds, g)) return false;
+        }
+        const uint32_t c = l + leaf / 2, r = l + leaf;
+        if (leaf == 4 ? !(resolve_two(P, l, c, ds, g) && resolve_two(P, c, r, ds, g))
+                      : !(resolve_three(P, l, c, ds, g) && resolve_three(P, c, r, ds, g)))
+            return false;
+    }
+    return true;
+}
+
+// Walks the curvatures of a path: seg(kappa-like value of the two tangents) until it returns false.
+template <class TanFn, class SegFn>
+__device__ __forceinline__ bool walk_path(const PathPts &P, uint32_t N, TanFn tan, SegFn seg)
+{
+    F3 at = P.get(0), before{0.f, 0.f, 0.f};
+    for (uint32_t i = 0; i < N; ++i) {
+        const F3 next = P.get(i + 1);
+        const F3 t = tan(next, at);
+        if (i > 0 && !seg(t, before)) return false;
+        before = t;
+        at = next;
+    }
+    return true;
+}
+
+// log10 weight of a path with the compensated weigher's arithmetic (path_log10: the same
+// tangents, bins, entries and fractions; the interpolation corrections add up in FP64).
+template <bool EXACT>
+__device__ bool weigh_comp(const PathPts &P, uint32_t N, const CompConsts &kc, const float2 *__restrict__ tab, double &w)
+{
+    unsigned long long isum = 0;
+    double csum = 0.0;
+    float ks = 0.f, kk = 0.f;
+    uint32_t clamped = 0;
+    auto tan = [&](F3 b, F3 a) {
+        const float x = b.x - a.x, y = b.y - a.y, z = b.z - a.z;
+        const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kc.kscale;
+        return F3{x * r, y * r, z * r};
+    };
+    walk_path(P, N, tan, [&](F3 t, F3 b) {
+        const float dx = t.x - b.x, dy = t.y - b.y, dz = t.z - b.z;
+        int32_t L;
+        const float frac = bin_of<true>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), kc, true, clamped, L);
+        const float2 e = tab_load<true>(tab, L);
+        if (EXACT) {
+            kahan_add(ks, kk, __log2f(fmaf(frac * kc.step, e.y, e.x)) * kLog10_2);
+        } else {
+            isum += __float_as_uint(e.x);
+            csum += (double)frac * (double)e.y;
+        }
+        return true;
+    });
+    w = EXACT ? (double)ks - (double)kk : kc.lw_offset + (double)isum * kc.inv_scale + csum;
+    return !isnan(w);
+}
+
+// The same with the plain weigher's arithmetic (weigh_plain_kernel, chain_plain.cu: the
+// reference's FP32 operations), the segment weights multiplied as mantissas and exponents.
+__device__ bool weigh_plain(const PathPts &P, uint32_t N, float inv_ds, const float *__restrict__ lut, const dev::LutMeta &m,
+                            double absorption_factor, double &w)
+{
+    double prod = 1.0, logs = 0.0;
+    int esum = 0;
+    uint32_t clamped = 0;
+    auto tan = [&](F3 b, F3 a) {
+        const float x = __fsub_rn(b.x, a.x), y = __fsub_rn(b.y, a.y), z = __fsub_rn(b.z, a.z);
+        const float r = dev::rinvnorm(x, y, z);
+        return F3{__fmul_rn(x, r), __fmul_rn(y, r), __fmul_rn(z, r)};
+    };
+    auto normalise = [&] {
+        esum += (__double2hiint(prod) >> 20) - 1023;
+        prod = __hiloint2double((__double2hiint(prod) & 0x000fffff) | 0x3ff00000, __double2loint(prod));
+    };
+    const bool ok = walk_path(P, N, tan, [&](F3 t, F3 b) {
+        const float kappa = __fsqrt_rn(dev::rdot3(__fmul_rn(__fsub_rn(t.x, b.x), inv_ds), __fmul_rn(__fsub_rn(t.y, b.y), inv_ds),
+                                                  __fmul_rn(__fsub_rn(t.z, b.z), inv_ds)));
+        double blend = 0.0;
+        if (dev::rbin_blend(kappa, lut, m, blend, clamped) < 0) return false;
+        const double v = __dmul_rn(blend, absorption_factor);
+        const int hi = __double2hiint(v);
+        if (hi < 0x00100000 || hi >= 0x7ff00000) {   // not a positive normal number: rare
+            const double lg = log10(v);
+            logs += lg;
+            return !isnan(lg);
+        }
+        esum += (hi >> 20) - 1023;
+        prod *= __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(v));
+        if (prod >= 1e300) normalise();
+        return true;
+    });
+    if (!ok) return false;
+    w = log10(prod) + (double)esum * 0.30102999566398119521 + logs;
+    return !isnan(w);
+}
+
+constexpr int kMsegThreads = 128;
+
+// FORM 0: the plain weigher; 1: the compensated fixed-point table (a path through a steep bin, or with
+// a NaN curvature, again through the linear one); 2: the linear table. Writes one sample per path.
+template <int FORM>
+__global__ void __launch_bounds__(kMsegThreads, 6)
+msegment_kernel(MSegSpec s, MSegWeigh wg, CompConsts kc, float *__restrict__ scratch, ChainOut *__restrict__ out)
+{
+    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, threads = (size_t)gridDim.x * blockDim.x;
+    const PathPts P{scratch + tid, threads};
+    const uint32_t N = s.n_segments;
     P.set(0, F3{s.p0[0], s.p0[1], s.p0[2]});
     P.set(1, F3{s.p1[0], s.p1[1], s.p1[2]});
     P.set(N - 1, F3{s.pm1[0], s.pm1[1], s.pm1[2]});
     P.set(N, F3{s.pm[0], s.pm[1], s.pm[2]});
-    const uint64_t path = s.path0 + i;
-    Draws g{s.seed, (uint32_t)path, (uint32_t)(path >> 32), s.experiment ^ 0x4D534547u};
-    const double ds = s.ds;
-    // explicit stack of (m, l, r) spans, left half on top (the reference's order)
-    struct Span {
-        int m;
-        uint32_t l, r;
-    };
-    Span stack[40];
-    int top = 0;
-    stack[top++] = Span{(int)N - 2, 1u, N - 1};
-    bool ok = true;
-    while (top > 0 && ok) {
-        const Span sp = stack[--top];
-        ok = place_centre(P, sp.m, sp.l, sp.r, ds, g);
-        if (!ok) break;
-        const int h = sp.m / 2;
-        const uint32_t c = sp.l + (uint32_t)h;
-        if (h == 2) {
-            ok = resolve_two(P, sp.l, c, ds, g) && resolve_two(P, c, sp.r, ds, g);
-        } else if (h == 3) {
-            ok = resolve_three(P, sp.l, c, ds, g) && resolve_three(P, c, sp.r, ds, g);
-        } else {
-            // the host validated N - 2 as resolvable, so h is even and the stack stays
-            // within 2 entries per level of a depth below 20
-            if (top + 2 > 40) {
-                ok = false;
-                break;
+    const dev::LutMeta m{wg.meta.min_k, wg.meta.max_k, wg.meta.step, wg.meta.bins};
+    for (uint64_t i = tid; i < s.n_paths; i += threads) {
+        double w = 0.0;
+        bool ok = build_path(s, P, s.path0 + i);
+        if (ok) {
+            if constexpr (FORM == 0) {
+                ok = weigh_plain(P, N, wg.inv_ds, wg.lut, m, wg.absorption_factor, w);
+            } else {
+                ok = weigh_comp<FORM == 2>(P, N, kc, FORM == 2 ? wg.lin : wg.fix, w);
+                if (FORM == 1 && !ok) ok = weigh_comp<true>(P, N, kc, wg.lin, w);
+                w += (double)(N - 1) * wg.log10_absorption;
             }
-            stack[top++] = Span{h, c, sp.r};
-            stack[top++] = Span{h, sp.l, c};
         }
+        ChainOut o;
+        o.log10_sum = ok ? w : -INFINITY;
+        o.valid = ok ? 1u : 0u;
+        o.failed = ok ? 0u : 1u;
+        o.clamped = 0;
+        o.pad = 0;
+        out[i] = o;
     }
-    if (!ok) {
-        const float nan = __int_as_float(0x7fffffff);
-        P.set(2, F3{nan, nan, nan});
-    }
-}
-
-// Weighed paths as per-path "chains" for the FP64 reduction (independent samples: the
-// spread over them gives the estimate's standard error).
-__global__ void __launch_bounds__(256) pack_paths_kernel(const double *__restrict__ w, const uint8_t *__restrict__ valid,
-                                                         uint64_t n, ChainOut *__restrict__ out)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    ChainOut o;
-    o.log10_sum = valid[i] ? w[i] : -INFINITY;
-    o.valid = valid[i] ? 1u : 0u;
-    o.failed = valid[i] ? 0u : 1u;
-    o.clamped = 0;
-    o.pad = 0;
-    out[i] = o;
 }
 
 }  // namespace
 
-cudaError_t launch_msegment_paths(uint32_t n_segments, float ds, const float p0[3], const float p1[3],
-                                  const float pm1[3], const float pm[3], uint64_t seed, uint32_t experiment,
-                                  uint64_t path0, uint64_t n_paths, float *pos, cudaStream_t st)
+// Threads of a launch: 768 per SM (N = 66, 2^21 paths: 4.03 ms at 768, 4.07 at 1024, 4.35 at 512; the step is
+// bound by issue, 40 k instructions per path, and instruction fetch), fewer while their columns
+// exceed 384 MB (the context keeps them), and no more than there are paths.
+uint32_t msegment_threads(uint32_t n_segments, uint64_t n_paths)
+{
+    constexpr uint64_t kSms = 148;
+    const uint64_t column = 3 * sizeof(float) * (uint64_t)(n_segments + 1);
+    const uint64_t t = std::min({kSms * 768, std::max<uint64_t>((384ull << 20) / column, 1), std::max<uint64_t>(n_paths, 1)});
+    return (uint32_t)((t + kMsegThreads - 1) / kMsegThreads * kMsegThreads);
+}
+
+cudaError_t launch_msegment(uint32_t n_segments, float ds, const float p0[3], const float p1[3], const float pm1[3],
+                            const float pm[3], uint64_t seed, uint32_t experiment, uint64_t path0, uint64_t n_paths,
+                            uint32_t threads, const MSegWeigh &wg, float *scratch, ChainOut *out, cudaStream_t st)
 {
     if (n_paths == 0) return cudaSuccess;
     MSegSpec s{};
@@ -312,15 +457,11 @@ cudaError_t launch_msegment_paths(uint32_t n_segments, float ds, const float p0[
     s.experiment = experiment;
     s.path0 = path0;
     s.n_paths = n_paths;
-    const uint64_t blocks = (n_paths + 127) / 128;
-    msegment_paths_kernel<<<(unsigned)blocks, 128, 0, st>>>(s, pos);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_paths(const double *w, const uint8_t *valid, uint64_t n, ChainOut *out, cudaStream_t st)
-{
-    if (n == 0) return cudaSuccess;
-    pack_paths_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, valid, n, out);
+    const CompConsts kc = make_consts(wg.inv_ds, wg.meta, n_segments, wg.lf);
+    const unsigned blocks = threads / kMsegThreads;
+    if (wg.plain) msegment_kernel<0><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
+    else if (wg.exact || wg.lf.inv_scale == 0.0) msegment_kernel<2><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
+    else msegment_kernel<1><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
     return cudaGetLastError();
 }
 

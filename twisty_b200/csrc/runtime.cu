@@ -95,6 +95,16 @@ struct BatchBufs {
     }
 };
 
+// Workspaces of the M-segment estimator, kept by the context (a column of points per thread of a
+// launch, a sample per path of a launch, its slices).
+struct MSegBufs {
+    DevBuf points, samples, red, slices;
+    void release()
+    {
+        for (DevBuf *b : {&points, &samples, &red, &slices}) b->release();
+    }
+};
+
 // Outputs of the batched adjoint (twisty_adjoint_batch); every pointer nullable but grad.
 struct BatchAdjointOut {
     double *grad;     // [n][5]
@@ -177,6 +187,7 @@ struct twisty_ctx {
     uint32_t kernels_per_launch = 0;
     bool launched = false;
     BatchBufs batch;
+    MSegBufs mseg;
     BatchGraph batch_graph;
 };
 
@@ -990,6 +1001,7 @@ void twisty_destroy(twisty_ctx *ctx)
     for (DevBuf *b : bufs) b->release();
     ctx->batch_graph.release();
     ctx->batch.release();
+    ctx->mseg.release();
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1046,9 +1058,9 @@ twisty_status twisty_run(twisty_ctx *ctx, const twisty_bc *bc, twisty_result *re
 // Independent-sample M-segment Monte Carlo (MSegmentPathGenerationMC,
 // Experiments/ExperimentBase.cpp:1246-1386): fresh random curves from the recursive
 // bootstrapper, weighed with the context's table (plain form: the reference's FP32 semantics;
-// compensated: the fixed-point weigher), the estimate being their mean weight. Paths are built
-// and weighed in chunks of at most 1 GB of positions; each chunk's FP64 reduction treats its
-// paths as independent samples, and the chunks combine by log-sum-exp, errors in quadrature.
+// compensated: the fixed-point weigher), the estimate being their mean weight. Each slice's FP64
+// reduction treats its paths as independent samples, and the slices combine by log-sum-exp,
+// errors in quadrature.
 twisty_status twisty_run_msegment(twisty_ctx *ctx, const twisty_bc *bc, twisty_result *res)
 {
     if (!ctx || !bc || !res) return TWISTY_ERR_INVALID_ARGUMENT;
@@ -1076,80 +1088,74 @@ twisty_status twisty_run_msegment(twisty_ctx *ctx, const twisty_bc *bc, twisty_r
             pm1[k] = ep[k] - ds * ed[k];
         }
         const uint64_t total = p.paths_to_generate;
+        // the samples reduce in slices of kSlice within chunks of `chunk` paths (1 GB of positions), one CTA
+        // each, combined on the host; a launch covers up to kLaunch paths of a chunk
+        constexpr uint64_t kSlice = 16384, kLaunch = 1ull << 21;
         const uint64_t per_path = 3 * sizeof(float) * (uint64_t)(N + 1);
         const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(total, (1ull << 30) / per_path));
-        cudaStream_t st = ctx->stream;
-        DevBuf dpos, dw, dv, dch, dred, drg;
-        struct Release {
-            DevBuf *b[6];
-            ~Release()
-            {
-                for (DevBuf *x : b) x->release();
+        struct Launch {
+            uint64_t path, n;
+            size_t slice;
+            uint32_t n_slices;
+        };
+        std::vector<Launch> launches;
+        std::vector<uint2> slices;
+        for (uint64_t c0 = 0; c0 < total; c0 += chunk) {
+            const uint64_t c1 = std::min(c0 + chunk, total);
+            for (uint64_t l0 = c0; l0 < c1; l0 += kLaunch) {
+                const uint64_t n = std::min(kLaunch, c1 - l0);
+                launches.push_back(Launch{l0, n, slices.size(), (uint32_t)((n + kSlice - 1) / kSlice)});
+                for (uint64_t s0 = 0; s0 < n; s0 += kSlice)
+                    slices.push_back(make_uint2((uint32_t)s0, (uint32_t)std::min(kSlice, n - s0)));
             }
-        } rel{{&dpos, &dw, &dv, &dch, &dred, &drg}};
-        // the samples of a chunk reduce in slices of kSlice, one CTA each, combined on the host
-        constexpr uint64_t kSlice = 16384;
-        const uint64_t max_slices = (chunk + kSlice - 1) / kSlice;
-        ck(dpos.ensure(per_path * chunk), "alloc paths");
-        ck(dw.ensure(sizeof(double) * chunk), "alloc weights");
-        ck(dv.ensure(chunk), "alloc validity");
-        ck(dch.ensure(sizeof(ChainOut) * chunk), "alloc samples");
-        ck(dred.ensure(sizeof(ReduceOut) * max_slices), "alloc result");
-        ck(drg.ensure(sizeof(uint2) * max_slices), "alloc slices");
-        std::vector<uint2> slices(max_slices);
-        for (uint64_t k = 0; k < max_slices; ++k) slices[k] = make_uint2((uint32_t)(k * kSlice), (uint32_t)kSlice);
-        std::vector<ReduceOut> parts(max_slices);
+        }
+        cudaStream_t st = ctx->stream;
+        const uint64_t per_launch = std::min(std::min(chunk, kLaunch), std::max<uint64_t>(total, 1));
+        const uint32_t threads = msegment_threads(N, per_launch);
+        MSegBufs &B = ctx->mseg;
+        ck(B.points.ensure(per_path * threads), "alloc points");
+        ck(B.samples.ensure(sizeof(ChainOut) * per_launch), "alloc samples");
+        ck(B.red.ensure(sizeof(ReduceOut) * std::max<size_t>(1, slices.size())), "alloc result");
+        ck(B.slices.ensure(sizeof(uint2) * std::max<size_t>(1, slices.size())), "alloc slices");
+        std::vector<ReduceOut> parts(slices.size());
         const double af = (double)std::exp(-p.absorption * ds);
-        const float inv_ds = (float)N / bc->arclength;
+        const MSegWeigh wg{p.form == TWISTY_FORM_PLAIN_FP32 ? 1 : 0, ctx->exact_blend, (float)N / bc->arclength, af, std::log10(af),
+                           ctx->meta, ctx->lf, ctx->lut32.as<float>(), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>()};
         const uint64_t seed = seed_of(p.perturb_seed);
         double m = -std::numeric_limits<double>::infinity(), sum = 0.0, var = 0.0;
         uint64_t valid = 0, failed = 0;
         float gpu_ms = 0.f;
-        for (uint64_t done = 0; done < total; done += chunk) {
-            const uint64_t n = std::min(chunk, total - done);
+        if (total) {
+            ck(cudaMemcpyAsync(B.slices.p, slices.data(), sizeof(uint2) * slices.size(), cudaMemcpyHostToDevice, st), "upload slices");
             ck(cudaEventRecord(ctx->ev[0], st), "event");
-            ck(launch_msegment_paths(N, ds, sp, p1, pm1, ep, seed, p.experiment_id, p.chain_offset * total + done, n,
-                                     dpos.as<float>(), st),
-               "path generation");
-            if (p.form == TWISTY_FORM_PLAIN_FP32)
-                ck(launch_weigh_plain(dpos.as<float>(), n, N, inv_ds, ctx->lut32.as<float>(), ctx->meta, af,
-                                      dw.as<double>(), dv.as<uint8_t>(), nullptr, st),
-                   "weigh kernel");
-            else
-                ck(launch_weigh_comp(dpos.as<float>(), n, N, inv_ds, ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
-                                     ctx->exact_blend, ctx->meta, std::log10(af), dw.as<double>(), dv.as<uint8_t>(),
-                                     nullptr, st, ctx->lf),
-                   "weigh kernel");
-            ck(launch_pack_paths(dw.as<double>(), dv.as<uint8_t>(), n, dch.as<ChainOut>(), st), "pack");
-            const uint64_t ns = (n + kSlice - 1) / kSlice;
-            slices[ns - 1].y = (uint32_t)(n - (ns - 1) * kSlice);
-            ck(cudaMemcpyAsync(drg.p, slices.data(), sizeof(uint2) * ns, cudaMemcpyHostToDevice, st), "upload slices");
-            slices[ns - 1].y = (uint32_t)kSlice;
-            ck(launch_reduce_segments(dch.as<ChainOut>(), drg.as<uint2>(), (uint32_t)ns, dred.as<ReduceOut>(), st),
-               "reduction");
+            for (const Launch &l : launches) {
+                ck(launch_msegment(N, ds, sp, p1, pm1, ep, seed, p.experiment_id, p.chain_offset * total + l.path, l.n, threads,
+                                   wg, B.points.as<float>(), B.samples.as<ChainOut>(), st),
+                   "M-segment paths");
+                ck(launch_reduce_segments(B.samples.as<ChainOut>(), B.slices.as<uint2>() + l.slice, l.n_slices,
+                                          B.red.as<ReduceOut>() + l.slice, st),
+                   "reduction");
+            }
             ck(cudaEventRecord(ctx->ev[1], st), "event");
-            ck(cudaMemcpyAsync(parts.data(), dred.p, sizeof(ReduceOut) * ns, cudaMemcpyDeviceToHost, st), "read result");
-            ck(cudaStreamSynchronize(st), "M-segment chunk");
-            float ms = 0.f;
-            ck(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]), "event time");
-            gpu_ms += ms;
-            for (uint64_t k = 0; k < ns; ++k) {
-                const ReduceOut &r = parts[k];
-                valid += r.valid;
-                failed += r.failed;
-                if (r.valid && r.log10_sum > -std::numeric_limits<double>::infinity()) {
-                    // running log-sum-exp of the chunk sums, absolute standard errors in quadrature
-                    const double se = std::isnan(r.rel_se) ? 0.0 : r.rel_se;
-                    if (r.log10_sum > m) {
-                        const double f = std::pow(10.0, m - r.log10_sum);
-                        sum *= f;
-                        var *= f * f;
-                        m = r.log10_sum;
-                    }
-                    const double x = std::pow(10.0, r.log10_sum - m);
-                    sum += x;
-                    var += (se * x) * (se * x);
+            ck(cudaMemcpyAsync(parts.data(), B.red.p, sizeof(ReduceOut) * parts.size(), cudaMemcpyDeviceToHost, st), "read result");
+            ck(cudaStreamSynchronize(st), "M-segment paths");
+            ck(cudaEventElapsedTime(&gpu_ms, ctx->ev[0], ctx->ev[1]), "event time");
+        }
+        for (const ReduceOut &r : parts) {
+            valid += r.valid;
+            failed += r.failed;
+            if (r.valid && r.log10_sum > -std::numeric_limits<double>::infinity()) {
+                // running log-sum-exp of the slice sums, absolute standard errors in quadrature
+                const double se = std::isnan(r.rel_se) ? 0.0 : r.rel_se;
+                if (r.log10_sum > m) {
+                    const double f = std::pow(10.0, m - r.log10_sum);
+                    sum *= f;
+                    var *= f * f;
+                    m = r.log10_sum;
                 }
+                const double x = std::pow(10.0, r.log10_sum - m);
+                sum += x;
+                var += (se * x) * (se * x);
             }
         }
         std::memset(res, 0, sizeof(*res));
