@@ -890,75 +890,4 @@ double norm_k4_log10(float z, float ds)
     return std::log10((double)result);
 }
 
-bool compensated_tables(const float *lut, uint32_t bins, float step, uint32_t n_segments, std::vector<float> &lin,
-                        std::vector<float> &fix, double &c0, double &inv_scale, int &wide, double &secant_err,
-                        uint32_t &steep)
-{
-    wide = 0;
-    lin.assign(2 * (size_t)bins, 0.0f);
-    fix.assign(2 * (size_t)bins, 0.0f);
-    c0 = 0.0;
-    inv_scale = 0.0;
-    secant_err = 0.0;
-    steep = 0;
-    bool positive = true;
-    std::vector<double> lg(bins);
-    std::vector<unsigned char> is_steep(bins, 0);
-    double lo = INFINITY, hi = -INFINITY;
-    const double st = (double)step;
-    for (uint32_t i = 0; i < bins; ++i) {
-        const float a = lut[i], b = lut[i + 1 < bins ? i + 1 : i];
-        lin[2 * i] = a;
-        lin[2 * i + 1] = b - a;
-        if (!(a > 0.0f) || !std::isfinite(a)) {
-            positive = false;
-            continue;
-        }
-        lg[i] = std::log10((double)a);
-        lo = std::min(lo, lg[i]);
-        hi = std::max(hi, lg[i]);
-        if (i + 1 < bins) {
-            const double r = (double)b / (double)a - 1.0;
-            const double e = (st * r) * (st * r) / (8.0 * 2.302585092994046);
-            if (e > kSecantBound) {
-                is_steep[i] = 1;
-                ++steep;
-            } else {
-                secant_err = std::max(secant_err, e);
-            }
-        }
-    }
-    if (!positive) {
-        secant_err = INFINITY;
-        return false;
-    }
-    // largest s (at most 30) with range * 2^s + 65 <= (2^31 - 1) / (n_segments + 1); else the
-    // wide form, range * 2^s + 65 <= (2^32 - 1) / 32
-    const double range = hi - lo;
-    double cap = std::floor(2147483647.0 / (double)(n_segments + 1));
-    int s = 30;
-    while (s > 0 && range * std::ldexp(1.0, s) + 65.0 > cap) --s;
-    if (s < 22) {
-        wide = 1;
-        cap = std::floor(4294967295.0 / 32.0);
-        s = 30;
-        while (s > 0 && range * std::ldexp(1.0, s) + 65.0 > cap) --s;
-    }
-    if (s < 22 || steep > bins / kSteepFraction) {
-        wide = 0;
-        return false;
-    }
-    inv_scale = std::ldexp(1.0, -s);
-    c0 = lo - 64.0 * inv_scale;
-    for (uint32_t i = 0; i < bins; ++i) {
-        const double e = 64.0 + std::nearbyint((lg[i] - lo) * std::ldexp(1.0, s));
-        const uint32_t u = (uint32_t)std::min(e, cap - 1.0);
-        std::memcpy(&fix[2 * i], &u, 4);
-        double delta = 0.0;
-        if (i + 1 < bins) delta = std::log10(1.0 + st * ((double)lut[i + 1] / (double)lut[i] - 1.0));
-        fix[2 * i + 1] = is_steep[i] ? std::numeric_limits<float>::quiet_NaN() : (float)delta;
-    }
-    return true;
-}
-
 }  // namespace twisty

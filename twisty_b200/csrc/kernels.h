@@ -69,9 +69,18 @@ struct LutBuildSpec {
 };
 cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, double *d_mus, double *d_eps,
                              cudaStream_t st);
-// Non-positive entries replaced by the smallest non-negative one (PathWeightUtils.cpp:
-// 327-344); min/max returned through minmax[2]; float copy written to out32.
-cudaError_t launch_lut_finalize(uint32_t bins, double *lut64, float *out32, double *minmax, cudaStream_t st);
+// What a single run's tables came out as: the smallest and largest entry (finalize only), the
+// fixed-point form (LogFixed; inv_scale 0 when the table takes the exact blend), the largest secant
+// error of the bins that are not steep (infinite for a table with non-positive entries).
+struct TableInfo {
+    double min_w, max_w, c0, inv_scale, secant_err;
+    int32_t wide, steep, fixed_ok, nonfinite;
+};
+// finalize: non-positive entries of lut64 replaced by the smallest non-negative one
+// (PathWeightUtils.cpp:327-344) and the float copy written to lut32 (else lut32 is given); then
+// the compensated forms of paths of n_segments (launch_comp_tables_batch's rules).
+cudaError_t launch_single_tables(uint32_t bins, float step, uint32_t n_segments, int finalize, double *lut64, float *lut32, float2 *lin,
+                                 float2 *fix, TableInfo *info, cudaStream_t st);
 // Batches of n tables of `bins` entries, table x at offset x*bins: build (specs in device
 // memory, derivatives off), finalize (minmax + 3x), and the compensated-form tables (struct
 // LogFixed below; steps[x] = bin width, nsegs[x] = N of the paths the fixed point is scaled

@@ -17,6 +17,7 @@
 #include "device_common.cuh"
 
 #include <cfloat>
+#include <cooperative_groups.h>
 #include <math_constants.h>
 
 namespace twisty {
@@ -24,7 +25,7 @@ namespace {
 
 constexpr int kLutThreads = 256;
 // bins whose secant (fixed-point form) errs by more than this per segment are steep; a table
-// with more than bins / kSteepFractionDev of them takes the exact blend (same rule on the host)
+// with more than bins / kSteepFractionDev of them takes the exact blend
 constexpr double kSecantBoundDev = 1e-7;
 constexpr uint32_t kSteepFractionDev = 16;
 
@@ -335,8 +336,7 @@ __global__ void __launch_bounds__(1024) lut_finalize_kernel(uint32_t bins, doubl
     }
 }
 
-// Compensated-form tables of one experiment per CTA, the device twin of the host's
-// compensated_tables (same rules): lin = (L_i, L_{i+1} - L_i); fix = (round((log10 L_i - c0)
+// Compensated-form tables of one experiment per CTA: lin = (L_i, L_{i+1} - L_i); fix = (round((log10 L_i - c0)
 // 2^s) as uint32, log10(1 + step (L_{i+1}/L_i - 1))) with c0 = min log10 L - 64 2^-s and the
 // largest s <= 30 keeping (N+1) (range 2^s + 65) below 2^31, else the wide form with
 // 32 (range 2^s + 65) below 2^32. Bins whose secant error exceeds 1e-7 per segment are
@@ -435,7 +435,148 @@ __global__ void __launch_bounds__(1024) comp_tables_kernel(uint32_t bins, const 
     }
 }
 
+// One table's finalisation and compensated forms in one launch of a cluster: the rules of
+// lut_finalize_kernel (when `finalize`; else lut32 is the table) and of comp_tables_kernel, with
+// the bins spread over kTabCtas SMs -- three FP64 logs a bin are 20 us on one SM at 8192 bins -- and the
+// minima, maxima and counts combined through the cluster's shared memory. A single run used to
+// read its table back, take the logs on the host and upload both forms: 0.15 ms at 4096 bins,
+// 0.5 ms at 20000.
+constexpr int kTabCtas = 8;
+
+struct TabStats {
+    double mn, mx, lo, hi, err;
+    int arg, bad, steep, nonfinite;
+    __device__ __forceinline__ void take(const TabStats &o)
+    {
+        if (o.mn < mn || (o.mn == mn && o.arg < arg)) { mn = o.mn; arg = o.arg; }
+        mx = fmax(mx, o.mx);
+        lo = fmin(lo, o.lo);
+        hi = fmax(hi, o.hi);
+        err = fmax(err, o.err);
+        bad |= o.bad;
+        steep += o.steep;
+        nonfinite |= o.nonfinite;
+    }
+    __device__ __forceinline__ TabStats shuffled(int off) const
+    {
+        constexpr uint32_t F = 0xffffffffu;
+        return TabStats{__shfl_xor_sync(F, mn, off), __shfl_xor_sync(F, mx, off), __shfl_xor_sync(F, lo, off), __shfl_xor_sync(F, hi, off),
+                        __shfl_xor_sync(F, err, off), __shfl_xor_sync(F, arg, off), __shfl_xor_sync(F, bad, off),
+                        __shfl_xor_sync(F, steep, off), __shfl_xor_sync(F, nonfinite, off)};
+    }
+};
+
+// Combines the threads' statistics over the cluster (in every thread). s_cta: this CTA's part, `s_warp` scratch.
+__device__ TabStats cluster_stats(TabStats t, const TabStats &none, TabStats *s_warp, TabStats *s_cta)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    for (int o = 16; o > 0; o >>= 1) t.take(t.shuffled(o));
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) s_warp[w] = t;
+    __syncthreads();
+    if (w == 0) {
+        t = l < (int)(blockDim.x >> 5) ? s_warp[l] : none;
+        for (int o = 16; o > 0; o >>= 1) t.take(t.shuffled(o));
+        if (l == 0) *s_cta = t;
+    }
+    cl.sync();
+    t = *cl.map_shared_rank(s_cta, 0);
+    for (int r = 1; r < kTabCtas; ++r) t.take(*cl.map_shared_rank(s_cta, r));
+    return t;
+}
+
+__global__ void __cluster_dims__(kTabCtas, 1, 1) __launch_bounds__(1024)
+single_tables_kernel(uint32_t bins, float step, uint32_t n_segments, int finalize, double *lut64, float *lut32, float2 *lin, float2 *fix,
+                     TableInfo *info)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ TabStats s_warp[32], s_first, s_second;
+    const uint32_t t0 = cl.block_rank() * blockDim.x + threadIdx.x, tn = kTabCtas * blockDim.x;
+    const double first = finalize ? (double)(float)lut64[0] : 0.0;
+    const TabStats none{first, first, DBL_MAX, -DBL_MAX, 0.0, 0, 0, 0, 0};
+    TabStats a = none;
+    if (finalize) {
+        // min/max selection on the float values, as the reference keeps them; the first entry counts whatever its sign
+        for (uint32_t i = t0; i < bins; i += tn) {
+            const double v = (double)(float)lut64[i];
+            if (i > 0 && v < a.mn && v >= 0.0) { a.mn = v; a.arg = (int)i; }
+            if (i > 0 && v > a.mx && v >= 0.0) a.mx = v;
+        }
+        a = cluster_stats(a, none, s_warp, &s_first);
+        const double mn64 = lut64[a.arg];
+        cl.sync();   // every CTA has the replacement before any writes
+        for (uint32_t i = t0; i < bins; i += tn) {
+            double v = lut64[i];
+            if ((float)v <= 0.0f) v = mn64;
+            lut64[i] = v;
+            lut32[i] = (float)v;
+        }
+        cl.sync();   // a bin's right neighbour may be another CTA's
+    }
+    const double st = (double)step;
+    auto steepness = [&](float x, float y, double &r) {
+        r = (double)y / (double)x - 1.0;
+        return (st * r) * (st * r) / (8.0 * 2.302585092994046);
+    };
+    TabStats b = none;
+    for (uint32_t i = t0; i < bins; i += tn) {
+        const float x = lut32[i], y = lut32[i + 1 < bins ? i + 1 : i];
+        lin[i] = make_float2(x, y - x);
+        if (!isfinite(x)) b.nonfinite = 1;
+        if (!(x > 0.0f) || !isfinite(x)) {
+            b.bad = 1;
+            continue;
+        }
+        const double lg = log10((double)x);
+        b.lo = fmin(b.lo, lg);
+        b.hi = fmax(b.hi, lg);
+        if (i + 1 < bins) {
+            double r;
+            const double e = steepness(x, y, r);
+            if (e > kSecantBoundDev) ++b.steep;
+            else b.err = fmax(b.err, e);
+        }
+    }
+    b = cluster_stats(b, none, s_warp, &s_second);
+    double cap = floor(2147483647.0 / (double)(n_segments + 1));
+    int s = 30;
+    while (s > 0 && (b.hi - b.lo) * ldexp(1.0, s) + 65.0 > cap) --s;
+    int wide = 0;
+    if (s < 22) {
+        wide = 1;
+        cap = floor(4294967295.0 / 32.0);
+        s = 30;
+        while (s > 0 && (b.hi - b.lo) * ldexp(1.0, s) + 65.0 > cap) --s;
+    }
+    const bool usable = !b.bad && (uint32_t)b.steep <= bins / kSteepFractionDev && s >= 22;
+    const double inv_scale = ldexp(1.0, -s);
+    if (t0 == 0)
+        *info = TableInfo{a.mn, a.mx, usable ? b.lo - 64.0 * inv_scale : 0.0, usable ? inv_scale : 0.0, b.bad ? INFINITY : b.err,
+                          usable ? wide : 0, b.steep, usable ? 1 : 0, b.nonfinite};
+    if (usable)
+        for (uint32_t i = t0; i < bins; i += tn) {
+            const float x = lut32[i];
+            const double e = 64.0 + rint((log10((double)x) - b.lo) * ldexp(1.0, s));
+            float delta = 0.0f;
+            if (i + 1 < bins) {
+                double r;
+                delta = steepness(x, lut32[i + 1], r) > kSecantBoundDev ? __int_as_float(0x7fffffff) : (float)log10(1.0 + st * r);
+            }
+            fix[i] = make_float2(__uint_as_float((uint32_t)fmin(e, cap - 1.0)), delta);
+        }
+    cl.sync();   // the CTAs' shared memory stays until everyone has read it
+}
+
 }  // namespace
+
+cudaError_t launch_single_tables(uint32_t bins, float step, uint32_t n_segments, int finalize, double *lut64, float *lut32, float2 *lin,
+                                 float2 *fix, TableInfo *info, cudaStream_t st)
+{
+    single_tables_kernel<<<kTabCtas, 1024, 0, st>>>(bins, step, n_segments, finalize, lut64, lut32, lin, fix, info);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_lut_build_batch(const LutBuildSpec *d_specs, uint32_t n, uint32_t bins, double *out64,
                                    cudaStream_t st)
@@ -471,12 +612,6 @@ cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, double *d_mus
         lut_build_fast_kernel<<<(s.bins + kFastThreads - 1) / kFastThreads, kFastThreads, 0, st>>>(s, out64);
     else
         lut_build_kernel<<<s.bins, kLutThreads, 0, st>>>(s, out64, d_mus, d_eps);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_lut_finalize(uint32_t bins, double *lut64, float *out32, double *minmax, cudaStream_t st)
-{
-    lut_finalize_kernel<<<1, 1024, 0, st>>>(bins, lut64, out32, minmax);
     return cudaGetLastError();
 }
 

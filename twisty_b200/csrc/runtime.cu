@@ -329,13 +329,14 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
     ck(ctx->lut32.ensure(sizeof(float) * bins), "alloc table");
     ck(ctx->fixtab.ensure(sizeof(float2) * bins), "alloc fixed-point table");
     ck(ctx->lintab.ensure(sizeof(float2) * bins), "alloc linear table");
-    ck(ctx->lutaux.ensure(sizeof(double) * 4), "alloc table scratch");
-    std::vector<float> host32(bins);
+    ck(ctx->lutaux.ensure(sizeof(TableInfo)), "alloc table scratch");
+    int finalize = 0;
+    std::vector<float> host32;
     if (p.lut_mode == TWISTY_LUT_MULTI_DS) {
         if (derivatives) fail(TWISTY_ERR_UNSUPPORTED, "derivative tables need lut_mode FP64");
         check_multi(ctx, p);
         const uint32_t i = multi_closest(ctx, ds);
-        std::memcpy(host32.data(), ctx->multi.host.data() + (size_t)i * bins, sizeof(float) * bins);
+        host32.assign(ctx->multi.host.data() + (size_t)i * bins, ctx->multi.host.data() + (size_t)(i + 1) * bins);
         ctx->meta = ctx->multi.meta[i];
         ctx->min_w = ctx->multi.min_w[i];
         ctx->max_w = ctx->multi.max_w[i];
@@ -358,6 +359,7 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
     } else if (p.lut_mode == TWISTY_LUT_FAITHFUL) {
         if (derivatives) fail(TWISTY_ERR_UNSUPPORTED, "derivative tables need lut_mode FP64");
         float mm[2];
+        host32.resize(bins);
         if (!lut_faithful_host(p.mu, p.eps, p.scatter, p.min_bound, p.max_bound, p.bias, p.num_steps_int, bins, ds,
                                host32.data(), mm))
             fail(TWISTY_ERR_INVALID_CONFIG, "invalid table parameters");
@@ -396,36 +398,27 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
             ck(ctx->deps.ensure(sizeof(double) * bins), "alloc derivative table");
         }
         ck(launch_lut_build(s, ctx->lut64.as<double>(), ctx->dmus.as<double>(), ctx->deps.as<double>(), st), "table build");
-        ck(launch_lut_finalize(bins, ctx->lut64.as<double>(), ctx->lut32.as<float>(), ctx->lutaux.as<double>(), st),
-           "table finalize");
-        double mm[3];
-        ck(cudaMemcpyAsync(mm, ctx->lutaux.p, sizeof(double) * 3, cudaMemcpyDeviceToHost, st), "read table range");
-        ck(cudaMemcpyAsync(host32.data(), ctx->lut32.p, sizeof(float) * bins, cudaMemcpyDeviceToHost, st), "read table");
-        ck(cudaStreamSynchronize(st), "table build");
-        ctx->min_w = mm[0];
-        ctx->max_w = mm[1];
+        finalize = 1;
         ctx->meta = LutMetaF{min_k, max_k, step, (int32_t)bins};
     }
-    for (uint32_t i = 0; i < bins; ++i)
-        if (!std::isfinite(host32[i])) fail(TWISTY_ERR_LUT_INVALID, "weight table has non-finite entries");
     // compensated-form tables, the fixed-point one scaled for paths of this N. Bins where the
     // fixed-point secant would err by more than 1e-7 per segment carry a NaN slope (paths
     // crossing them are re-weighed through the linear table); a table with too many of
     // them, or too wide a range, takes the exact blend.
-    std::vector<float> lin, fix;
-    double c0 = 0.0, inv_scale = 0.0, err = 0.0;
-    int wide = 0;
-    uint32_t steep = 0;
-    const bool fixed_ok = compensated_tables(host32.data(), bins, ctx->meta.step, p.num_segments, lin, fix, c0,
-                                             inv_scale, wide, err, steep);
-    ck(cudaMemcpyAsync(ctx->lintab.p, lin.data(), sizeof(float) * lin.size(), cudaMemcpyHostToDevice, st), "upload linear table");
-    if (fixed_ok)
-        ck(cudaMemcpyAsync(ctx->fixtab.p, fix.data(), sizeof(float) * fix.size(), cudaMemcpyHostToDevice, st),
-           "upload fixed-point table");
-    ck(cudaStreamSynchronize(st), "tables");
-    ctx->secant_err = err;
-    ctx->exact_blend = fixed_ok ? 0 : 1;
-    ctx->lf = fixed_ok ? LogFixed{c0, inv_scale, wide, (int32_t)steep} : LogFixed{0.0, 0.0, 0, (int32_t)steep};
+    ck(launch_single_tables(bins, ctx->meta.step, p.num_segments, finalize, ctx->lut64.as<double>(), ctx->lut32.as<float>(),
+                            ctx->lintab.as<float2>(), ctx->fixtab.as<float2>(), ctx->lutaux.as<TableInfo>(), st),
+       "tables");
+    TableInfo ti;
+    ck(cudaMemcpyAsync(&ti, ctx->lutaux.p, sizeof(ti), cudaMemcpyDeviceToHost, st), "read table range");
+    ck(cudaStreamSynchronize(st), "table build");
+    if (ti.nonfinite) fail(TWISTY_ERR_LUT_INVALID, "weight table has non-finite entries");
+    if (finalize) {
+        ctx->min_w = ti.min_w;
+        ctx->max_w = ti.max_w;
+    }
+    ctx->secant_err = ti.secant_err;
+    ctx->exact_blend = ti.fixed_ok ? 0 : 1;
+    ctx->lf = LogFixed{ti.c0, ti.inv_scale, ti.wide, ti.steep};
     std::memcpy(ctx->lut_key, key, sizeof(key));
     ctx->lut_ready = true;
 }
