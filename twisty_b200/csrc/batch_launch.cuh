@@ -23,13 +23,12 @@ struct BatchExp {
     uint32_t pad;
 };
 
-// Per-experiment inputs of the batched adjoint replay beyond BatchExp (whose table is then the
-// linear table, staged in shared memory): the derivative tables with respect to mu_s and eps
-// (launch_deriv_tables layout) and the reference the path weights are scaled by.
+// Per-experiment inputs of the batched adjoint replay beyond BatchExp (whose table is staged in shared
+// memory: the fixed-point one, or the linear one for the exact blend): the derivative tables with
+// respect to mu_s and eps (deriv_tables_kernel) and the reference the path weights are scaled by.
 struct BatchAdjExp {
     const float4 *dtab;
-    float ref_log10;
-    uint32_t pad;
+    double ref_log10;
 };
 
 // Each returns false when the shape is not among its own; else launches (sets e) or reports
@@ -117,10 +116,10 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restri
 }
 
 // Adjoint replay of a batch: the forward pass's work items, each CTA staging its experiment's
-// linear table and running the chains in the adjoint mode of the chain body (exact blend,
-// curvatures recomputed, nothing stored per step); per-chain gradient sums go to
+// table and running the chains in the adjoint mode of the chain body (fixed-point table, or the exact
+// blend; curvatures recomputed, nothing stored per step); per-chain gradient sums go to
 // grad[(out_offset + chain) * 6 ...].
-template <int G, int SPL, int MAXT>
+template <int G, int SPL, bool EXACT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) batch_adjoint_kernel(const BatchExp *__restrict__ exps,
                                                                 const BatchAdjExp *__restrict__ adj,
                                                                 const uint2 *__restrict__ items, uint32_t n_items,
@@ -156,11 +155,25 @@ __global__ void __launch_bounds__(MAXT, 1) batch_adjoint_kernel(const BatchExp *
         ma.ref_log10 = a.ref_log10;
         ma.grad = grad + (size_t)e.out_offset * 6;
         const uint32_t chain = it.y + warp * CPW + q;
-        chain_body<G, SPL, true, true, false, kModeAdjoint>(e.spec, e.kc, e.init_seg,
+        chain_body<G, SPL, EXACT, EXACT, false, kModeAdjoint>(e.spec, e.kc, e.init_seg,
                                                             reinterpret_cast<const float2 *>(smem4), st, Lanes<G>::base_of(lane), j,
                                                             chain, chain < e.spec.n_chains, nullptr, ma);
         __syncthreads();
     }
+}
+
+template <int G, int SPL, bool EXACT>
+cudaError_t batch_adjoint_t(const BatchShape &s, const BatchExp *exps, const BatchAdjExp *adj, const uint2 *items,
+                            uint32_t n_items, uint32_t *counter, double *grad, int bins, int grid, size_t smem,
+                            cudaStream_t st, int *occ)
+{
+    if (s.warps * 32 > kAdjointThreads) return cudaErrorInvalidConfiguration;
+    auto kern = batch_adjoint_kernel<G, SPL, EXACT, kAdjointThreads>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, s.warps * 32, smem);
+    kern<<<grid, s.warps * 32, smem, st>>>(exps, adj, items, n_items, counter, grad, bins);
+    return cudaGetLastError();
 }
 
 template <int G, int SPL>
@@ -168,14 +181,8 @@ cudaError_t batch_adjoint_g(const BatchShape &s, const BatchExp *exps, const Bat
                             uint32_t n_items, uint32_t *counter, double *grad, int bins, int grid, size_t smem,
                             cudaStream_t st, int *occ)
 {
-    constexpr int MAXT = batch_max_threads(G, SPL);
-    if (s.warps * 32 > MAXT) return cudaErrorInvalidConfiguration;
-    auto kern = batch_adjoint_kernel<G, SPL, MAXT>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, s.warps * 32, smem);
-    kern<<<grid, s.warps * 32, smem, st>>>(exps, adj, items, n_items, counter, grad, bins);
-    return cudaGetLastError();
+    return s.exact ? batch_adjoint_t<G, SPL, true>(s, exps, adj, items, n_items, counter, grad, bins, grid, smem, st, occ)
+                   : batch_adjoint_t<G, SPL, false>(s, exps, adj, items, n_items, counter, grad, bins, grid, smem, st, occ);
 }
 
 template <int G, int SPL, bool EXACT, bool LS, bool CL, bool SP>

@@ -73,7 +73,7 @@ cudaError_t launch_mode(int mode, const ChainSpec &c, const CompTuning &t, const
     if (c.has_eval_shift && mode != kModeForward) return cudaErrorInvalidValue;
     if (c.n_chains == 0) return cudaSuccess;
     const bool shift = c.has_eval_shift != 0;
-    const bool exact = t.exact_blend || mode == kModeAdjoint || lf.inv_scale == 0.0 || shift;
+    const bool exact = t.exact_blend || lf.inv_scale == 0.0 || shift;
     const CompConsts kc = make_consts(c.inv_ds, m, c.n_segments, lf);
     const size_t smem = comp_smem_bytes(t, (uint32_t)m.bins);
     const uint32_t blocks = comp_blocks(c, t);
@@ -134,19 +134,6 @@ __global__ void __launch_bounds__(256) grad_reduce_segments_kernel(const double 
     }
 }
 
-// Derivative tables in the linear table's form: per bin (dmu_i, dmu_{i+1} - dmu_i, deps_i,
-// deps_{i+1} - deps_i), the last bin's changes 0; tables of `bins` entries back to back.
-__global__ void deriv_table_kernel(const double *__restrict__ dmu, const double *__restrict__ deps, uint32_t bins,
-                                   size_t n, float4 *__restrict__ out)
-{
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const bool last = (i % bins) == bins - 1;
-        const float m0 = (float)dmu[i], e0 = (float)deps[i];
-        const float m1 = last ? m0 : (float)dmu[i + 1], e1 = last ? e0 : (float)deps[i + 1];
-        out[i] = make_float4(m0, m1 - m0, e0, e1 - e0);
-    }
-}
-
 }  // namespace
 
 cudaError_t launch_grad_reduce_segments(const double *grad_chains, const uint2 *ranges, uint32_t n, double *out,
@@ -156,17 +143,6 @@ cudaError_t launch_grad_reduce_segments(const double *grad_chains, const uint2 *
     grad_reduce_segments_kernel<<<n, 256, 0, st>>>(grad_chains, ranges, out);
     return cudaGetLastError();
 }
-
-cudaError_t launch_deriv_tables(const double *dmu, const double *deps, uint32_t bins, uint32_t n_tables, float4 *out,
-                                cudaStream_t st)
-{
-    const size_t n = (size_t)bins * n_tables;
-    if (n == 0) return cudaSuccess;
-    const size_t blocks = std::min<size_t>((n + 255) / 256, 148 * 16);
-    deriv_table_kernel<<<(unsigned)blocks, 256, 0, st>>>(dmu, deps, bins, n, out);
-    return cudaGetLastError();
-}
-
 
 bool comp_table_needs_clamp(float inv_ds, const LutMetaF &m)
 {
@@ -334,17 +310,25 @@ cudaError_t launch_comp_export(const ChainSpec &c, const CompTuning &t, const fl
     return launch_mode(kModeExport, c, t, init_seg, fixtab, lintab, m, out, nullptr, ma, lf, st);
 }
 
-cudaError_t launch_comp_adjoint(const ChainSpec &c, const CompTuning &t, const float *init_seg, const float2 *lintab,
-                                LutMetaF m, const float4 *dtab, float ref_log10, double *grad_chains, double *grad_out,
-                                cudaStream_t st)
+bool comp_adjoint_fixed(const LogFixed &lf, float inv_ds, const LutMetaF &m)
+{
+    return lf.inv_scale != 0.0 && lf.steep == 0 && !comp_table_needs_clamp(inv_ds, m);
+}
+
+cudaError_t launch_comp_adjoint(const ChainSpec &c, const CompTuning &tuning, const float *init_seg, const float2 *fixtab,
+                                const float2 *lintab, LutMetaF m, const float4 *dtab, double ref_log10, double *grad_chains,
+                                double *grad_out, cudaStream_t st, LogFixed lf)
 {
     ModeArgs ma{};
     ma.log10_abs = log10(c.absorption_factor);
     ma.dtab = dtab;
     ma.ref_log10 = ref_log10;
     ma.grad = grad_chains;
-    cudaError_t e = launch_mode(kModeAdjoint, c, t, init_seg, lintab, lintab, m, nullptr, nullptr, ma,
-                                LogFixed{0.0, 0.0}, st);
+    CompTuning t = tuning;
+    t.warps_per_block = std::min(t.warps_per_block, kAdjointThreads / 32);
+    t.exact_blend = comp_adjoint_fixed(lf, c.inv_ds, m) ? 0 : 1;
+    cudaError_t e = launch_mode(kModeAdjoint, c, t, init_seg, fixtab, lintab, m, nullptr, nullptr, ma,
+                                t.exact_blend ? LogFixed{0.0, 0.0, 0, 0} : lf, st);
     if (e != cudaSuccess) return e;
     grad_reduce_kernel<<<1, 1024, 0, st>>>(grad_chains, c.n_chains, grad_out);
     return cudaGetLastError();

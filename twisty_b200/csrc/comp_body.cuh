@@ -86,10 +86,10 @@ struct ModeArgs {
     float *exp_pos;      // [chains][steps][N+1][3]
     double *exp_w;       // [chains][steps] log10 weights (absorption included, normaliser not)
     float x0[3];
-    // adjoint: per bin (dL/dmu_s, its change to the next bin, dL/deps, its change to the next
-    // bin) -- the derivative tables in the linear table's form, one 16-byte load per segment
+    // adjoint: the derivative tables, one 16-byte load per segment (deriv_tables_kernel: the ratio
+    // form with the fixed-point table, the linear form with the exact blend)
     const float4 *dtab;
-    float ref_log10;     // log10 of the forward sum of path weights (normaliser and absorption excluded)
+    double ref_log10;    // log10 of the forward sum of path weights (normaliser and absorption excluded)
     double *grad;        // [chains][6]: d/dmu_s, d/deps, d/dx, d/dy, d/dz (log10 units), sum of weights
 };
 
@@ -714,7 +714,8 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                                              uint32_t qb, uint32_t j, uint32_t chain, bool real_chain,
                                              ChainOut *__restrict__ out, const ModeArgs &ma)
 {
-    constexpr bool FIX = !EXACT && MODE != kModeAdjoint;
+    constexpr bool FIX = !EXACT;
+    constexpr bool ADJ = MODE == kModeAdjoint;
     const uint32_t N = c.n_segments;
     using Lay = Layout<G, SPL>;
     // segment record (tangent, length) of segment index s = owner*SPL + m
@@ -802,6 +803,10 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
 
     const SmemLoad<G, SPL, SHIFT> load_smem{st, qb, j, N - 2, c.eval_shift, kc.kscale, inv_ks};
     const ShflNext<G> next_smem{};
+    // adjoint with the fixed-point table: the reference as a path total, and the tangents and weight of the
+    // step whose receiver gradient this lane works out
+    const long long adj_ref = ADJ && FIX ? llrint((ma.ref_log10 - kc.lw_offset) * (double)kc.fscale) : 0;
+    [[maybe_unused]] float adj_w = 0.f, adj_t[9] = {};
     // The chain's running log-sum-exp (fixed-point form). It starts from the total 0 with an empty
     // sum: the first path's total is its new maximum.
     auto lse_add = [&](unsigned long long tot) {
@@ -1108,6 +1113,74 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
             const uint32_t wstep = step - c.burn_in;
             const bool active = wstep < steps_c;
 
+            if constexpr (ADJ && FIX) {
+                // The path's total as the forward pass takes it, and beside each table entry the derivatives of its
+                // log in one 16-byte load: two packed operations a segment, where the exact blend takes a log2, a
+                // compensated sum, a reciprocal and two blends. Image replay (48 pixels, N = 512, 2^17 paths
+                // each): 1030 -> 504 warp-instructions per path, 6.76 -> 4.54 ms; the shared-memory and L1 pipe
+                // then binds (92 % of its wavefronts).
+                uint32_t isum = 0;
+                float c0 = 0.f, c1 = 0.f;
+                F2 g = pack2(0.f, 0.f);
+                auto entry = [&](int32_t L, float frac, bool valid, float &cc) {
+                    const float2 en = s_tab[L];
+                    const float4 dv = __ldg(ma.dtab + L);
+                    isum += valid ? __float_as_uint(en.x) : 0u;
+                    const float c2 = fmaf(frac, en.y, cc);
+                    cc = valid ? c2 : cc;
+                    const F2 gn = add2(g, fma2(pack2(frac, frac), pack2(dv.z, dv.w), pack2(dv.x, dv.y)));
+                    g.v = valid ? gn.v : g.v;
+                };
+                auto seg1 = [&](uint32_t, float qq, bool valid) {
+                    int32_t L;
+                    const float frac = bin_of<false>(qq, kc, valid, clamped, L);
+                    entry(L, frac, valid, c0);
+                };
+                auto seg2 = [&](uint32_t, uint32_t, F2 qq, bool v0, bool v1) {
+                    int32_t L0, L1;
+                    const F2 f = bins_of(qq, kc, L0, L1);
+                    entry(L0, f.lo(), v0, c0);
+                    entry(L1, f.hi(), v1, c1);
+                };
+                if (N == (uint32_t)(G * SPL))
+                    for_curvatures<G, SPL, true>(j, N, load_smem, next_smem, seg2, seg1);
+                else
+                    for_curvatures<G, SPL, false>(j, N, load_smem, next_smem, seg2, seg1);
+                const float csum = c0 + c1;
+                const bool bad = ((__ballot_sync(FULL, isnan(csum)) >> qb) & Lanes<G>::MASK) != 0u;
+                isum += (uint32_t)__float2int_rn(csum * kc.fscale);
+                const unsigned long long tot =
+                      kc.wide ? group_sum<G>((unsigned long long)isum) : (unsigned long long)group_sum<G>(isum);
+                const bool use = active && !bad;
+                const float wt = use ? ex2_approx((float)((long long)tot - adj_ref) * kc.l2s) : 0.f;
+                if (use) {
+                    acc[0] = fmaf(wt, g.lo(), acc[0]);
+                    acc[1] = fmaf(wt, g.hi(), acc[1]);
+                    if (j == 0) acc[5] += wt;
+                }
+                // the receiver's part: lane j keeps the last three tangents of the steps j mod G, and
+                // every G steps all lanes work out theirs together
+                if (wstep % G == j) {
+                    adj_w = wt;
+                    Lay::get(st.t, Lay::slot((N - 3) / SPL, (N - 3) % SPL, qb), adj_t[0], adj_t[1], adj_t[2]);
+                    Lay::get(st.t, Lay::slot((N - 2) / SPL, (N - 2) % SPL, qb), adj_t[3], adj_t[4], adj_t[5]);
+                    Lay::get(st.t, Lay::slot((N - 1) / SPL, (N - 1) % SPL, qb), adj_t[6], adj_t[7], adj_t[8]);
+                }
+                if (wstep % G == G - 1 || wstep + 1u == c.steps) {
+                    if (adj_w > 0.f) {
+                        float t3[3], t2[3], t1[3], g3[3];
+                        for (int i = 0; i < 3; ++i) {
+                            t3[i] = adj_t[i] * inv_ks;
+                            t2[i] = adj_t[3 + i] * inv_ks;
+                            t1[i] = adj_t[6 + i] * inv_ks;
+                        }
+                        receiver_grad(t3, t2, t1, st.l[N - 2], ma.lin, kc, c.inv_ds, g3);
+                        for (int i = 0; i < 3; ++i) acc[2 + i] += adj_w * g3[i];
+                    }
+                    adj_w = 0.f;
+                }
+                continue;
+            }
             if (FIX) {
                 bool bad = false;
                 unsigned long long tot = 0;
@@ -1222,7 +1295,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
             }
 
             double w;
-            if (MODE == kModeAdjoint) {
+            if (ADJ) {
                 // log10 weight and d/d(mu_s), d/d(eps) of this lane's segments (exact blend): the
                 // blend from the staged linear table, the derivative blends from one 16-byte load
                 float s = 0.f, cc = 0.f, gmu = 0.f, geps = 0.f;
@@ -1266,7 +1339,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     receiver_grad(t3, t2, t1, v2.w, s_tab, kc, c.inv_ds, g3);
                 }
                 if (active && !isnan(w)) {
-                    const float wt = exp2f((float)(w - (double)ma.ref_log10) * kLog2_10);
+                    const float wt = exp2f((float)(w - ma.ref_log10) * kLog2_10);
                     acc[0] += wt * gmu * kInvLn10;
                     acc[1] += wt * geps * kInvLn10;
                     acc[2] += wt * g3[0];
@@ -1345,7 +1418,11 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
         }
     }
     clamped = group_sum<G>(clamped);
-    if (MODE == kModeAdjoint) {
+    if (ADJ) {
+        if (FIX) {   // the fixed-point form leaves the natural log's factor to the end
+            acc[0] *= kInvLn10;
+            acc[1] *= kInvLn10;
+        }
 #pragma unroll
         for (int i = 0; i < 6; ++i) acc[i] = group_sum<G>(acc[i]);
         if (j == 0 && real_chain)

@@ -89,7 +89,7 @@ template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INC
 cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const float *init_seg, const float2 *tab,
                      ChainOut *out, double2 *partials, const ModeArgs &ma, size_t smem, uint32_t blocks, cudaStream_t st)
 {
-    constexpr int MAXT = comp_max_threads(G, SPL);
+    constexpr int MAXT = MODE == kModeAdjoint ? kAdjointThreads : comp_max_threads(G, SPL);
     if (warps * 32 > MAXT) return cudaErrorInvalidConfiguration;
     auto kern = comp_chain_kernel<G, SPL, EXACT, CLAMP, SHIFT, MAXT, MODE, INCR, STEEP, LUTG>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -107,7 +107,8 @@ cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const 
 }
 
 // Instantiated variants: forward (fixed/exact x clamp/no clamp, plus an exact+clamp+shift
-// variant for receiver-shifted evaluation), export (fixed/exact with clamp), adjoint (exact);
+// variant for receiver-shifted evaluation), export (fixed/exact with clamp), adjoint (fixed without clamp,
+// exact with);
 // the fixed-point forward, incremental and export variants again with the steep-bin fallback;
 // with the table in global memory (lut_global), the forward variants only.
 template <int G, int SPL>
@@ -130,7 +131,8 @@ cudaError_t launch_g(int mode, bool exact, bool clamp, bool shift, bool steep, c
 #define TWISTY_L(E, CL, SH, MO) launch_t<G, SPL, E, CL, SH, MO>(c, kc, w, init_seg, tab, out, partials, ma, smem, blocks, st)
 #define TWISTY_S(CL, MO, IN) \
     launch_t<G, SPL, false, CL, false, MO, IN, true>(c, kc, w, init_seg, tab, out, partials, ma, smem, blocks, st)
-    if (mode == kModeAdjoint) return TWISTY_L(true, true, false, kModeAdjoint);
+    if (mode == kModeAdjoint)
+        return exact ? TWISTY_L(true, true, false, kModeAdjoint) : TWISTY_L(false, false, false, kModeAdjoint);
     if (mode == kModeExport) {
         if (exact) return TWISTY_L(true, true, false, kModeExport);
         return steep ? TWISTY_S(true, kModeExport, false) : TWISTY_L(false, true, false, kModeExport);

@@ -64,11 +64,17 @@ struct LutBuildSpec {
     float ds;
     float min_k, step;       // the float grid (faithful) ...
     double step64;           // ... and its double twin
-    int faithful;
-    int derivatives;         // also d/d(mu_s) and d/d(eps) tables (adjoint)
 };
-cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, double *d_mus, double *d_eps,
-                             cudaStream_t st);
+cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, cudaStream_t st);
+// One derivative table of the adjoint: from specs[spec], into out (one float4 per bin, deriv_tables_kernel);
+// ratio: as derivatives of ln L of the blend over the float table lut.
+struct DerivJob {
+    const float *lut;
+    float4 *out;
+    uint32_t spec;
+    int32_t ratio;
+};
+cudaError_t launch_deriv_tables(const LutBuildSpec *d_specs, const DerivJob *d_jobs, uint32_t n, uint32_t bins, cudaStream_t st);
 // What a single run's tables came out as: the smallest and largest entry (finalize only), the
 // fixed-point form (LogFixed; inv_scale 0 when the table takes the exact blend), the largest secant
 // error of the bins that are not steep (infinite for a table with non-positive entries).
@@ -82,7 +88,7 @@ struct TableInfo {
 cudaError_t launch_single_tables(uint32_t bins, float step, uint32_t n_segments, int finalize, double *lut64, float *lut32, float2 *lin,
                                  float2 *fix, TableInfo *info, cudaStream_t st);
 // Batches of n tables of `bins` entries, table x at offset x*bins: build (specs in device
-// memory, derivatives off), finalize (minmax + 3x), and the compensated-form tables (struct
+// memory, finalize (minmax + 3x), and the compensated-form tables (struct
 // LogFixed below; steps[x] = bin width, nsegs[x] = N of the paths the fixed point is scaled
 // for, ok[x] = 1 when the fixed-point form is usable).
 cudaError_t launch_lut_build_batch(const LutBuildSpec *d_specs, uint32_t n, uint32_t bins, double *out64,
@@ -162,10 +168,15 @@ cudaError_t launch_comp_export(const ChainSpec &c, const CompTuning &t, const fl
                                ChainOut *out, cudaStream_t st, LogFixed lf = LogFixed{0.0, 0.0});
 // Adjoint replay: per chain the weight-averaged gradients of log10 w with respect to
 // (mu_s, eps, receiver x, y, z) and the sum of the weights w/10^ref_log10, reduced over
-// chains into grad_out[6]. dtab: the derivative tables as launch_deriv_tables lays them out.
-cudaError_t launch_comp_adjoint(const ChainSpec &c, const CompTuning &t, const float *init_seg, const float2 *lintab,
-                                LutMetaF m, const float4 *dtab, float ref_log10, double *grad_chains, double *grad_out,
-                                cudaStream_t st);
+// chains into grad_out[6]. dtab: the derivative tables (launch_deriv_tables, `ratio` as comp_adjoint_fixed says).
+cudaError_t launch_comp_adjoint(const ChainSpec &c, const CompTuning &t, const float *init_seg, const float2 *fixtab,
+                                const float2 *lintab, LutMetaF m, const float4 *dtab, double ref_log10, double *grad_chains,
+                                double *grad_out, cudaStream_t st, LogFixed lf);
+// Whether the adjoint replays with the fixed-point table and ratio derivative tables (no steep bins, no
+// clamping), else with the exact blend and linear ones.
+bool comp_adjoint_fixed(const LogFixed &lf, float inv_ds, const LutMetaF &m);
+// Threads per CTA the adjoint kernels are compiled for (80 registers whatever the shape).
+constexpr int kAdjointThreads = 768;
 
 // Batched persistent form: one launch runs the chains of many experiments that share a
 // kernel shape. Work items (experiment, first chain) are taken from *d_counter (zeroed by
@@ -204,15 +215,15 @@ int batch_blocks_per_sm(const BatchShape &s, int bins);
 cudaError_t launch_batch(const BatchShape &s, const void *d_exps, const uint2 *d_items, uint32_t n_items,
                          uint32_t *d_counter, ChainOut *out, int bins, int grid, cudaStream_t st);
 
-// Batched adjoint replay: the experiments packed as for launch_batch (their table being the
-// linear one, staged in shared memory by every shape), plus per experiment its derivative
-// tables (device, launch_deriv_tables layout) and the log10 reference the path weights are
+// Batched adjoint replay: the experiments packed as for launch_batch (their table, fixed-point or, for the
+// shapes with `exact`, linear, staged in shared memory by every shape), plus per experiment its derivative
+// tables (device, launch_deriv_tables) and the log10 reference the path weights are
 // scaled by (the experiment's forward log10 sum without absorption).
 // grad[(out_offset + chain) * 6 + k]: the chain's sums of 10^(w - ref) d log10 w / d (mu_s,
 // eps, receiver x, y, z) and of 10^(w - ref).
 struct BatchAdjHost {
     const float4 *dtab;
-    float ref_log10;
+    double ref_log10;
 };
 size_t batch_adj_bytes();
 void batch_pack_adjoint(const BatchAdjHost *in, uint32_t n, void *dst);
@@ -223,10 +234,6 @@ cudaError_t launch_batch_adjoint(const BatchShape &s, const void *d_exps, const 
 // Per range ranges[x] = (first chain, count): the sums over its chains of the 6 gradient entries.
 cudaError_t launch_grad_reduce_segments(const double *grad_chains, const uint2 *ranges, uint32_t n, double *out,
                                         cudaStream_t st);
-// Derivative tables d/d(mu_s), d/d(eps) (double, n_tables x bins) in the form the adjoint reads:
-// per bin float4 (dmu_i, dmu_{i+1} - dmu_i, deps_i, deps_{i+1} - deps_i).
-cudaError_t launch_deriv_tables(const double *dmu, const double *deps, uint32_t bins, uint32_t n_tables, float4 *out,
-                                cudaStream_t st);
 
 // Path-weight histogram (chain_plain.cu): w[n] log10 path weights (NaN: not counted), counted as
 // 10^(w + log10_norm) into nbins <= 12288 equal buckets over [lo, hi] (outside: the end buckets).

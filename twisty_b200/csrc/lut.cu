@@ -2,13 +2,12 @@
 //
 // The reference builds its table with an OpenMP loop over bins, each bin a composite
 // Simpson quadrature of IntegrandRT whose terms are sorted then summed
-// (Twisty/PathWeightUtils.cpp:281-433). The faithful form and the derivative tables use one
-// CTA per bin: every thread takes a strided share of the nodes and keeps a
-// Neumaier-compensated FP64 sum, and the CTA combines the partial sums pairwise. The plain
-// FP64 form (single tables and batches) uses lut_build_fast_kernel: one thread per bin over
-// node weights shared by all bins (the integrand factors into a bin-independent weight times
-// sin(kds p)). The compensated sums replace the sort (they are at least as accurate), so the
-// float table matches the reference's to within one float ulp rather than bit for bit.
+// (Twisty/PathWeightUtils.cpp:281-433). Here one thread sweeps a bin over node weights that all bins
+// share (the integrand factors into a bin-independent weight times sin(kds p); the derivatives
+// with respect to mu_s and eps into three more weights times its sine and cosine). The
+// compensated sums replace the sort (they are at least as accurate), so the float table
+// matches the reference's to within one float ulp rather than bit for bit (the faithful table
+// mode is built on host threads).
 //
 // The node set keeps the reference's rule exactly: weights h/3 * {1, 4, 2, ..., 4, 2, 1}
 // with the odd loop ending at node n-3 and the even loop at n-4 (nodes n-2 and n-1 are
@@ -23,61 +22,10 @@
 namespace twisty {
 namespace {
 
-constexpr int kLutThreads = 256;
 // bins whose secant (fixed-point form) errs by more than this per segment are steep; a table
 // with more than bins / kSteepFractionDev of them takes the exact blend
 constexpr double kSecantBoundDev = 1e-7;
 constexpr uint32_t kSteepFractionDev = 16;
-
-struct Integrand {
-    double kds, bds, reg, m;   // reg = config mu, m = config eps (phase parameter)
-    int faithful;
-    float np_f;                // float phase normaliser (faithful)
-    double np_d, dlnnp_dm;     // double phase normaliser and its log-derivative in m
-};
-
-__device__ __forceinline__ double phase(const Integrand &g, double p)
-{
-    if (g.faithful) {
-        // GaussianPhase / SimpleGaussianPhase in float (PathWeightUtils.cpp:19-33)
-        const float pf = (float)p, mf = (float)g.m;
-        const float val = __fmul_rn(__fmul_rn(__fmul_rn(-mf, pf), pf), 0.5f);
-        return (double)__fmul_rn(g.np_f, expf(val));
-    }
-    return g.np_d * exp(-g.m * p * p * 0.5);
-}
-
-// f(p) = p exp(bds*phase(p) - reg^2 p^2/2) * sin(kds p)/kds   (IntegrandRT, :350-369)
-__device__ __forceinline__ double integrand(const Integrand &g, double p)
-{
-    const double ph = phase(g, p);
-    const double scattering = p * exp(g.bds * ph - 1.0 * (g.reg * g.reg * p * p * 0.5));
-    return scattering * (g.kds > 0.0 ? sin(g.kds * p) / g.kds : p);
-}
-
-// Derivatives of f (double form): df/dbds, df/dp, df/dm.
-__device__ __forceinline__ void integrand_derivs(const Integrand &g, double p, double &f, double &f_bds,
-                                                 double &f_p, double &f_m)
-{
-    const double ph = g.np_d * exp(-g.m * p * p * 0.5);
-    const double e = exp(g.bds * ph - g.reg * g.reg * p * p * 0.5);
-    double s, sp;
-    if (g.kds > 0.0) {
-        double sn, cs;
-        sincos(g.kds * p, &sn, &cs);
-        s = sn / g.kds;
-        sp = cs;
-    } else {
-        s = p;
-        sp = 1.0;
-    }
-    f = p * e * s;
-    f_bds = f * ph;
-    const double ph_p = -g.m * p * ph;
-    f_p = e * s + p * e * (g.bds * ph_p - g.reg * g.reg * p) * s + p * e * sp;
-    const double ph_m = ph * (g.dlnnp_dm - 0.5 * p * p);
-    f_m = f * g.bds * ph_m;
-}
 
 struct Neumaier {
     double s = 0.0, c = 0.0;
@@ -90,100 +38,7 @@ struct Neumaier {
     __device__ __forceinline__ double value() const { return s + c; }
 };
 
-__device__ double block_sum(double v, double *red)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (w == 0) {
-        r = (l < (int)(blockDim.x >> 5)) ? red[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    }
-    return r;  // valid in thread 0
-}
-
-// One bin of one table, integrated by the whole CTA.
-__device__ __forceinline__ void build_bin(const LutBuildSpec &s, uint32_t bin, double *out64, double *d_mus,
-                                          double *d_eps, double *red)
-{
-    const uint32_t n = s.num_steps_int;
-    Integrand g;
-    g.faithful = s.faithful;
-    g.reg = (double)s.mu;
-    g.m = (double)s.eps;
-    double h, weight, start, maxb, tp;
-    if (s.faithful) {
-        const float kappa = __fadd_rn(s.min_k, __fmul_rn((float)bin, s.step));
-        g.kds = (double)__fmul_rn(kappa, s.ds);
-        g.bds = (double)__fmul_rn(s.scatter, s.ds);
-        g.np_f = __fdiv_rn(__fsqrt_rn(__fmul_rn(__fmul_rn(dev::kPiF, s.eps), 0.5f)),
-                           __fsub_rn(1.0f, expf(__fdiv_rn(-2.0f, s.eps))));
-        h = (double)__fdiv_rn(__fsub_rn(s.max_bound, s.min_bound), (float)n);
-        weight = (double)(1.0f / 3.0f) * h;
-        start = (double)s.min_bound;
-        maxb = (double)s.max_bound;
-        tp = (double)dev::kPiF;
-    } else {
-        const double ds = (double)s.ds;
-        g.kds = (double)bin * s.step64 * ds;
-        g.bds = (double)s.scatter * ds;
-        maxb = 10.0 / (double)s.eps;
-        h = maxb / (double)n;
-        weight = h / 3.0;
-        start = 0.0;
-        tp = CUDART_PI;
-    }
-    const double em = exp(-2.0 / g.m);
-    g.np_d = sqrt((CUDART_PI * g.m) * 0.5) / (1.0 - em);
-    g.dlnnp_dm = 0.5 / g.m - (2.0 / (g.m * g.m)) * em / (1.0 - em);
-
-    Neumaier acc, acc_mus, acc_eps;
-    for (uint32_t j = threadIdx.x; j <= n; j += blockDim.x) {
-        double c;
-        if (j == 0 || j == n) c = 1.0;
-        else if (j >= n - 2) c = 0.0;            // dropped nodes n-2, n-1
-        else c = (j & 1u) ? 4.0 : 2.0;
-        if (c == 0.0) continue;
-        const double p = (j == n) ? maxb : start + (double)j * h;
-        if (s.derivatives && !s.faithful) {
-            double f, f_bds, f_p, f_m;
-            integrand_derivs(g, p, f, f_bds, f_p, f_m);
-            acc.add(c * f);
-            acc_mus.add(c * f_bds);
-            acc_eps.add(c * (-p * f_p / g.m + f_m));
-        } else {
-            acc.add(integrand(g, p) * weight * c);
-        }
-    }
-    const double total = block_sum(acc.value(), red);
-    if (s.derivatives && !s.faithful) {
-        const double t_mus = block_sum(acc_mus.value(), red);
-        const double t_eps = block_sum(acc_eps.value(), red);
-        if (threadIdx.x == 0) {
-            const double scale = weight / (2.0 * tp * tp) * (double)s.bias;
-            const double I = total * scale;
-            out64[bin] = I;
-            // d/d(mu_s): bds = mu_s * ds
-            d_mus[bin] = t_mus * scale * (double)s.ds;
-            // d/d(eps): h and every node move with maxBound = 10/eps
-            d_eps[bin] = -I / g.m + t_eps * scale;
-        }
-    } else if (threadIdx.x == 0) {
-        out64[bin] = (total / (2.0 * tp * tp)) * (double)s.bias;
-    }
-}
-
-__global__ void __launch_bounds__(kLutThreads) lut_build_kernel(LutBuildSpec s, double *out64,
-                                                                 double *d_mus, double *d_eps)
-{
-    __shared__ double red[kLutThreads / 32];
-    build_bin(s, blockIdx.x, out64, d_mus, d_eps, red);
-}
-
-// The FP64 form without derivatives factors: node j contributes w_j sin(kds p_j) / kds with
+// The FP64 form factors: node j contributes w_j sin(kds p_j) / kds with
 // w_j = c_j (h/3) p_j exp(bds phase(p_j) - reg^2 p_j^2 / 2) the same for every bin. A CTA
 // of kFastThreads threads covers that many consecutive bins of one table: it stages w_j for a
 // chunk of nodes in shared memory and each thread sweeps its bin over the chunk, stepping
@@ -191,8 +46,7 @@ __global__ void __launch_bounds__(kLutThreads) lut_build_kernel(LutBuildSpec s, 
 // nodes, so the phase drift stays at the level of the direct argument's own rounding
 // (kds j h carries a relative error of one ulp either way). Runs are summed plainly and
 // folded into a Neumaier total; node n (p = maxBound exactly) is added with a direct sin;
-// bin 0 (kds = 0) takes the limit sin(kds p)/kds -> p. Against the per-node quadrature
-// (lut_build_kernel) it replaces two exp and one sin per node and bin by five FMAs.
+// bin 0 (kds = 0) takes the limit sin(kds p)/kds -> p.
 constexpr int kFastThreads = 128;
 constexpr uint32_t kFastChunk = 1024;
 constexpr uint32_t kRun = 64;
@@ -277,6 +131,116 @@ __global__ void __launch_bounds__(kFastThreads) lut_build_batch_kernel(const Lut
     __shared__ double sw[kFastChunk];
     const LutBuildSpec s = specs[blockIdx.y];
     build_fast(s, blockIdx.x * kFastThreads, out64 + (size_t)blockIdx.y * bins, sw);
+}
+
+// Derivative tables of the adjoint, dL/dmu_s and dL/deps, from the same quadrature differentiated under
+// the integral (the nodes move with maxBound = 10/eps). With e = exp(bds phase(p) - reg^2 p^2 / 2),
+// s = sin(kds p)/kds and g = bds phase'(p) - reg^2 p, node j adds c_j times
+//   w1 s,  w1 = p e                                   to the integral I,
+//   w1 phase s                                        to dI/dbds,
+//   w2 s + w3 cos(kds p),  w2 = p e (bds dphase/deps - (1 + p g)/eps),  w3 = -p^2 e/eps   to dI/deps + I/eps.
+// A thread sweeps one bin, as build_fast does (the first form integrated each bin by a CTA with two
+// exponentials and a sincos per node: 0.13-0.24 ms per 4096-bin table, one launch each).
+// Out: per bin, one float4 of both tables. ratio 0: (dmu_i, dmu_{i+1} - dmu_i, deps_i, deps_{i+1} - deps_i), the form
+// of the linear table. ratio 1: (dmu/L, deps/L) at the bin's left end and their change across the
+// bin, the derivatives of ln L of the blend as chords over the bin: with no steep bin they differ from the
+// quotient of the blends by under (step a)^2/4 < 5e-7 of it, a = L_{i+1}/L_i - 1, and mostly by far less
+// than a float's rounding.
+constexpr int kDerivBins = kFastThreads - 1;   // the last thread of a CTA only serves as a neighbour
+constexpr uint32_t kDerivChunk = 512;
+
+__global__ void __launch_bounds__(kFastThreads)
+deriv_tables_kernel(const LutBuildSpec *__restrict__ specs, const DerivJob *__restrict__ jobs, uint32_t bins)
+{
+    __shared__ double w1[kDerivChunk], w1p[kDerivChunk], w2[kDerivChunk], w3[kDerivChunk];
+    __shared__ double s_mu[kFastThreads], s_eps[kFastThreads];
+    const DerivJob job = jobs[blockIdx.y];
+    const LutBuildSpec s = specs[job.spec];
+    const uint32_t n = s.num_steps_int;
+    const double m = (double)s.eps, reg = (double)s.mu, ds = (double)s.ds, bds = (double)s.scatter * ds;
+    const double maxb = 10.0 / m, h = maxb / (double)n;
+    const double em = exp(-2.0 / m);
+    const double np_d = sqrt((CUDART_PI * m) * 0.5) / (1.0 - em);
+    const double dlnnp = 0.5 / m - (2.0 / (m * m)) * em / (1.0 - em);
+    auto node = [&](double p, double c, double &a1, double &a1p, double &a2, double &a3) {
+        const double ph = np_d * exp(-m * p * p * 0.5);
+        const double e = c * exp(bds * ph - reg * reg * p * p * 0.5);
+        const double g = -bds * m * p * ph - reg * reg * p;
+        a1 = p * e;
+        a1p = a1 * ph;
+        a2 = a1 * (bds * ph * (dlnnp - 0.5 * p * p) - (1.0 + p * g) / m);
+        a3 = -p * p * e / m;
+    };
+    const uint32_t bin = blockIdx.x * kDerivBins + threadIdx.x;
+    const double kds = (double)bin * s.step64 * ds;
+    const bool zero_k = !(kds > 0.0);
+    double st, ct;
+    sincos(kds * h, &st, &ct);
+    uint32_t n_eff = n;   // past p_cut every weight is zero (build_fast)
+    if (reg > 0.0) {
+        const double j_cut = ceil(sqrt(2.0 * (bds * np_d + 750.0)) / reg / h) + 2.0;
+        if (j_cut < (double)n) n_eff = (uint32_t)j_cut;
+    }
+    Neumaier t1, tmu, teps;
+    for (uint32_t c0 = 0; c0 < n_eff; c0 += kDerivChunk) {
+        const uint32_t cn = min(kDerivChunk, n_eff - c0);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < cn; i += blockDim.x) {
+            const uint32_t j = c0 + i;
+            const double c = (j == 0) ? 1.0 : (j >= n - 2) ? 0.0 : ((j & 1u) ? 4.0 : 2.0);
+            node((double)j * h, c, w1[i], w1p[i], w2[i], w3[i]);
+        }
+        __syncthreads();
+        for (uint32_t r0 = 0; r0 < cn; r0 += kRun) {
+            double sn, cs;
+            sincos(kds * ((double)(c0 + r0) * h), &sn, &cs);
+            const uint32_t rn = min(kRun, cn - r0);
+            double r1 = 0.0, rmu = 0.0, r2 = 0.0, r3 = 0.0;
+#pragma unroll 4
+            for (uint32_t i = r0; i < r0 + rn; ++i) {
+                const double q = zero_k ? (double)(c0 + i) * h : sn;   // sin(kds p)/kds -> p
+                r1 = fma(w1[i], q, r1);
+                rmu = fma(w1p[i], q, rmu);
+                r2 = fma(w2[i], q, r2);
+                r3 = fma(w3[i], cs, r3);
+                const double t = fma(sn, ct, cs * st);
+                cs = fma(cs, ct, -(sn * st));
+                sn = t;
+            }
+            const double k = zero_k ? 1.0 : kds;
+            t1.add(r1 / k);
+            tmu.add(rmu / k);
+            teps.add(r2 / k);
+            teps.add(r3);
+        }
+    }
+    {
+        double a1, a1p, a2, a3, sn, cs;
+        node(maxb, 1.0, a1, a1p, a2, a3);
+        sincos(kds * maxb, &sn, &cs);
+        const double q = zero_k ? maxb : sn / kds;
+        t1.add(a1 * q);
+        tmu.add(a1p * q);
+        teps.add(a2 * q);
+        teps.add(a3 * cs);
+    }
+    const double scale = h / 3.0 / (2.0 * CUDART_PI * CUDART_PI) * (double)s.bias;
+    s_mu[threadIdx.x] = tmu.value() * scale * ds;   // bds = mu_s ds
+    s_eps[threadIdx.x] = -(t1.value() * scale) / m + teps.value() * scale;
+    __syncthreads();
+    if (bin >= bins || threadIdx.x == kFastThreads - 1) return;
+    const int right = bin + 1 < bins ? threadIdx.x + 1 : threadIdx.x;
+    const double mu0 = s_mu[threadIdx.x], mu1 = s_mu[right], e0 = s_eps[threadIdx.x], e1 = s_eps[right];
+    float4 o;
+    if (job.ratio) {
+        const double L0 = (double)job.lut[bin], L1 = (double)job.lut[bin + 1 < bins ? bin + 1 : bin], x = (double)s.step;
+        const double end = L0 + x * (L1 - L0);
+        const double am = mu0 / L0, ae = e0 / L0;
+        o = make_float4((float)am, (float)ae, (float)((mu0 + x * (mu1 - mu0)) / end - am), (float)((e0 + x * (e1 - e0)) / end - ae));
+    } else {
+        o = make_float4((float)mu0, (float)mu1 - (float)mu0, (float)e0, (float)e1 - (float)e0);
+    }
+    job.out[bin] = o;
 }
 
 // Replace non-positive entries by the smallest non-negative one and emit the float copy
@@ -605,13 +569,18 @@ cudaError_t launch_comp_tables_batch(uint32_t n, uint32_t bins, const float *lut
     return cudaGetLastError();
 }
 
-cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, double *d_mus, double *d_eps, cudaStream_t st)
+cudaError_t launch_lut_build(const LutBuildSpec &s, double *out64, cudaStream_t st)
 {
     if (s.bins < 2 || s.num_steps_int < 4 || (s.num_steps_int & 1u)) return cudaErrorInvalidValue;
-    if (!s.faithful && !s.derivatives)
-        lut_build_fast_kernel<<<(s.bins + kFastThreads - 1) / kFastThreads, kFastThreads, 0, st>>>(s, out64);
-    else
-        lut_build_kernel<<<s.bins, kLutThreads, 0, st>>>(s, out64, d_mus, d_eps);
+    lut_build_fast_kernel<<<(s.bins + kFastThreads - 1) / kFastThreads, kFastThreads, 0, st>>>(s, out64);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_deriv_tables(const LutBuildSpec *d_specs, const DerivJob *d_jobs, uint32_t n, uint32_t bins, cudaStream_t st)
+{
+    if (n == 0) return cudaSuccess;
+    if (n > 65535u) return cudaErrorInvalidValue;
+    deriv_tables_kernel<<<dim3((bins + kDerivBins - 1) / kDerivBins, n), kFastThreads, 0, st>>>(d_specs, d_jobs, bins);
     return cudaGetLastError();
 }
 

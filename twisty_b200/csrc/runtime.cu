@@ -85,11 +85,11 @@ uint64_t seed_of(uint32_t s)
 // size allocate nothing (DevBuf::ensure only grows). The last row serves the batched adjoint.
 struct BatchBufs {
     DevBuf specs, lut64, lut32, fix, lin, steps, nsegs, lf, ok, init_seg, exps, items, counters, chain_out, ranges, red;
-    DevBuf dtab, d64mu, d64eps, d64scratch, adj_exps, adj_aux, adj_items, adj_counters, grad, grad_sum;
+    DevBuf dtab, djobs, dspecs, adj_exps, adj_aux, adj_items, adj_counters, grad, grad_sum;
     void release()
     {
         DevBuf *all[] = {&specs, &lut64, &lut32, &fix, &lin, &steps, &nsegs, &lf, &ok, &init_seg, &exps, &items,
-                         &counters, &chain_out, &ranges, &red, &dtab, &d64mu, &d64eps, &d64scratch,
+                         &counters, &chain_out, &ranges, &red, &dtab, &djobs, &dspecs,
                          &adj_exps, &adj_aux, &adj_items, &adj_counters, &grad, &grad_sum};
         for (DevBuf *b : all) b->release();
     }
@@ -149,7 +149,7 @@ struct twisty_ctx {
     // tables for the current key
     bool lut_ready = false;
     uint64_t lut_key[4] = {0, 0, 0, 0};
-    DevBuf lut64, lut32, fixtab, lintab, dmus, deps, lutaux;
+    DevBuf lut64, lut32, fixtab, lintab, lutaux;
     LutMetaF meta{};
     double min_w = 0, max_w = 0, secant_err = 0;
     int exact_blend = 0;
@@ -304,7 +304,28 @@ void check_multi(const twisty_ctx *ctx, const twisty_params &p)
         fail(TWISTY_ERR_LUT_INVALID, "the multi-ds tables were built for other weighting parameters");
 }
 
-void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
+// The FP64 table of the parameters at this ds, on the float grid of the WeightLookupTableIntegral ctor
+// (PathWeightUtils.cpp:281-289).
+LutBuildSpec table_spec(const twisty_params &p, float ds)
+{
+    const uint32_t bins = p.num_curvature_steps;
+    LutBuildSpec s{};
+    s.mu = p.mu;
+    s.eps = p.eps;
+    s.scatter = p.scatter;
+    s.min_bound = p.min_bound;
+    s.max_bound = p.max_bound;
+    s.bias = p.bias;
+    s.num_steps_int = p.num_steps_int;
+    s.bins = bins;
+    s.ds = ds;
+    s.min_k = 0.0f;
+    s.step = (float)((2.0 / (double)ds) * (double)1.01f) / (float)(bins - 1);
+    s.step64 = ((2.0 / (double)ds) * 1.01) / (double)(bins - 1);
+    return s;
+}
+
+void build_tables(twisty_ctx *ctx, float ds)
 {
     const twisty_params &p = ctx->p;
     const uint32_t bins = p.num_curvature_steps;
@@ -322,7 +343,7 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
     key[1] = ((uint64_t)f[0] << 32) | f[1];
     key[2] = ((uint64_t)f[2] << 32) | f[3];
     key[3] = ((uint64_t)f[4] << 32) ^ ((uint64_t)f[5]) ^ ((uint64_t)bins << 8) ^ ((uint64_t)p.num_steps_int << 40) ^
-             (derivatives ? 1ull : 0ull) ^ (p.lut_mode == TWISTY_LUT_MULTI_DS ? ((uint64_t)ctx->multi.gen << 1) : 0ull);
+             (p.lut_mode == TWISTY_LUT_MULTI_DS ? ((uint64_t)ctx->multi.gen << 1) : 0ull);
     if (ctx->lut_ready && std::memcmp(key, ctx->lut_key, sizeof(key)) == 0) return;
     ctx->lut_ready = false;
     cudaStream_t st = ctx->stream;
@@ -333,7 +354,6 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
     int finalize = 0;
     std::vector<float> host32;
     if (p.lut_mode == TWISTY_LUT_MULTI_DS) {
-        if (derivatives) fail(TWISTY_ERR_UNSUPPORTED, "derivative tables need lut_mode FP64");
         check_multi(ctx, p);
         const uint32_t i = multi_closest(ctx, ds);
         host32.assign(ctx->multi.host.data() + (size_t)i * bins, ctx->multi.host.data() + (size_t)(i + 1) * bins);
@@ -357,7 +377,6 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
         ck(cudaMemcpyAsync(ctx->lut64.p, h64.data(), sizeof(double) * bins, cudaMemcpyHostToDevice, st), "upload table");
         ck(cudaStreamSynchronize(st), "sync");
     } else if (p.lut_mode == TWISTY_LUT_FAITHFUL) {
-        if (derivatives) fail(TWISTY_ERR_UNSUPPORTED, "derivative tables need lut_mode FP64");
         float mm[2];
         host32.resize(bins);
         if (!lut_faithful_host(p.mu, p.eps, p.scatter, p.min_bound, p.max_bound, p.bias, p.num_steps_int, bins, ds,
@@ -373,33 +392,11 @@ void build_tables(twisty_ctx *ctx, float ds, bool derivatives)
         ck(cudaMemcpyAsync(ctx->lut64.p, h64.data(), sizeof(double) * bins, cudaMemcpyHostToDevice, st), "upload table");
         ck(cudaStreamSynchronize(st), "sync");
     } else {
-        // WeightLookupTableIntegral ctor (PathWeightUtils.cpp:281-289), float grid
-        const float min_k = 0.0f;
-        const float max_k = (float)((2.0 / (double)ds) * (double)1.01f);
-        const float step = (max_k - min_k) / (float)(bins - 1);
-        LutBuildSpec s{};
-        s.mu = p.mu;
-        s.eps = p.eps;
-        s.scatter = p.scatter;
-        s.min_bound = p.min_bound;
-        s.max_bound = p.max_bound;
-        s.bias = p.bias;
-        s.num_steps_int = p.num_steps_int;
-        s.bins = bins;
-        s.ds = ds;
-        s.min_k = min_k;
-        s.step = step;
-        s.step64 = ((2.0 / (double)ds) * 1.01) / (double)(bins - 1);
-        s.faithful = 0;
-        s.derivatives = derivatives ? 1 : 0;
+        const LutBuildSpec s = table_spec(p, ds);
         ck(ctx->lut64.ensure(sizeof(double) * bins), "alloc table");
-        if (derivatives) {
-            ck(ctx->dmus.ensure(sizeof(double) * bins), "alloc derivative table");
-            ck(ctx->deps.ensure(sizeof(double) * bins), "alloc derivative table");
-        }
-        ck(launch_lut_build(s, ctx->lut64.as<double>(), ctx->dmus.as<double>(), ctx->deps.as<double>(), st), "table build");
+        ck(launch_lut_build(s, ctx->lut64.as<double>(), st), "table build");
         finalize = 1;
-        ctx->meta = LutMetaF{min_k, max_k, step, (int32_t)bins};
+        ctx->meta = LutMetaF{0.0f, (float)((2.0 / (double)ds) * (double)1.01f), s.step, (int32_t)bins};
     }
     // compensated-form tables, the fixed-point one scaled for paths of this N. Bins where the
     // fixed-point secant would err by more than 1e-7 per segment carry a NaN slope (paths
@@ -500,7 +497,7 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
     const twisty_bc bc = *bcp;
     const uint32_t N = p.num_segments;
     const float ds = bc.arclength / (float)N;
-    build_tables(ctx, ds, false);
+    build_tables(ctx, ds);
     ctx->log10_norm = normalizer_log10(ctx, N, ds, bc);
     // initial curve
     std::vector<float> pos;
@@ -620,7 +617,7 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
             ctx->lut_ready = false;
             twisty_params saved = ctx->p;
             ctx->p.lut_mode = TWISTY_LUT_FP64;
-            build_tables(ctx, ds, false);
+            build_tables(ctx, ds);
             ctx->p = saved;
         }
     } else {
@@ -988,7 +985,7 @@ void twisty_destroy(twisty_ctx *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    DevBuf *bufs[] = {&ctx->lut64, &ctx->lut32, &ctx->fixtab, &ctx->lintab, &ctx->dmus, &ctx->deps, &ctx->lutaux,
+    DevBuf *bufs[] = {&ctx->lut64, &ctx->lut32, &ctx->fixtab, &ctx->lintab, &ctx->lutaux,
                       &ctx->init_pos, &ctx->init_seg, &ctx->state, &ctx->chain_out, &ctx->partials, &ctx->reduce_out,
                       &ctx->norm_scratch, &ctx->multi.dev, &ctx->check_state, &ctx->check_out};
     for (DevBuf *b : bufs) b->release();
@@ -1068,7 +1065,7 @@ twisty_status twisty_run_msegment(twisty_ctx *ctx, const twisty_bc *bc, twisty_r
             fail(TWISTY_ERR_UNSUPPORTED, "M-segment paths come from the recursive bootstrapper: N-2 in {4, 6, 8, 12, 16, 24, 32, 48, ...}");
         set_device(ctx);
         const float ds = bc->arclength / (float)N;
-        build_tables(ctx, ds, false);
+        build_tables(ctx, ds);
         const double log10_norm = normalizer_log10(ctx, N, ds, *bc);
         // the fixed points (ExperimentBase.cpp:1253-1260)
         const float sp[3] = {bc->start_pos.x, bc->start_pos.y, bc->start_pos.z};
@@ -1179,7 +1176,7 @@ twisty_status twisty_weight_paths(twisty_ctx *ctx, const twisty_bc *bc, const fl
         set_device(ctx);
         const uint32_t N = ctx->p.num_segments;
         const float ds = bc->arclength / (float)N;
-        build_tables(ctx, ds, false);
+        build_tables(ctx, ds);
         if (n_paths == 0) return;
         cudaStream_t st = ctx->stream;
         DevBuf dpos, dw, dv, db;
@@ -1223,7 +1220,7 @@ twisty_status twisty_build_lut(twisty_ctx *ctx, float ds, float *lut, twisty_lut
     return guard(ctx, [&] {
         validate(ctx->p);
         set_device(ctx);
-        build_tables(ctx, ds, false);
+        build_tables(ctx, ds);
         if (lut) {
             ck(cudaMemcpyAsync(lut, ctx->lut32.p, sizeof(float) * ctx->p.num_curvature_steps, cudaMemcpyDeviceToHost,
                                ctx->stream), "read table");
@@ -1693,43 +1690,29 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
     // table of the multi-ds set the experiments take theirs from
     const uint32_t ntab = multi ? ctx->multi.n : n;
     ck(B.dtab.ensure(sizeof(float4) * (size_t)bins * ntab), "alloc derivative tables");
-    ck(B.d64mu.ensure(sizeof(double) * (size_t)bins * ntab), "alloc derivative tables");
-    ck(B.d64eps.ensure(sizeof(double) * (size_t)bins * ntab), "alloc derivative tables");
-    ck(B.d64scratch.ensure(sizeof(double) * (size_t)bins), "alloc derivative tables");
-    std::vector<char> tab_used(ntab, multi ? 0 : 1);
-    if (multi)
-        for (uint32_t e = 0; e < n; ++e) tab_used[eh[e].multi_index] = 1;
-    ck(cudaEventRecord(ctx->ev[0], st), "event");
-    for (uint32_t t = 0; t < ntab; ++t) {
-        if (!tab_used[t]) continue;
-        LutBuildSpec s{};
-        if (multi) {
-            s.mu = p.mu;
-            s.eps = p.eps;
-            s.scatter = p.scatter;
-            s.min_bound = p.min_bound;
-            s.max_bound = p.max_bound;
-            s.bias = p.bias;
-            s.num_steps_int = p.num_steps_int;
-            s.bins = bins;
-            s.ds = ctx->multi.ds[t];
-            s.min_k = 0.0f;
-            s.step = ctx->multi.meta[t].step;
-            s.step64 = ((2.0 / (double)s.ds) * 1.01) / (double)(bins - 1);
-        } else {
-            s = specs[t];
-        }
-        s.faithful = 0;
-        s.derivatives = 1;
-        ck(launch_lut_build(s, B.d64scratch.as<double>(), B.d64mu.as<double>() + (size_t)t * bins,
-                            B.d64eps.as<double>() + (size_t)t * bins, st),
-           "derivative tables");
+    // the replay takes the fixed-point table where it has no steep bins (the same for all
+    // experiments of a table: steepness and range are the table's)
+    auto fixed_of = [&](uint32_t e) { return okv[e] != 0 && comp_adjoint_fixed(lf[e], eh[e].spec.inv_ds, eh[e].meta); };
+    std::vector<DerivJob> jobs;
+    std::vector<LutBuildSpec> dspecs;
+    std::vector<char> have(ntab, 0);
+    for (uint32_t e = 0; e < n; ++e) {
+        const uint32_t t = multi ? eh[e].multi_index : e;
+        if (have[t]) continue;
+        have[t] = 1;
+        const float *lut = multi ? ctx->multi.dev.as<float>() + (size_t)t * bins : B.lut32.as<float>() + (size_t)t * bins;
+        jobs.push_back(DerivJob{lut, B.dtab.as<float4>() + (size_t)t * bins, (uint32_t)dspecs.size(), fixed_of(e) ? 1 : 0});
+        dspecs.push_back(multi ? table_spec(p, ctx->multi.ds[t]) : specs[e]);
     }
-    ck(launch_deriv_tables(B.d64mu.as<double>(), B.d64eps.as<double>(), bins, ntab, B.dtab.as<float4>(), st),
-       "derivative tables");
+    ck(B.djobs.ensure(sizeof(DerivJob) * jobs.size()), "alloc derivative tables");
+    ck(B.dspecs.ensure(sizeof(LutBuildSpec) * dspecs.size()), "alloc derivative tables");
+    ck(cudaMemcpyAsync(B.djobs.p, jobs.data(), sizeof(DerivJob) * jobs.size(), cudaMemcpyHostToDevice, st), "upload");
+    ck(cudaMemcpyAsync(B.dspecs.p, dspecs.data(), sizeof(LutBuildSpec) * dspecs.size(), cudaMemcpyHostToDevice, st), "upload");
+    ck(cudaEventRecord(ctx->ev[0], st), "event");
+    ck(launch_deriv_tables(B.dspecs.as<LutBuildSpec>(), B.djobs.as<DerivJob>(), (uint32_t)jobs.size(), bins, st), "derivative tables");
     ck(cudaEventRecord(ctx->ev[1], st), "event");
 
-    // experiments for the replay: the linear table staged in shared memory, the exact blend
+    // experiments for the replay: their fixed-point table staged in shared memory, or the linear one (exact blend)
     std::vector<BatchExpHost> bx(n);
     std::vector<BatchAdjHost> ax(n);
     struct AdjBucket {
@@ -1742,22 +1725,22 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
     for (uint32_t e = 0; e < n; ++e) {
         const ExpHost &h = eh[e];
         bx[e] = bh[e];
-        bx[e].lf = LogFixed{0.0, 0.0, 0, 0};
-        bx[e].tab = B.lin.as<float2>() + (size_t)e * bins;
+        const bool fixed = fixed_of(e);
+        bx[e].lf = fixed ? lf[e] : LogFixed{0.0, 0.0, 0, 0};
+        bx[e].tab = (fixed ? B.fix.as<float2>() : B.lin.as<float2>()) + (size_t)e * bins;
         const uint32_t t = multi ? h.multi_index : e;
         const double log10_abs = std::log10(h.spec.absorption_factor);
         const bool ok = red[e].valid > 0 && std::isfinite(red[e].log10_sum);
         ax[e] = BatchAdjHost{B.dtab.as<float4>() + (size_t)t * bins,
-                             ok ? (float)(red[e].log10_sum - (double)(h.N - 1) * log10_abs) : 0.0f};
+                             ok ? red[e].log10_sum - (double)(h.N - 1) * log10_abs : 0.0};
         if (h.spec.n_chains == 0) continue;
-        BatchShape sh{h.t.group, h.t.spl, std::min(h.t.warps_per_block, batch_max_threads(h.t.group, h.t.spl) / 32), 1, 1,
-                      1, 0};
+        BatchShape sh{h.t.group, h.t.spl, std::min(h.t.warps_per_block, kAdjointThreads / 32), fixed ? 0 : 1, 1, fixed ? 0 : 1, 0};
         while (sh.warps > 4 && batch_smem_bytes(sh, bins) > kSmemCap) sh.warps -= 4;
         if (batch_smem_bytes(sh, bins) > kSmemCap)
             fail(TWISTY_ERR_UNSUPPORTED, exp_msg(e, "weight table too large to stage for the adjoint"));
         AdjBucket *bk = nullptr;
         for (AdjBucket &b : abk)
-            if (b.shape.group == sh.group && b.shape.spl == sh.spl && b.shape.warps == sh.warps) bk = &b;
+            if (b.shape.group == sh.group && b.shape.spl == sh.spl && b.shape.warps == sh.warps && b.shape.exact == sh.exact) bk = &b;
         if (!bk) {
             abk.push_back(AdjBucket{});
             abk.back().shape = sh;
@@ -1951,21 +1934,26 @@ twisty_status twisty_adjoint(twisty_ctx *ctx, const twisty_bc *bc, const twisty_
         prepare(ctx, bc);
         const uint32_t N = ctx->p.num_segments;
         const float ds = bc->arclength / (float)N;
-        build_tables(ctx, ds, true);
         const uint32_t bins = ctx->p.num_curvature_steps;
         const ChainSpec &c = ctx->spec;
-        DevBuf dtab, dg, dout;
+        cudaStream_t st = ctx->stream;
+        DevBuf dtab, dg, dout, djob;
         try {
             ck(dtab.ensure(sizeof(float4) * bins), "alloc");
             ck(dg.ensure(sizeof(double) * 6 * std::max<uint32_t>(c.n_chains, 1)), "alloc");
             ck(dout.ensure(sizeof(double) * 6), "alloc");
-            ck(launch_deriv_tables(ctx->dmus.as<double>(), ctx->deps.as<double>(), bins, 1, dtab.as<float4>(), ctx->stream),
+            struct {
+                LutBuildSpec spec;
+                DerivJob job;
+            } up{table_spec(ctx->p, ds), DerivJob{ctx->lut32.as<float>(), dtab.as<float4>(), 0u, comp_adjoint_fixed(ctx->lf, c.inv_ds, ctx->meta) ? 1 : 0}};
+            ck(djob.ensure(sizeof(up)), "alloc");
+            ck(cudaMemcpyAsync(djob.p, &up, sizeof(up), cudaMemcpyHostToDevice, st), "upload");
+            ck(launch_deriv_tables(djob.as<LutBuildSpec>(),
+                                   reinterpret_cast<const DerivJob *>(djob.as<char>() + ((char *)&up.job - (char *)&up)), 1, bins, st),
                "derivative tables");
             const double ref = fwd->log10_weight - fwd->log10_normalizer - (double)(N - 1) * std::log10(c.absorption_factor);
-            CompTuning t = staged_tuning(ctx);
-            t.exact_blend = 1;
-            ck(launch_comp_adjoint(c, t, ctx->init_seg.as<float>(), ctx->lintab.as<float2>(), ctx->meta,
-                                   dtab.as<float4>(), (float)ref, dg.as<double>(), dout.as<double>(), ctx->stream),
+            ck(launch_comp_adjoint(c, staged_tuning(ctx), ctx->init_seg.as<float>(), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
+                                   ctx->meta, dtab.as<float4>(), ref, dg.as<double>(), dout.as<double>(), st, ctx->lf),
                "adjoint kernel");
             double g[6];
             ck(cudaMemcpyAsync(g, dout.p, sizeof(g), cudaMemcpyDeviceToHost, ctx->stream), "read gradient");
@@ -1978,10 +1966,10 @@ twisty_status twisty_adjoint(twisty_ctx *ctx, const twisty_bc *bc, const twisty_
             grad[3] = g[3] / g[5];
             grad[4] = g[4] / g[5];
         } catch (...) {
-            dtab.release(); dg.release(); dout.release();
+            dtab.release(); dg.release(); dout.release(); djob.release();
             throw;
         }
-        dtab.release(); dg.release(); dout.release();
+        dtab.release(); dg.release(); dout.release(); djob.release();
     });
 }
 
