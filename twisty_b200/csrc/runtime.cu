@@ -81,6 +81,81 @@ uint64_t seed_of(uint32_t s)
 
 }  // namespace
 
+// Copies large host arrays to the device: a pageable copy goes through one driver thread's staging
+// (16 GB/s measured); here a few threads fill a ring of pinned chunks, each copied as soon as it is full,
+// on the call's stream. Returns when the array has been read and copied. The ring (kThreads x 1 MB) belongs to
+// the context and is made by its second copy of kMin bytes and more: pinning it takes some 4 ms, more than
+// one copy wins (50 MB of positions: 3.1 -> 1.2 ms).
+struct Uploader {
+    static constexpr size_t kChunk = 1u << 20, kMin = 4u << 20;
+    static constexpr int kThreads = 4;
+    unsigned char *ring = nullptr;
+    cudaEvent_t free_ev[kThreads] = {};
+    bool again = false;   // a large copy has gone before
+    void release()
+    {
+        if (ring) cudaFreeHost(ring);
+        ring = nullptr;
+        for (cudaEvent_t &e : free_ev) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+    }
+    cudaError_t copy(int device, void *dst, const void *src, size_t bytes, cudaStream_t st)
+    {
+        if (bytes < kMin || !again) {
+            again |= bytes >= kMin;
+            return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        }
+        cudaError_t e = cudaSuccess;
+        if (!ring) {
+            e = cudaHostAlloc(reinterpret_cast<void **>(&ring), kChunk * kThreads, cudaHostAllocDefault);
+            for (cudaEvent_t &ev : free_ev)
+                if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                release();   // no pinned memory to be had: the driver's own staging
+                return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+            }
+        }
+        const size_t chunks = (bytes + kChunk - 1) / kChunk;
+        std::atomic<size_t> next{0};
+        std::atomic<int> err{(int)cudaSuccess};
+        auto work = [&](int slot) {
+            cudaError_t r = cudaSetDevice(device);
+            unsigned char *buf = ring + (size_t)slot * kChunk;
+            bool used = false;
+            while (r == cudaSuccess && err.load() == (int)cudaSuccess) {
+                const size_t c = next.fetch_add(1);
+                if (c >= chunks) break;
+                const size_t at = c * kChunk, n = std::min(kChunk, bytes - at);
+                if (used) r = cudaEventSynchronize(free_ev[slot]);
+                if (r != cudaSuccess) break;
+                std::memcpy(buf, static_cast<const unsigned char *>(src) + at, n);
+                r = cudaMemcpyAsync(static_cast<unsigned char *>(dst) + at, buf, n, cudaMemcpyHostToDevice, st);
+                if (r == cudaSuccess) r = cudaEventRecord(free_ev[slot], st);
+                used = true;
+            }
+            // the slot is free again for the next call
+            if (used) {
+                const cudaError_t w = cudaEventSynchronize(free_ev[slot]);
+                if (r == cudaSuccess) r = w;
+            }
+            if (r != cudaSuccess) err.store((int)r);
+        };
+        std::thread pool[kThreads - 1];
+        int started = 0;
+        try {
+            for (; started < kThreads - 1; ++started) pool[started] = std::thread(work, started + 1);
+        } catch (...) {
+            // fewer threads than wanted: the others take their share
+        }
+        work(0);
+        for (int i = 0; i < started; ++i) pool[i].join();
+        return (cudaError_t)err.load();
+    }
+};
+
 // Device buffers of batched runs, kept by the context so that repeated batches of the same
 // size allocate nothing (DevBuf::ensure only grows). The last row serves the batched adjoint.
 struct BatchBufs {
@@ -93,6 +168,27 @@ struct BatchBufs {
                          &adj_exps, &adj_aux, &adj_items, &adj_counters, &grad, &grad_sum};
         for (DevBuf *b : all) b->release();
     }
+};
+
+// Device buffers of the calls that used to allocate and free theirs (a cudaMalloc or cudaFree waits for
+// the device: 0.1-0.3 ms each), kept by the context; the ones above kKeepBytes are given back when the
+// call ends.
+struct CallBufs {
+    static constexpr size_t kKeepBytes = 256ull << 20;
+    DevBuf a, b, c, d;
+    void release()
+    {
+        for (DevBuf *x : {&a, &b, &c, &d}) x->release();
+    }
+    void trim()
+    {
+        for (DevBuf *x : {&a, &b, &c, &d})
+            if (x->bytes > kKeepBytes) x->release();
+    }
+};
+struct Trim {
+    CallBufs &b;
+    ~Trim() { b.trim(); }
 };
 
 // Workspaces of the M-segment estimator, kept by the context (a column of points per thread of a
@@ -141,7 +237,7 @@ struct twisty_ctx {
     twisty_params p{};
     int device = 0;
     int sm_count = 148;
-    std::string device_name;
+    std::string name;            // of the device, once the tuning cache needed it
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::string err;
@@ -180,7 +276,7 @@ struct twisty_ctx {
     double prepare_start = 0.0;
     std::vector<float> user_curve;
     std::vector<float> init_pos_host;
-    DevBuf init_pos, init_seg, state, chain_out, partials, reduce_out, norm_scratch;
+    DevBuf init_pos, state, chain_out, partials, reduce_out, norm_scratch;
     DevBuf check_state, check_out;   // the FP64 replay of the first chains (fp64_check_chains)
     uint32_t check_chains = 0;
     double check_meta[3] = {0.0, 0.0, 0.0};   // min_k, max_k, step of the FP64 replay's table
@@ -188,6 +284,9 @@ struct twisty_ctx {
     bool launched = false;
     BatchBufs batch;
     MSegBufs mseg;
+    CallBufs call;
+    Uploader upload;
+    cudaStream_t pass_stream = nullptr;   // the stream of the last launch
     BatchGraph batch_graph;
 };
 
@@ -238,6 +337,15 @@ struct TuneEntry {
 std::mutex g_tune_mu;
 std::vector<TuneEntry> g_tune;
 
+// The device's name, asked for only when the cache has entries to compare it with or to record
+// (cudaGetDeviceProperties takes 3.9 ms, which every context used to pay).
+std::string device_name(int device)
+{
+    cudaDeviceProp prop{};
+    ck(cudaGetDeviceProperties(&prop, device), "device query");
+    return prop.name;
+}
+
 void tune_record(const TuneEntry &e)
 {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -249,11 +357,12 @@ void tune_record(const TuneEntry &e)
     g_tune.push_back(e);
 }
 
-bool tune_lookup(const std::string &device, uint32_t n, uint32_t bins, CompTuning &t)
+bool tune_lookup(twisty_ctx *ctx, uint32_t n, uint32_t bins, CompTuning &t)
 {
     std::lock_guard<std::mutex> lk(g_tune_mu);
+    if (!g_tune.empty() && ctx->name.empty()) ctx->name = device_name(ctx->device);
     for (const TuneEntry &x : g_tune)
-        if (x.device == device && x.n == n && x.bins == bins) {
+        if (x.n == n && x.bins == bins && x.device == ctx->name) {
             CompTuning c = t;
             c.group = (int)x.group;
             c.spl = (int)x.spl;
@@ -487,7 +596,11 @@ CompTuning staged_tuning(const twisty_ctx *ctx)
     return t;
 }
 
-void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
+// The initial curve's segment vectors, after its points.
+const float *init_segments(const twisty_ctx *ctx) { return ctx->init_pos.as<float>() + 3 * (size_t)(ctx->spec.n_segments + 1); }
+
+// wait false: what follows runs on the context's stream, after the uploads.
+void prepare(twisty_ctx *ctx, const twisty_bc *bcp, bool wait = true)
 {
     const double t0 = now_ms();
     validate(ctx->p);
@@ -541,7 +654,7 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
     } else if (p.form == TWISTY_FORM_COMPENSATED) {
         ctx->tuning = comp_default_tuning(N, false, p.paths_to_generate, p.paths_to_skip);
         bool default_shape = !p.comp_group && !p.comp_spl && !p.comp_warps;
-        if (default_shape && tune_lookup(ctx->device_name, N, p.num_curvature_steps, ctx->tuning)) default_shape = false;
+        if (default_shape && tune_lookup(ctx, N, p.num_curvature_steps, ctx->tuning)) default_shape = false;
         if (p.comp_group || p.comp_spl) {
             if (!p.comp_group || !p.comp_spl) fail(TWISTY_ERR_INVALID_CONFIG, "comp_group and comp_spl are set together");
             ctx->tuning.group = (int)p.comp_group;
@@ -601,10 +714,9 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
     layout(ctx, p.paths_to_generate, requested, max_steps);
 
     cudaStream_t st = ctx->stream;
-    ck(ctx->init_pos.ensure(sizeof(float) * pos.size()), "alloc curve");
-    ck(ctx->init_seg.ensure(sizeof(float) * seg.size()), "alloc curve");
+    ck(ctx->init_pos.ensure(sizeof(float) * (pos.size() + seg.size())), "alloc curve");
+    pos.insert(pos.end(), seg.begin(), seg.end());   // the points, then the segment vectors
     ck(cudaMemcpyAsync(ctx->init_pos.p, pos.data(), sizeof(float) * pos.size(), cudaMemcpyHostToDevice, st), "upload curve");
-    ck(cudaMemcpyAsync(ctx->init_seg.p, seg.data(), sizeof(float) * seg.size(), cudaMemcpyHostToDevice, st), "upload curve");
     const uint32_t C = std::max<uint32_t>(c.n_chains, 1);
     ck(ctx->chain_out.ensure(sizeof(ChainOut) * C), "alloc chain results");
     ck(ctx->reduce_out.ensure(sizeof(ReduceOut)), "alloc result");
@@ -639,7 +751,7 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp)
             ctx->check_meta[2] = ctx->meta.step;
         }
     }
-    ck(cudaStreamSynchronize(st), "prepare");
+    if (wait) ck(cudaStreamSynchronize(st), "prepare");
     ctx->kernels_per_launch = c.n_chains ? 2 + (ctx->check_chains ? 1 : 0) : 0;
     ctx->bc = bc;
     ctx->prepared = true;
@@ -652,6 +764,7 @@ void launch(twisty_ctx *ctx, cudaStream_t st)
     if (!ctx->prepared) fail(TWISTY_ERR_INVALID_ARGUMENT, "twisty_launch before twisty_prepare");
     set_device(ctx);
     const ChainSpec &c = ctx->spec;
+    ctx->pass_stream = st;
     ck(cudaEventRecord(ctx->ev[0], st), "event");
     if (c.n_chains) {
         const twisty_params &p = ctx->p;
@@ -666,7 +779,7 @@ void launch(twisty_ctx *ctx, cudaStream_t st)
                                   step, (int32_t)p.num_curvature_steps, ctx->chain_out.as<ChainOut>(), st),
                "fp64 chain kernel");
         } else {
-            ck(launch_comp_chains(c, ctx->tuning, ctx->init_seg.as<float>(), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
+            ck(launch_comp_chains(c, ctx->tuning, init_segments(ctx), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
                                   ctx->meta, ctx->chain_out.as<ChainOut>(), ctx->partials.as<double2>(), st, ctx->lf),
                "compensated chain kernel");
         }
@@ -696,8 +809,8 @@ void collect(twisty_ctx *ctx, twisty_result *res)
     set_device(ctx);
     ReduceOut r{};
     r.log10_sum = -std::numeric_limits<double>::infinity();
-    // The pass may have been enqueued on any stream; its last event orders the copy.
-    ck(cudaEventSynchronize(ctx->ev[2]), "sync");
+    // The pass may have been enqueued on any stream; then its last event orders the copy.
+    if (ctx->pass_stream != ctx->stream || !ctx->spec.n_chains) ck(cudaEventSynchronize(ctx->ev[2]), "sync");
     if (ctx->spec.n_chains) {
         ck(cudaMemcpyAsync(&r, ctx->reduce_out.p, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream), "read result");
         ck(cudaStreamSynchronize(ctx->stream), "read result");
@@ -965,9 +1078,6 @@ twisty_status twisty_create(const twisty_params *p, twisty_ctx **out)
         int sms = 0;
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device), "device query");
         ctx->sm_count = sms;
-        cudaDeviceProp prop{};
-        ck(cudaGetDeviceProperties(&prop, ctx->device), "device query");
-        ctx->device_name = prop.name;
         ck(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "stream");
         for (auto &e : ctx->ev) ck(cudaEventCreate(&e), "event");
     });
@@ -986,12 +1096,14 @@ void twisty_destroy(twisty_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DevBuf *bufs[] = {&ctx->lut64, &ctx->lut32, &ctx->fixtab, &ctx->lintab, &ctx->lutaux,
-                      &ctx->init_pos, &ctx->init_seg, &ctx->state, &ctx->chain_out, &ctx->partials, &ctx->reduce_out,
+                      &ctx->init_pos, &ctx->state, &ctx->chain_out, &ctx->partials, &ctx->reduce_out,
                       &ctx->norm_scratch, &ctx->multi.dev, &ctx->check_state, &ctx->check_out};
     for (DevBuf *b : bufs) b->release();
     ctx->batch_graph.release();
     ctx->batch.release();
     ctx->mseg.release();
+    ctx->call.release();
+    ctx->upload.release();
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1038,7 +1150,7 @@ twisty_status twisty_run(twisty_ctx *ctx, const twisty_bc *bc, twisty_result *re
     if (!ctx || !res) return TWISTY_ERR_INVALID_ARGUMENT;
     return guard(ctx, [&] {
         const double t0 = now_ms();
-        prepare(ctx, bc);
+        prepare(ctx, bc, false);
         launch(ctx, ctx->stream);
         collect(ctx, res);
         res->total_ms = now_ms() - t0;
@@ -1179,38 +1291,32 @@ twisty_status twisty_weight_paths(twisty_ctx *ctx, const twisty_bc *bc, const fl
         build_tables(ctx, ds);
         if (n_paths == 0) return;
         cudaStream_t st = ctx->stream;
-        DevBuf dpos, dw, dv, db;
+        DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dv = ctx->call.c, &db = ctx->call.d;
+        const Trim trim{ctx->call};
         const size_t np = 3 * (size_t)(N + 1) * n_paths;
-        try {
-            ck(dpos.ensure(sizeof(float) * np), "alloc paths");
-            ck(dw.ensure(sizeof(double) * n_paths), "alloc weights");
-            ck(dv.ensure(n_paths), "alloc validity");
-            if (bins) ck(db.ensure(sizeof(int32_t) * (N - 1) * n_paths), "alloc bins");
-            ck(cudaMemcpyAsync(dpos.p, pos, sizeof(float) * np, cudaMemcpyHostToDevice, st), "upload paths");
-            const float inv_ds = (float)N / bc->arclength;
-            const double af = (double)std::exp(-ctx->p.absorption * ds);
-            if (form == TWISTY_FORM_COMPENSATED) {
-                ck(launch_weigh_comp(dpos.as<float>(), n_paths, N, inv_ds, ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
-                                     ctx->exact_blend, ctx->meta, std::log10(af), dw.as<double>(), dv.as<uint8_t>(),
-                                     bins ? db.as<int32_t>() : nullptr, st, ctx->lf),
-                   "weigh kernel");
-            } else if (form == TWISTY_FORM_PLAIN_FP32) {
-                ck(launch_weigh_plain(dpos.as<float>(), n_paths, N, inv_ds, ctx->lut32.as<float>(), ctx->meta, af,
-                                      dw.as<double>(), dv.as<uint8_t>(), bins ? db.as<int32_t>() : nullptr, st),
-                   "weigh kernel");
-            } else {
-                fail(TWISTY_ERR_UNSUPPORTED, "weight_paths supports the plain and compensated forms");
-            }
-            ck(cudaMemcpyAsync(log10w, dw.p, sizeof(double) * n_paths, cudaMemcpyDeviceToHost, st), "read weights");
-            if (valid) ck(cudaMemcpyAsync(valid, dv.p, n_paths, cudaMemcpyDeviceToHost, st), "read validity");
-            if (bins) ck(cudaMemcpyAsync(bins, db.p, sizeof(int32_t) * (N - 1) * n_paths, cudaMemcpyDeviceToHost, st), "read bins");
-            ck(cudaStreamSynchronize(st), "weigh");
-        } catch (...) {
-            cudaStreamSynchronize(st);
-            dpos.release(); dw.release(); dv.release(); db.release();
-            throw;
+        ck(dpos.ensure(sizeof(float) * np), "alloc paths");
+        ck(dw.ensure(sizeof(double) * n_paths), "alloc weights");
+        ck(dv.ensure(n_paths), "alloc validity");
+        if (bins) ck(db.ensure(sizeof(int32_t) * (N - 1) * n_paths), "alloc bins");
+        ck(ctx->upload.copy(ctx->device, dpos.p, pos, sizeof(float) * np, st), "upload paths");
+        const float inv_ds = (float)N / bc->arclength;
+        const double af = (double)std::exp(-ctx->p.absorption * ds);
+        if (form == TWISTY_FORM_COMPENSATED) {
+            ck(launch_weigh_comp(dpos.as<float>(), n_paths, N, inv_ds, ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
+                                 ctx->exact_blend, ctx->meta, std::log10(af), dw.as<double>(), dv.as<uint8_t>(),
+                                 bins ? db.as<int32_t>() : nullptr, st, ctx->lf),
+               "weigh kernel");
+        } else if (form == TWISTY_FORM_PLAIN_FP32) {
+            ck(launch_weigh_plain(dpos.as<float>(), n_paths, N, inv_ds, ctx->lut32.as<float>(), ctx->meta, af,
+                                  dw.as<double>(), dv.as<uint8_t>(), bins ? db.as<int32_t>() : nullptr, st),
+               "weigh kernel");
+        } else {
+            fail(TWISTY_ERR_UNSUPPORTED, "weight_paths supports the plain and compensated forms");
         }
-        dpos.release(); dw.release(); dv.release(); db.release();
+        ck(cudaMemcpyAsync(log10w, dw.p, sizeof(double) * n_paths, cudaMemcpyDeviceToHost, st), "read weights");
+        if (valid) ck(cudaMemcpyAsync(valid, dv.p, n_paths, cudaMemcpyDeviceToHost, st), "read validity");
+        if (bins) ck(cudaMemcpyAsync(bins, db.p, sizeof(int32_t) * (N - 1) * n_paths, cudaMemcpyDeviceToHost, st), "read bins");
+        ck(cudaStreamSynchronize(st), "weigh");
     });
 }
 
@@ -1396,7 +1502,7 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         {
             // a tuned shape the batched kernel does not have keeps the default
             CompTuning tuned = h.t;
-            if (tune_lookup(ctx->device_name, N, bins, tuned)) {
+            if (tune_lookup(ctx, N, bins, tuned)) {
                 const int w = std::min(tuned.warps_per_block, batch_max_threads(tuned.group, tuned.spl) / 32);
                 if (batch_shape_supported(BatchShape{tuned.group, tuned.spl, w, 0, 1, 0, 0}, N, 2)) h.t = tuned;
             }
@@ -1854,12 +1960,13 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
     if (!ctx || !bc) return TWISTY_ERR_INVALID_ARGUMENT;
     return guard(ctx, [&] {
         const double t0 = now_ms();
-        prepare(ctx, bc);
+        prepare(ctx, bc, false);
         launch(ctx, ctx->stream);
         twisty_result r{};
         collect(ctx, &r);
         const ChainSpec &c = ctx->spec;
         const uint32_t N = c.n_segments;
+        const size_t stride = 3 * (size_t)(N + 1);
         std::vector<float> hpos;
         std::vector<double> hw;
         std::vector<uint32_t> chain_of;
@@ -1871,50 +1978,59 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
             ce.n_chains = E;
             ce.last_steps = (E == c.n_chains) ? c.last_steps : c.steps;
             const size_t npaths = (size_t)E * c.steps;
-            DevBuf dpos, dw, dout;
-            try {
-                ck(dpos.ensure(sizeof(float) * 3 * (size_t)(N + 1) * npaths), "alloc export buffer");
-                ck(dw.ensure(sizeof(double) * npaths), "alloc export buffer");
-                ck(dout.ensure(sizeof(ChainOut) * E), "alloc export buffer");
-                ck(cudaMemsetAsync(dw.p, 0xff, sizeof(double) * npaths, ctx->stream), "memset");  // NaN: not written
-                if (ctx->p.form == TWISTY_FORM_PLAIN_FP32) {
-                    ck(launch_plain_chains(ce, ctx->init_pos.as<float>(), ctx->state.as<float>(), ctx->lut32.as<float>(),
-                                           ctx->meta, dout.as<ChainOut>(), ctx->stream, dpos.as<float>(), dw.as<double>()),
-                       "export replay");
-                } else if (ctx->p.form == TWISTY_FORM_COMPENSATED) {
-                    if (ce.has_eval_shift) fail(TWISTY_ERR_UNSUPPORTED, "eval_end_shift applies to forward passes of the compensated form only");
-                    const float x0[3] = {bc->start_pos.x, bc->start_pos.y, bc->start_pos.z};
-                    ck(launch_comp_export(ce, staged_tuning(ctx), ctx->init_seg.as<float>(), ctx->fixtab.as<float2>(),
-                                          ctx->lintab.as<float2>(), ctx->meta, x0, dpos.as<float>(), dw.as<double>(),
-                                          dout.as<ChainOut>(), ctx->stream, ctx->lf),
-                       "export replay");
-                } else {
-                    fail(TWISTY_ERR_UNSUPPORTED, "path export runs the plain and compensated forms");
-                }
-                std::vector<float> apos(3 * (size_t)(N + 1) * npaths);
-                std::vector<double> aw(npaths);
-                ck(cudaMemcpyAsync(apos.data(), dpos.p, sizeof(float) * apos.size(), cudaMemcpyDeviceToHost, ctx->stream), "read export");
-                ck(cudaMemcpyAsync(aw.data(), dw.p, sizeof(double) * npaths, cudaMemcpyDeviceToHost, ctx->stream), "read export");
-                ck(cudaStreamSynchronize(ctx->stream), "export");
-                // invalid paths are skipped, as the reference skips them before exporting
-                for (uint32_t ch = 0; ch < E && hw.size() < max_paths; ++ch) {
-                    const uint32_t steps = (ch == c.n_chains - 1) ? c.last_steps : c.steps;
-                    for (uint32_t s = 0; s < steps && hw.size() < max_paths; ++s) {
-                        const size_t i = (size_t)ch * c.steps + s;
-                        if (!std::isfinite(aw[i])) continue;
-                        hw.push_back(aw[i]);
-                        chain_of.push_back(ch);
-                        hpos.insert(hpos.end(), apos.begin() + i * 3 * (N + 1), apos.begin() + (i + 1) * 3 * (N + 1));
-                    }
-                }
-            } catch (...) {
-                dpos.release(); dw.release(); dout.release();
-                throw;
+            cudaStream_t st = ctx->stream;
+            DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dout = ctx->call.c;
+            const Trim trim{ctx->call};
+            ck(dpos.ensure(sizeof(float) * stride * npaths), "alloc export buffer");
+            ck(dw.ensure(sizeof(double) * npaths), "alloc export buffer");
+            ck(dout.ensure(sizeof(ChainOut) * E), "alloc export buffer");
+            ck(cudaMemsetAsync(dw.p, 0xff, sizeof(double) * npaths, st), "memset");  // NaN: not written
+            if (ctx->p.form == TWISTY_FORM_PLAIN_FP32) {
+                ck(launch_plain_chains(ce, ctx->init_pos.as<float>(), ctx->state.as<float>(), ctx->lut32.as<float>(),
+                                       ctx->meta, dout.as<ChainOut>(), st, dpos.as<float>(), dw.as<double>()),
+                   "export replay");
+            } else if (ctx->p.form == TWISTY_FORM_COMPENSATED) {
+                if (ce.has_eval_shift) fail(TWISTY_ERR_UNSUPPORTED, "eval_end_shift applies to forward passes of the compensated form only");
+                const float x0[3] = {bc->start_pos.x, bc->start_pos.y, bc->start_pos.z};
+                ck(launch_comp_export(ce, staged_tuning(ctx), init_segments(ctx), ctx->fixtab.as<float2>(),
+                                      ctx->lintab.as<float2>(), ctx->meta, x0, dpos.as<float>(), dw.as<double>(),
+                                      dout.as<ChainOut>(), st, ctx->lf),
+                   "export replay");
+            } else {
+                fail(TWISTY_ERR_UNSUPPORTED, "path export runs the plain and compensated forms");
             }
-            dpos.release(); dw.release(); dout.release();
+            std::vector<double> aw(npaths);
+            ck(cudaMemcpyAsync(aw.data(), dw.p, sizeof(double) * npaths, cudaMemcpyDeviceToHost, st), "read export");
+            ck(cudaStreamSynchronize(st), "export");
+            // invalid paths are skipped, as the reference skips them before exporting: the valid ones come back in
+            // runs of consecutive paths, straight into the caller's array where no files are written
+            struct Run {
+                size_t from, n;
+            };
+            std::vector<Run> runs;
+            for (uint32_t ch = 0; ch < E && hw.size() < max_paths; ++ch) {
+                const uint32_t steps = (ch == c.n_chains - 1) ? c.last_steps : c.steps;
+                for (uint32_t s = 0; s < steps && hw.size() < max_paths; ++s) {
+                    const size_t i = (size_t)ch * c.steps + s;
+                    if (!std::isfinite(aw[i])) continue;
+                    hw.push_back(aw[i]);
+                    chain_of.push_back(ch);
+                    if (!runs.empty() && runs.back().from + runs.back().n == i) ++runs.back().n;
+                    else runs.push_back(Run{i, 1});
+                }
+            }
+            if (dir || pos) {
+                if (dir) hpos.resize(hw.size() * stride);
+                float *to = dir ? hpos.data() : pos;
+                for (const Run &run : runs) {
+                    ck(cudaMemcpyAsync(to, dpos.as<float>() + run.from * stride, sizeof(float) * run.n * stride, cudaMemcpyDeviceToHost, st), "read export");
+                    to += run.n * stride;
+                }
+                ck(cudaStreamSynchronize(st), "export");
+            }
         }
         const uint64_t n = hw.size();
-        if (pos && n) std::memcpy(pos, hpos.data(), sizeof(float) * hpos.size());
+        if (pos && dir && n) std::memcpy(pos, hpos.data(), sizeof(float) * hpos.size());
         if (log10w && n) std::memcpy(log10w, hw.data(), sizeof(double) * n);
         if (n_written) *n_written = n;
         if (dir) write_path_batch(dir, *bc, N, ctx->log10_norm, hpos, hw, chain_of);
@@ -1931,45 +2047,40 @@ twisty_status twisty_adjoint(twisty_ctx *ctx, const twisty_bc *bc, const twisty_
         if (ctx->p.lut_mode != TWISTY_LUT_FP64) fail(TWISTY_ERR_UNSUPPORTED, "the adjoint needs lut_mode FP64 (derivative tables)");
         const twisty_vec3 &sh = ctx->p.eval_end_shift;
         if (sh.x != 0.f || sh.y != 0.f || sh.z != 0.f) fail(TWISTY_ERR_UNSUPPORTED, "eval_end_shift applies to forward passes only");
-        prepare(ctx, bc);
+        prepare(ctx, bc, false);
         const uint32_t N = ctx->p.num_segments;
         const float ds = bc->arclength / (float)N;
         const uint32_t bins = ctx->p.num_curvature_steps;
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
-        DevBuf dtab, dg, dout, djob;
-        try {
-            ck(dtab.ensure(sizeof(float4) * bins), "alloc");
-            ck(dg.ensure(sizeof(double) * 6 * std::max<uint32_t>(c.n_chains, 1)), "alloc");
-            ck(dout.ensure(sizeof(double) * 6), "alloc");
-            struct {
-                LutBuildSpec spec;
-                DerivJob job;
-            } up{table_spec(ctx->p, ds), DerivJob{ctx->lut32.as<float>(), dtab.as<float4>(), 0u, comp_adjoint_fixed(ctx->lf, c.inv_ds, ctx->meta) ? 1 : 0}};
-            ck(djob.ensure(sizeof(up)), "alloc");
-            ck(cudaMemcpyAsync(djob.p, &up, sizeof(up), cudaMemcpyHostToDevice, st), "upload");
-            ck(launch_deriv_tables(djob.as<LutBuildSpec>(),
-                                   reinterpret_cast<const DerivJob *>(djob.as<char>() + ((char *)&up.job - (char *)&up)), 1, bins, st),
-               "derivative tables");
-            const double ref = fwd->log10_weight - fwd->log10_normalizer - (double)(N - 1) * std::log10(c.absorption_factor);
-            ck(launch_comp_adjoint(c, staged_tuning(ctx), ctx->init_seg.as<float>(), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
-                                   ctx->meta, dtab.as<float4>(), ref, dg.as<double>(), dout.as<double>(), st, ctx->lf),
-               "adjoint kernel");
-            double g[6];
-            ck(cudaMemcpyAsync(g, dout.p, sizeof(g), cudaMemcpyDeviceToHost, ctx->stream), "read gradient");
-            ck(cudaStreamSynchronize(ctx->stream), "adjoint");
-            if (!(g[5] > 0.0)) fail(TWISTY_ERR_INVALID_ARGUMENT, "forward result does not match this experiment");
-            const double sigma = std::sqrt((double)ctx->p.eps);
-            grad[0] = g[0] / g[5];
-            grad[1] = g[1] / g[5] * 2.0 * sigma;   // eps = sigma^2
-            grad[2] = g[2] / g[5];
-            grad[3] = g[3] / g[5];
-            grad[4] = g[4] / g[5];
-        } catch (...) {
-            dtab.release(); dg.release(); dout.release(); djob.release();
-            throw;
-        }
-        dtab.release(); dg.release(); dout.release(); djob.release();
+        DevBuf &dtab = ctx->call.a, &dg = ctx->call.b, &dout = ctx->call.c, &djob = ctx->call.d;
+        const Trim trim{ctx->call};
+        ck(dtab.ensure(sizeof(float4) * bins), "alloc");
+        ck(dg.ensure(sizeof(double) * 6 * std::max<uint32_t>(c.n_chains, 1)), "alloc");
+        ck(dout.ensure(sizeof(double) * 6), "alloc");
+        struct {
+            LutBuildSpec spec;
+            DerivJob job;
+        } up{table_spec(ctx->p, ds), DerivJob{ctx->lut32.as<float>(), dtab.as<float4>(), 0u, comp_adjoint_fixed(ctx->lf, c.inv_ds, ctx->meta) ? 1 : 0}};
+        ck(djob.ensure(sizeof(up)), "alloc");
+        ck(cudaMemcpyAsync(djob.p, &up, sizeof(up), cudaMemcpyHostToDevice, st), "upload");
+        ck(launch_deriv_tables(djob.as<LutBuildSpec>(),
+                               reinterpret_cast<const DerivJob *>(djob.as<char>() + ((char *)&up.job - (char *)&up)), 1, bins, st),
+           "derivative tables");
+        const double ref = fwd->log10_weight - fwd->log10_normalizer - (double)(N - 1) * std::log10(c.absorption_factor);
+        ck(launch_comp_adjoint(c, staged_tuning(ctx), init_segments(ctx), ctx->fixtab.as<float2>(), ctx->lintab.as<float2>(),
+                               ctx->meta, dtab.as<float4>(), ref, dg.as<double>(), dout.as<double>(), st, ctx->lf),
+           "adjoint kernel");
+        double g[6];
+        ck(cudaMemcpyAsync(g, dout.p, sizeof(g), cudaMemcpyDeviceToHost, ctx->stream), "read gradient");
+        ck(cudaStreamSynchronize(ctx->stream), "adjoint");
+        if (!(g[5] > 0.0)) fail(TWISTY_ERR_INVALID_ARGUMENT, "forward result does not match this experiment");
+        const double sigma = std::sqrt((double)ctx->p.eps);
+        grad[0] = g[0] / g[5];
+        grad[1] = g[1] / g[5] * 2.0 * sigma;   // eps = sigma^2
+        grad[2] = g[2] / g[5];
+        grad[3] = g[3] / g[5];
+        grad[4] = g[4] / g[5];
     });
 }
 
@@ -1982,17 +2093,11 @@ twisty_status twisty_weight_histogram(twisty_ctx *ctx, const twisty_bc *bc, doub
         if (ctx->p.form == TWISTY_FORM_FP64) fail(TWISTY_ERR_UNSUPPORTED, "the histogram replays the plain or compensated form");
         if (ctx->p.eval_end_shift.x != 0.f || ctx->p.eval_end_shift.y != 0.f || ctx->p.eval_end_shift.z != 0.f)
             fail(TWISTY_ERR_UNSUPPORTED, "eval_end_shift applies to forward passes only");
-        prepare(ctx, bc);
+        prepare(ctx, bc, false);
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
-        DevBuf dw, dout, dcnt;
-        struct Release {
-            DevBuf *b[3];
-            ~Release()
-            {
-                for (DevBuf *x : b) x->release();
-            }
-        } rel{{&dw, &dout, &dcnt}};
+        DevBuf &dw = ctx->call.a, &dout = ctx->call.b, &dcnt = ctx->call.c;
+        const Trim trim{ctx->call};
         ck(dcnt.ensure(sizeof(unsigned long long) * n_buckets), "alloc histogram");
         ck(cudaMemsetAsync(dcnt.p, 0, sizeof(unsigned long long) * n_buckets, st), "memset");
         if (c.n_chains) {
@@ -2012,7 +2117,7 @@ twisty_status twisty_weight_histogram(twisty_ctx *ctx, const twisty_bc *bc, doub
                                            ctx->meta, dout.as<ChainOut>(), st, nullptr, dw.as<double>()),
                        "histogram replay");
                 else
-                    ck(launch_comp_export(ce, staged_tuning(ctx), ctx->init_seg.as<float>(), ctx->fixtab.as<float2>(),
+                    ck(launch_comp_export(ce, staged_tuning(ctx), init_segments(ctx), ctx->fixtab.as<float2>(),
                                           ctx->lintab.as<float2>(), ctx->meta, x0, nullptr, dw.as<double>(),
                                           dout.as<ChainOut>(), st, ctx->lf),
                        "histogram replay");
@@ -2127,7 +2232,8 @@ twisty_status twisty_autotune(twisty_ctx *ctx, const twisty_bc *bc, uint64_t tri
         ctx->p = saved;
         ctx->prepared = false;
         if (best_rate < 0) fail(TWISTY_ERR_UNSUPPORTED, "no shape ran: " + last_err);
-        tune_record(TuneEntry{ctx->device_name, N, bins, (uint32_t)bestc.group, (uint32_t)bestc.spl,
+        if (ctx->name.empty()) ctx->name = device_name(ctx->device);
+        tune_record(TuneEntry{ctx->name, N, bins, (uint32_t)bestc.group, (uint32_t)bestc.spl,
                               (uint32_t)bestc.warps, best_rate});
         best->num_segments = N;
         best->bins = bins;
