@@ -83,9 +83,8 @@ struct ModeArgs {
     // steep bin (NaN slope) are re-weighed through it
     const float2 *lin;
     // export
-    float *exp_pos;      // [chains][steps][N+1][3]
+    float *exp_pos;      // [chains][steps][N+1][3]; the chain kernel leaves unit tangents there (segment s at point s + 1)
     double *exp_w;       // [chains][steps] log10 weights (absorption included, normaliser not)
-    float x0[3];
     // adjoint: the derivative tables, one 16-byte load per segment (deriv_tables_kernel: the ratio
     // form with the fixed-point table, the linear form with the exact blend)
     const float4 *dtab;
@@ -307,14 +306,14 @@ struct Tan2 {
 // H apart keep every difference of neighbours a difference of two register pairs,
 // P_{h+1} - P_h, with load.pair(h) = the tangents of segments j*SPL + h and j*SPL + h + H (the upper
 // half of the last pair of an odd SPL is not read). The others walk their segments in order.
-template <int G, int SPL, bool FULLN, class Load, class NextFn, class Seg2Fn, class Seg1Fn>
+template <int G, int SPL, bool FULLN, bool PACKED = comp_packed(G, SPL), class Load, class NextFn, class Seg2Fn, class Seg1Fn>
 __device__ __forceinline__ void for_curvatures(uint32_t j, uint32_t N, const Load &load, NextFn next, Seg2Fn seg2, Seg1Fn seg1)
 {
     constexpr int H = (SPL + 1) / 2;
     constexpr bool ODD = SPL & 1;
     const uint32_t base = j * SPL;
     float nx, ny, nz;
-    if constexpr (!comp_packed(G, SPL)) {
+    if constexpr (!PACKED) {
         float t0x = 0.f, t0y = 0.f, t0z = 0.f, px = 0.f, py = 0.f, pz = 0.f;
 #pragma unroll
         for (int m = 0; m < SPL; ++m) {
@@ -392,7 +391,8 @@ __device__ __forceinline__ float2 tab_load(const float2 *__restrict__ tab, int32
 // Generic full recompute of one path's log10 weight (absorption excluded), for the exact
 // table or, with 64-bit lane sums, for the fixed-point table at any lane width. bin_sink(i,
 // bin) receives every curvature's bin (-1 for NaN).
-template <int G, int SPL, bool EXACT, bool CLAMP, bool GLOBAL = false, class Load, class NextFn, class BinFn>
+template <int G, int SPL, bool EXACT, bool CLAMP, bool GLOBAL = false, bool PACKED = comp_packed(G, SPL), class Load, class NextFn,
+          class BinFn>
 __device__ __forceinline__ double path_log10(uint32_t j, uint32_t N, const float2 *__restrict__ tab,
                                              const CompConsts &k, const Load &load, NextFn next, BinFn bin_sink,
                                              uint32_t &clamped)
@@ -419,9 +419,9 @@ __device__ __forceinline__ double path_log10(uint32_t j, uint32_t N, const float
     };
     // a chain that fills its group's slots: slot validity known at compile time
     if (N == (uint32_t)(G * SPL))
-        for_curvatures<G, SPL, true>(j, N, load, next, seg2, seg);
+        for_curvatures<G, SPL, true, PACKED>(j, N, load, next, seg2, seg);
     else
-        for_curvatures<G, SPL, false>(j, N, load, next, seg2, seg);
+        for_curvatures<G, SPL, false, PACKED>(j, N, load, next, seg2, seg);
     if (EXACT) {
         float hi = ks, lo = -kc;
         group_sum_pair<G>(hi, lo);
@@ -667,17 +667,19 @@ __device__ __forceinline__ void receiver_grad(const float t3[3], const float t2[
     }
 }
 
-// The CTA's segment lengths from the initial segment vectors (padding segments 1), computed as
-// the chain body computes them (|v| = |v|^2 rsqrt(|v|^2)); the CTA synchronises before use.
+// A segment's length as the chain body computes it: |v| = |v|^2 rsqrt(|v|^2).
+__device__ __forceinline__ float segment_length(const float *__restrict__ v)
+{
+    const float ss = fmaf(v[0], v[0], fmaf(v[1], v[1], v[2] * v[2]));
+    return ss * rsqrtf(ss);
+}
+
+// The CTA's segment lengths from the initial segment vectors (padding segments 1); the CTA
+// synchronises before use.
 __device__ __forceinline__ void fill_lengths(float *s_len, const float *__restrict__ init_seg, uint32_t n, uint32_t slots)
 {
     for (uint32_t s = threadIdx.x; s < slots; s += blockDim.x) {
-        float len = 1.f;
-        if (s < n) {
-            const float x = init_seg[3 * s], y = init_seg[3 * s + 1], z = init_seg[3 * s + 2];
-            const float ss = fmaf(x, x, fmaf(y, y, z * z));
-            len = ss * rsqrtf(ss);
-        }
+        const float len = s < n ? segment_length(init_seg + 3 * s) : 1.f;
         s_len[s] = len;
     }
 }
@@ -867,6 +869,22 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
         }
     };
     auto no_bins = [](uint32_t, int32_t) {};
+    // export: this lane's unit tangents, each in the place of its segment's end point
+    // (export_positions_kernel makes the points of them, every path at once: in this loop, one chain's steps
+    // wait for one another)
+    auto export_tangents = [&](uint32_t wstep) {
+        float *dst = ma.exp_pos + ((size_t)chain * c.steps + wstep) * 3 * (size_t)(N + 1);
+#pragma unroll
+        for (int m = 0; m < SPL; ++m) {
+            const uint32_t s = j * SPL + m;
+            if (s < N) {
+                const float4 v = load_rec(j, m);
+                dst[3 * (s + 1)] = v.x;
+                dst[3 * (s + 1) + 1] = v.y;
+                dst[3 * (s + 1) + 2] = v.z;
+            }
+        }
+    };
 
     for (uint32_t base = 0; base < total; base += G) {
         const dev::Proposal pr = dev::draw_step(c.seed, c.experiment, gchain, base + j, N, c.k_eff, c.max_angle);
@@ -1241,49 +1259,12 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                 }
                 if (MODE == kModeExport) {
                     const double w = bad ? NAN : kc.lw_offset + (double)tot * kc.inv_scale;
-                    // positions below
                     if (active) {
                         const size_t pidx = (size_t)chain * c.steps + wstep;
                         if (j == 0) ma.exp_w[pidx] = isnan(w) ? NAN : w + (N - 1) * ma.log10_abs;
                     }
                 }
-                if (MODE == kModeExport && ma.exp_pos) {
-                    // positions x_0 + prefix sums of l_s t_s, in double; every lane takes part in
-                    // the scan, only active chains write (a weights-only replay passes no buffer)
-                    double px = 0.0, py = 0.0, pz = 0.0;
-                    double lx[SPL], ly[SPL], lz[SPL];
-#pragma unroll
-                    for (int m = 0; m < SPL; ++m) {
-                        const float4 v = load_rec(j, m);
-                        const double l = (j * SPL + m < N) ? (double)v.w : 0.0;
-                        px += l * (double)v.x;
-                        py += l * (double)v.y;
-                        pz += l * (double)v.z;
-                        lx[m] = px; ly[m] = py; lz[m] = pz;
-                    }
-                    double ex = px, ey = py, ez = pz;  // inclusive scan of lane totals
-#pragma unroll
-                    for (int o = 1; o < G; o <<= 1) {
-                        const double ux = __shfl_up_sync(FULL, ex, o * Lanes<G>::STRIDE), uy = __shfl_up_sync(FULL, ey, o * Lanes<G>::STRIDE),
-                                     uz = __shfl_up_sync(FULL, ez, o * Lanes<G>::STRIDE);
-                        if ((int)j >= o) { ex += ux; ey += uy; ez += uz; }
-                    }
-                    ex -= px; ey -= py; ez -= pz;  // exclusive
-                    if (active) {
-                        const size_t pidx = (size_t)chain * c.steps + wstep;
-                        float *dst = ma.exp_pos + pidx * 3 * (size_t)(N + 1);
-                        if (j == 0) { dst[0] = ma.x0[0]; dst[1] = ma.x0[1]; dst[2] = ma.x0[2]; }
-#pragma unroll
-                        for (int m = 0; m < SPL; ++m) {
-                            const uint32_t s = j * SPL + m;
-                            if (s < N) {
-                                dst[3 * (s + 1)] = (float)((double)ma.x0[0] + ex + lx[m]);
-                                dst[3 * (s + 1) + 1] = (float)((double)ma.x0[1] + ey + ly[m]);
-                                dst[3 * (s + 1) + 2] = (float)((double)ma.x0[2] + ez + lz[m]);
-                            }
-                        }
-                    }
-                }
+                if (MODE == kModeExport && ma.exp_pos && active) export_tangents(wstep);
                 if (!active) continue;
                 if (bad) {
                     ++failed;
@@ -1348,45 +1329,12 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     if (j == 0) acc[5] += wt;
                 }
             } else {
-                w = path_log10<G, SPL, true, CLAMP, TAB_GLOBAL>(j, N, s_tab, kc, load_smem, next_smem, no_bins, clamped);
+                // segments in order: the rounding of the blend's float terms follows the order
+                w = path_log10<G, SPL, true, CLAMP, TAB_GLOBAL, false>(j, N, s_tab, kc, load_smem, next_smem, no_bins, clamped);
             }
-            if (MODE == kModeExport && !ma.exp_pos && active && j == 0)   // weights-only replay
-                ma.exp_w[(size_t)chain * c.steps + wstep] = isnan(w) ? NAN : w + (N - 1) * ma.log10_abs;
-            if (MODE == kModeExport && ma.exp_pos) {
-                double px = 0.0, py = 0.0, pz = 0.0;
-                double lx[SPL], ly[SPL], lz[SPL];
-#pragma unroll
-                for (int m = 0; m < SPL; ++m) {
-                    const float4 v = load_rec(j, m);
-                    const double l = (j * SPL + m < N) ? (double)v.w : 0.0;
-                    px += l * (double)v.x;
-                    py += l * (double)v.y;
-                    pz += l * (double)v.z;
-                    lx[m] = px; ly[m] = py; lz[m] = pz;
-                }
-                double ex = px, ey = py, ez = pz;
-#pragma unroll
-                for (int o = 1; o < G; o <<= 1) {
-                    const double ux = __shfl_up_sync(FULL, ex, o * Lanes<G>::STRIDE), uy = __shfl_up_sync(FULL, ey, o * Lanes<G>::STRIDE),
-                                 uz = __shfl_up_sync(FULL, ez, o * Lanes<G>::STRIDE);
-                    if ((int)j >= o) { ex += ux; ey += uy; ez += uz; }
-                }
-                ex -= px; ey -= py; ez -= pz;
-                if (active) {
-                    const size_t pidx = (size_t)chain * c.steps + wstep;
-                    float *dst = ma.exp_pos + pidx * 3 * (size_t)(N + 1);
-                    if (j == 0) { dst[0] = ma.x0[0]; dst[1] = ma.x0[1]; dst[2] = ma.x0[2]; }
-#pragma unroll
-                    for (int m = 0; m < SPL; ++m) {
-                        const uint32_t s = j * SPL + m;
-                        if (s < N) {
-                            dst[3 * (s + 1)] = (float)((double)ma.x0[0] + ex + lx[m]);
-                            dst[3 * (s + 1) + 1] = (float)((double)ma.x0[1] + ey + ly[m]);
-                            dst[3 * (s + 1) + 2] = (float)((double)ma.x0[2] + ez + lz[m]);
-                        }
-                    }
-                    if (j == 0) ma.exp_w[pidx] = isnan(w) ? NAN : w + (N - 1) * ma.log10_abs;
-                }
+            if (MODE == kModeExport && active) {
+                if (ma.exp_pos) export_tangents(wstep);   // a weights-only replay passes no buffer
+                if (j == 0) ma.exp_w[(size_t)chain * c.steps + wstep] = isnan(w) ? NAN : w + (N - 1) * ma.log10_abs;
             }
             if (!active) continue;
             if (isnan(w)) {
