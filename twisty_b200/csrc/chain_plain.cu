@@ -15,6 +15,7 @@
 #include "device_common.cuh"
 
 #include <cfloat>
+#include <cooperative_groups.h>
 
 namespace twisty {
 namespace {
@@ -381,6 +382,25 @@ __global__ void __launch_bounds__(kPlainThreads) fp64_chain_kernel(ChainSpec c, 
 // of that sum from the spread of the chain sums (chains are independent; their within-
 // chain correlation is absorbed by treating each chain sum as one observation).
 // ------------------------------------------------------------------------------------
+__device__ ReduceOut reduce_result(double mx, double s1, double s2, uint32_t n, unsigned long long valid, unsigned long long failed,
+                                   unsigned long long clamped)
+{
+    ReduceOut r;
+    r.max_chain_log10 = mx;
+    r.log10_sum = (mx > -INFINITY && s1 > 0.0) ? mx + log10(s1) : -INFINITY;
+    double se = NAN;
+    if (n > 1 && s1 > 0.0) {
+        const double mean = s1 / n;
+        const double var = fmax(0.0, (s2 - n * mean * mean) / (n - 1));
+        se = sqrt(n * var) / s1;
+    }
+    r.rel_se = se;
+    r.valid = valid;
+    r.failed = failed;
+    r.clamped = clamped;
+    return r;
+}
+
 // With ranges set, CTA x reduces the chains ranges[x] = (first, count) into out[x] (one
 // experiment of a batch per CTA).
 __global__ void __launch_bounds__(1024) reduce_kernel(const ChainOut *__restrict__ chains, uint32_t n,
@@ -449,22 +469,89 @@ __global__ void __launch_bounds__(1024) reduce_kernel(const ChainOut *__restrict
             nc += __shfl_xor_sync(0xffffffffu, nc, o);
         }
         if (l == 0) {
-            ReduceOut r;
-            r.max_chain_log10 = mx;
-            r.log10_sum = (mx > -INFINITY && s1 > 0.0) ? mx + log10(s1) : -INFINITY;
-            double se = NAN;
-            if (n > 1 && s1 > 0.0) {
-                const double mean = s1 / n;
-                const double var = fmax(0.0, (s2 - n * mean * mean) / (n - 1));
-                se = sqrt(n * var) / s1;
-            }
-            r.rel_se = se;
-            r.valid = nv;
-            r.failed = nf;
-            r.clamped = nc;
-            *out = r;
+            *out = reduce_result(mx, s1, s2, n, nv, nf, nc);
         }
     }
+}
+
+// The same reduction of one pass's chains by a cluster of 8 CTAs, for the passes of many chains: one CTA
+// makes two passes over them and an FP64 power of ten each on one SM. 16384 chains 17.8 -> 7.4 us, 40000 37.7 -> 10.0;
+// both take 6.7 at 4096, where the line lies (3072: 5.9 by one CTA, 6.7 by the cluster, whose CTAs start and meet later).
+constexpr int kReduceCtas = 8;
+constexpr uint32_t kReduceClusterFrom = 4096;
+
+struct ReducePart {
+    double mx, s1, s2;
+    unsigned long long nv, nf, nc;
+};
+
+__global__ void __cluster_dims__(kReduceCtas, 1, 1) __launch_bounds__(1024)
+reduce_cluster_kernel(const ChainOut *__restrict__ chains, uint32_t n, ReduceOut *__restrict__ out)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ ReducePart s_warp[32], s_cta;
+    __shared__ double s_max;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const uint32_t t0 = cl.block_rank() * blockDim.x + threadIdx.x, tn = kReduceCtas * blockDim.x;
+    double mx = -INFINITY;
+    for (uint32_t i = t0; i < n; i += tn) mx = fmax(mx, chains[i].log10_sum);
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (l == 0) s_warp[w].mx = mx;
+    __syncthreads();
+    if (w == 0) {
+        mx = s_warp[l].mx;
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (l == 0) s_max = mx;
+    }
+    cl.sync();
+    for (int r = 0; r < kReduceCtas; ++r) mx = fmax(mx, *cl.map_shared_rank(&s_max, r));
+    ReducePart p{mx, 0.0, 0.0, 0, 0, 0};
+    double c1 = 0.0;
+    for (uint32_t i = t0; i < n; i += tn) {
+        const ChainOut ch = chains[i];
+        if (mx > -INFINITY) {
+            const double x = (ch.log10_sum > -INFINITY) ? exp10(ch.log10_sum - mx) : 0.0;
+            const double y = x - c1, t = p.s1 + y;
+            c1 = (t - p.s1) - y;
+            p.s1 = t;
+            p.s2 += x * x;
+        }
+        p.nv += ch.valid;
+        p.nf += ch.failed;
+        p.nc += ch.clamped;
+    }
+    p.s1 -= c1;
+    auto fold = [&] {
+        for (int o = 16; o > 0; o >>= 1) {
+            p.s1 += __shfl_xor_sync(0xffffffffu, p.s1, o);
+            p.s2 += __shfl_xor_sync(0xffffffffu, p.s2, o);
+            p.nv += __shfl_xor_sync(0xffffffffu, p.nv, o);
+            p.nf += __shfl_xor_sync(0xffffffffu, p.nf, o);
+            p.nc += __shfl_xor_sync(0xffffffffu, p.nc, o);
+        }
+    };
+    fold();
+    if (l == 0) s_warp[w] = p;
+    __syncthreads();
+    if (w == 0) {
+        p = s_warp[l];
+        fold();
+        if (l == 0) s_cta = p;
+    }
+    cl.sync();
+    if (t0 == 0) {
+        for (int r = 1; r < kReduceCtas; ++r) {
+            const ReducePart &q = *cl.map_shared_rank(&s_cta, r);
+            p.s1 += q.s1;
+            p.s2 += q.s2;
+            p.nv += q.nv;
+            p.nf += q.nf;
+            p.nc += q.nc;
+        }
+        *out = reduce_result(mx, p.s1, p.s2, n, p.nv, p.nf, p.nc);
+    }
+    cl.sync();   // the CTAs' shared memory stays until it has been read
 }
 
 // ------------------------------------------------------------------------------------
@@ -542,7 +629,8 @@ cudaError_t launch_fp64_chains(const ChainSpec &c, const float *init_pos, double
 
 cudaError_t launch_reduce(const ChainOut *chains, uint32_t n, ReduceOut *out, cudaStream_t st)
 {
-    reduce_kernel<<<1, 1024, 0, st>>>(chains, n, out, nullptr);
+    if (n >= kReduceClusterFrom) reduce_cluster_kernel<<<kReduceCtas, 1024, 0, st>>>(chains, n, out);
+    else reduce_kernel<<<1, 1024, 0, st>>>(chains, n, out, nullptr);
     return cudaGetLastError();
 }
 
