@@ -706,8 +706,18 @@ void prepare(twisty_ctx *ctx, const twisty_bc *bcp, bool wait = true)
             ctx->tuning.lut_global = 1;
         }
         fit_table_smem(ctx->tuning, p.num_curvature_steps, p.comp_warps == 0);
-        if (!requested)
-            requested = (uint32_t)ctx->sm_count * (uint32_t)ctx->tuning.warps_per_block * (32u / (uint32_t)ctx->tuning.group);
+        if (!requested) {
+            const uint32_t per_warp = 32u / (uint32_t)ctx->tuning.group;
+            requested = (uint32_t)ctx->sm_count * (uint32_t)ctx->tuning.warps_per_block * per_warp;
+            // fewer paths than the grid has chains: a path per chain, on CTAs of just enough warps to
+            // reach every SM: they share its pipes with fewer others (N = 16, 2^14 paths: 14 warps on
+            // 147 SMs, not 32 on 64: 91 -> 54 us; N = 66, 2^12 paths: 123 -> 59). The chains are the same ones.
+            if (!p.comp_warps && p.paths_to_generate < requested) {
+                const uint64_t grid = (uint64_t)ctx->sm_count * per_warp;
+                const uint64_t need = std::max<uint64_t>((p.paths_to_generate + grid - 1) / grid, 1);
+                ctx->tuning.warps_per_block = (int)std::min<uint64_t>(need, (uint64_t)ctx->tuning.warps_per_block);
+            }
+        }
     } else {
         if (!requested) requested = (uint32_t)ctx->sm_count * 256;
     }
