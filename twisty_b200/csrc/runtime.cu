@@ -1682,6 +1682,15 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         const uint32_t cpb = (uint32_t)batch_chains_per_block(sh);
         for (uint32_t c0 = 0; c0 < h.spec.n_chains; c0 += cpb) bk.items.push_back(make_uint2(e, c0));
     }
+    // buckets start in the order of their longest item: a shape whose items run for most of the pass
+    // takes its SMs first, and the short items fill what is left (one after another in the
+    // order the experiments happened to come, the last long bucket set the end of the pass)
+    auto longest = [&](const Bucket &bk) {
+        double m = 0.0;
+        for (uint32_t e : bk.exps) m = std::max(m, ((double)eh[e].spec.burn_in + eh[e].spec.steps) * eh[e].N);
+        return m;
+    };
+    std::stable_sort(buckets.begin(), buckets.end(), [&](const Bucket &a, const Bucket &b) { return longest(a) > longest(b); });
     std::vector<uint2> items;
     for (Bucket &bk : buckets) {
         // longest work first: cost of an item ~ (burn-in + steps) x N
