@@ -40,3 +40,23 @@ def test_exported_points(N, chains, paths, zero):
     end = d[:, -1] - d[0, -1]
     assert np.abs(end).max() <= 43 * N * 2.0 ** -20 * S / N
     assert np.unique(d.reshape(d.shape[0], -1), axis=0).shape[0] > 1
+
+
+@pytest.mark.parametrize("chains", [5, 700, 0])
+def test_replay_beside_the_pass(chains):
+    """The replay runs beside the pass: exports that grow, shrink and take every chain, with passes between them on
+    one context, give the bits of fresh contexts, and the pass's result is the plain run's."""
+    N, S = 66, 7.92
+    p = T.default_params(num_segments=N, mu=1.0, eps=0.01, scatter=10.0, num_steps_int=2000, num_curvature_steps=1024,
+                         num_chains=chains, paths_to_generate=6000, paths_to_skip=11, max_sub_chain=32, max_angle=0.1, perturb_seed=8)
+    bcs = [T.make_bc((0, 0, 0), (0, 0, 1), (0, 0, f * S), (0, 0, 1), S) for f in (0.6, 0.7)]
+    with T.Context(p) as ctx:
+        for i, n in enumerate((1, 3000, 10, 6000, 6000, 1200)):
+            bc = bcs[i % 2]
+            pos, w, r = ctx.export_paths(bc, None, n)
+            q = ctx.run(bc)
+            with T.Context(p) as fresh:
+                pos2, w2, r2 = fresh.export_paths(bc, None, n)
+            assert w.size == n and np.array_equal(pos, pos2) and np.array_equal(w, w2)
+            assert r.log10_weight == r2.log10_weight == q.log10_weight and r.total_paths == q.total_paths == 6000
+            assert r.rel_std_error == q.rel_std_error and r.num_chains == q.num_chains

@@ -239,6 +239,7 @@ struct twisty_ctx {
     int sm_count = 148;
     std::string name;            // of the device, once the tuning cache needed it
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr; // an export's replay, beside the pass; made by the first one
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::string err;
 
@@ -1116,6 +1117,7 @@ void twisty_destroy(twisty_ctx *ctx)
     ctx->upload.release();
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -1982,9 +1984,14 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
         prepare(ctx, bc, false);
         launch(ctx, ctx->stream);
         twisty_result r{};
-        collect(ctx, &r);
         const ChainSpec &c = ctx->spec;
         const uint32_t N = c.n_segments;
+        // The compensated replay shares nothing with the pass but its tables and initial segments, which are there at
+        // the pass's first event, and keeps a few warps busy: it runs beside the pass, on a stream of its own
+        // that is drained before the call returns (N = 128, 2048 chains: pass 353 us, replay 510). The plain form's replay
+        // uses the pass's chain state and follows it.
+        const bool beside = ctx->p.form == TWISTY_FORM_COMPENSATED && !c.has_eval_shift && max_paths > 0 && c.n_chains > 0;
+        if (!beside) collect(ctx, &r);
         const size_t stride = 3 * (size_t)(N + 1);
         std::vector<float> hpos;
         std::vector<double> hw;
@@ -2000,6 +2007,19 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
             cudaStream_t st = ctx->stream;
             DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dout = ctx->call.c;
             const Trim trim{ctx->call};
+            struct Drain {   // before the buffers can go or serve another call
+                cudaStream_t s;
+                ~Drain()
+                {
+                    if (s) cudaStreamSynchronize(s);
+                }
+            };
+            if (beside) {
+                if (!ctx->side) ck(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking), "stream");
+                st = ctx->side;
+                ck(cudaStreamWaitEvent(st, ctx->ev[0], 0), "export");
+            }
+            const Drain drain{ctx->side};
             ck(dpos.ensure(sizeof(float) * stride * npaths), "alloc export buffer");
             ck(dw.ensure(sizeof(double) * npaths), "alloc export buffer");
             ck(dout.ensure(sizeof(ChainOut) * E), "alloc export buffer");
@@ -2048,6 +2068,7 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
                 ck(cudaStreamSynchronize(st), "export");
             }
         }
+        if (beside) collect(ctx, &r);
         const uint64_t n = hw.size();
         if (pos && dir && n) std::memcpy(pos, hpos.data(), sizeof(float) * hpos.size());
         if (log10w && n) std::memcpy(log10w, hw.data(), sizeof(double) * n);
