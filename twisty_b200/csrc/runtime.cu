@@ -1681,8 +1681,6 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
             fail(TWISTY_ERR_UNSUPPORTED, exp_msg(e, "no batched kernel shape fits"));
         Bucket &bk = bucket_of(sh);
         bk.exps.push_back(e);
-        const uint32_t cpb = (uint32_t)batch_chains_per_block(sh);
-        for (uint32_t c0 = 0; c0 < h.spec.n_chains; c0 += cpb) bk.items.push_back(make_uint2(e, c0));
     }
     // buckets start in the order of their longest item: a shape whose items run for most of the pass
     // takes its SMs first, and the short items fill what is left (one after another in the
@@ -1693,8 +1691,29 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         return m;
     };
     std::stable_sort(buckets.begin(), buckets.end(), [&](const Bucket &a, const Bucket &b) { return longest(a) > longest(b); });
+    double all = 0.0;   // the pass's chain steps x segments
+    for (const ExpHost &h : eh) all += ((double)h.spec.burn_in + h.spec.steps) * h.N * h.spec.n_chains;
     std::vector<uint2> items;
     for (Bucket &bk : buckets) {
+        // an item holds a CTA's worth of an experiment's chains; where one alone is more than two SMs' even share of the
+        // pass, smaller CTAs (of 3 warps or more) spread its chains over more SMs. Measured, calls of N = 16..1024 and
+        // 2^14 paths each: 128 experiments 3.2 -> 2.9 ms, 256 3.5 -> 3.1, 32 of N = 700..1000 3.0 -> 2.3; 64 of 2^16
+        // paths 5.9 -> 4.6. A line at 1 or 1.3 shares slows other calls by up to 10 % (200 of N = 16..200:
+        // 1.52 -> 1.68, the table staged more often), at 3 it misses the 256.
+        auto heaviest = [&] {
+            double m = 0.0;
+            for (uint32_t e : bk.exps) {
+                const ChainSpec &c = eh[e].spec;
+                m = std::max(m, ((double)c.burn_in + c.steps) * eh[e].N *
+                                    std::min(c.n_chains, (uint32_t)batch_chains_per_block(bk.shape)));
+            }
+            return m;
+        };
+        while (bk.shape.warps >= 6 && heaviest() > 2.0 * all / ctx->sm_count)
+            bk.shape.warps = (bk.shape.warps + 1) / 2;
+        const uint32_t cpb = (uint32_t)batch_chains_per_block(bk.shape);
+        for (uint32_t e : bk.exps)
+            for (uint32_t c0 = 0; c0 < eh[e].spec.n_chains; c0 += cpb) bk.items.push_back(make_uint2(e, c0));
         // longest work first: cost of an item ~ (burn-in + steps) x N
         std::stable_sort(bk.items.begin(), bk.items.end(), [&](const uint2 &a, const uint2 &b) {
             const ExpHost &x = eh[a.x], &y = eh[b.x];
