@@ -84,12 +84,25 @@ __global__ void __launch_bounds__(MAXT, 1) comp_chain_kernel(ChainSpec c, CompCo
 }
 
 // ------------------------------------------------------------------------------ launchers
+// The fixed-point forward kernels of 28 and 32 segments on 32 lanes are compiled twice: for the up to 16 warps that
+// their defaults run (12 to 16: shared memory holds no more beside the table), with 128 registers, and for
+// the 18 or 20 that an explicit shape or a tuned one may ask for, with 80. Under 80 registers the loads of a
+// lane's segments queue behind one another: N = 1024 3.76 -> 3.29 ms (2^22 paths, 8192 bins), 900
+// 3.73 -> 3.59, 896 (table through L1) 3.24 -> 2.90, 800 3.49 -> 3.19; 96 registers measured between or below.
+constexpr int kWideThreads = 512;
+template <int G, int SPL, bool EXACT, int MODE>
+constexpr bool wide_registers() { return G == 32 && SPL >= 28 && MODE == kModeForward && !EXACT; }
+
 template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INCR = false, bool STEEP = false,
-          bool LUTG = false>
+          bool LUTG = false, int MAXT = MODE == kModeAdjoint ? kAdjointThreads : comp_max_threads(G, SPL)>
 cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const float *init_seg, const float2 *tab,
                      ChainOut *out, double2 *partials, const ModeArgs &ma, size_t smem, uint32_t blocks, cudaStream_t st)
 {
-    constexpr int MAXT = MODE == kModeAdjoint ? kAdjointThreads : comp_max_threads(G, SPL);
+    if constexpr (wide_registers<G, SPL, EXACT, MODE>() && MAXT > kWideThreads) {
+        if (warps * 32 <= kWideThreads)
+            return launch_t<G, SPL, EXACT, CLAMP, SHIFT, MODE, INCR, STEEP, LUTG, kWideThreads>(c, kc, warps, init_seg, tab, out, partials,
+                                                                                                 ma, smem, blocks, st);
+    }
     if (warps * 32 > MAXT) return cudaErrorInvalidConfiguration;
     auto kern = comp_chain_kernel<G, SPL, EXACT, CLAMP, SHIFT, MAXT, MODE, INCR, STEEP, LUTG>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
