@@ -348,9 +348,9 @@ class FullExperimentRunnerOptimalPerturb : public ExperimentRunner {
     explicit FullExperimentRunnerOptimalPerturb(ExperimentParameters &p) : ExperimentRunner(p) {}
 };
 
-// Drop-in for twisty::FullExperimentRunnerOptimalPerturbOptimized_GPU, whose kernel design
-// (one chain per thread, state in global memory, FP64 log10 per segment) the plain FP32
-// form reproduces; the form the parameters select is used, so both names run the same code.
+// Drop-in for twisty::FullExperimentRunnerOptimalPerturbOptimized_GPU, whose arithmetic
+// (one chain per thread, FP32 state, FP64 log weights) the plain FP32 form reproduces, several
+// lanes to a chain; the form the parameters select is used, so both names run the same code.
 class FullExperimentRunnerOptimalPerturbOptimized_GPU : public ExperimentRunner {
    public:
     explicit FullExperimentRunnerOptimalPerturbOptimized_GPU(ExperimentParameters &p) : ExperimentRunner(p) {}
