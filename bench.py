@@ -362,7 +362,7 @@ def run_image_workload(args, T, torch, device, ws, rank, pg):
                    "d_log10_total_d_sigma": float(total[2]),
                    "replay_path_segments_per_s": sum(r.total_paths * I["N"] for r in res) / (float(tms[1]) / 1e3),
                    "note": "call = forward pass + derivative tables + adjoint replay; replay recomputes every "
-                           "curvature (exact blend) and stores nothing per step"}
+                           "curvature and stores nothing per step"}
     if pg:
         t = torch.tensor([per_step, e2e_ms], dtype=torch.float64, device=f"cuda:{device}")
         pg.all_reduce(t, op=pg.ReduceOp.MAX)
