@@ -8,6 +8,7 @@
 #include "host_util.h"
 #include "../../include/twisty_b200.h"
 
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -1832,24 +1833,30 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
     if (!adj) return;
 
     // ---- adjoint replay of the same chains (twisty_adjoint_batch)
-    // derivative tables d/d(mu_s), d/d(eps) in FP64 on the device: one per experiment, or one per
-    // table of the multi-ds set the experiments take theirs from
-    const uint32_t ntab = multi ? ctx->multi.n : n;
-    ck(B.dtab.ensure(sizeof(float4) * (size_t)bins * ntab), "alloc derivative tables");
-    // the replay takes the fixed-point table where it has no steep bins (the same for all
-    // experiments of a table: steepness and range are the table's)
+    // Derivative tables d/d(mu_s), d/d(eps) in FP64 on the device, one per table that experiments weigh with (their
+    // own, or one of the multi-ds set) and replay that reads it: the fixed-point replay takes the ratio form, the
+    // exact blend the linear one. Which replay an experiment takes is its own matter, not its table's: it may
+    // leave the curvature range of a table that a longer-ds experiment stays within, and the fixed
+    // point is scaled for its N.
     auto fixed_of = [&](uint32_t e) { return okv[e] != 0 && comp_adjoint_fixed(lf[e], eh[e].spec.inv_ds, eh[e].meta); };
     std::vector<DerivJob> jobs;
     std::vector<LutBuildSpec> dspecs;
-    std::vector<char> have(ntab, 0);
+    std::vector<uint32_t> job_of(n);
+    constexpr uint32_t kNone = 0xffffffffu;
+    std::vector<std::array<uint32_t, 2>> made(multi ? ctx->multi.n : n, {kNone, kNone});   // [table][ratio]
     for (uint32_t e = 0; e < n; ++e) {
         const uint32_t t = multi ? eh[e].multi_index : e;
-        if (have[t]) continue;
-        have[t] = 1;
-        const float *lut = multi ? ctx->multi.dev.as<float>() + (size_t)t * bins : B.lut32.as<float>() + (size_t)t * bins;
-        jobs.push_back(DerivJob{lut, B.dtab.as<float4>() + (size_t)t * bins, (uint32_t)dspecs.size(), fixed_of(e) ? 1 : 0});
-        dspecs.push_back(multi ? table_spec(p, ctx->multi.ds[t]) : specs[e]);
+        const int32_t ratio = fixed_of(e) ? 1 : 0;
+        if (made[t][ratio] == kNone) {
+            const float *lut = (multi ? ctx->multi.dev.as<float>() : B.lut32.as<float>()) + (size_t)t * bins;
+            made[t][ratio] = (uint32_t)jobs.size();
+            jobs.push_back(DerivJob{lut, nullptr, (uint32_t)dspecs.size(), ratio});
+            dspecs.push_back(multi ? table_spec(p, ctx->multi.ds[t]) : specs[e]);
+        }
+        job_of[e] = made[t][ratio];
     }
+    ck(B.dtab.ensure(sizeof(float4) * (size_t)bins * jobs.size()), "alloc derivative tables");
+    for (size_t k = 0; k < jobs.size(); ++k) jobs[k].out = B.dtab.as<float4>() + k * bins;
     ck(B.djobs.ensure(sizeof(DerivJob) * jobs.size()), "alloc derivative tables");
     ck(B.dspecs.ensure(sizeof(LutBuildSpec) * dspecs.size()), "alloc derivative tables");
     ck(cudaMemcpyAsync(B.djobs.p, jobs.data(), sizeof(DerivJob) * jobs.size(), cudaMemcpyHostToDevice, st), "upload");
@@ -1874,10 +1881,9 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         const bool fixed = fixed_of(e);
         bx[e].lf = fixed ? lf[e] : LogFixed{0.0, 0.0, 0, 0};
         bx[e].tab = (fixed ? B.fix.as<float2>() : B.lin.as<float2>()) + (size_t)e * bins;
-        const uint32_t t = multi ? h.multi_index : e;
         const double log10_abs = std::log10(h.spec.absorption_factor);
         const bool ok = red[e].valid > 0 && std::isfinite(red[e].log10_sum);
-        ax[e] = BatchAdjHost{B.dtab.as<float4>() + (size_t)t * bins,
+        ax[e] = BatchAdjHost{jobs[job_of[e]].out,
                              ok ? red[e].log10_sum - (double)(h.N - 1) * log10_abs : 0.0};
         if (h.spec.n_chains == 0) continue;
         BatchShape sh{h.t.group, h.t.spl, std::min(h.t.warps_per_block, kAdjointThreads / 32), fixed ? 0 : 1, 1, fixed ? 0 : 1, 0};
