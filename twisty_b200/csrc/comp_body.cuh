@@ -692,15 +692,15 @@ __device__ __forceinline__ void stage_table(float4 *smem4, const float2 *__restr
 }
 
 // Exact-blend weight of the group's current path through the linear table, for paths of a
-// fixed-point table that cross a steep bin. Not inlined: it runs rarely, and inlined its
-// registers would count against the hot loop's.
+// fixed-point table that cross a steep bin: in segment order, as every exact blend sums. Not
+// inlined: it runs rarely, and inlined its registers would count against the hot loop's.
 template <int G, int SPL, bool CLAMP>
 __device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j, uint32_t N,
                                               const float2 *__restrict__ lin, CompConsts kc)
 {
     const SmemLoad<G, SPL> load{st, qb, j, 0, nullptr, 0.f, 0.f};
     uint32_t unused = 0;
-    return path_log10<G, SPL, true, CLAMP, true>(j, N, lin, kc, load, ShflNext<G>{}, [](uint32_t, int32_t) {}, unused);
+    return path_log10<G, SPL, true, CLAMP, true, false>(j, N, lin, kc, load, ShflNext<G>{}, [](uint32_t, int32_t) {}, unused);
 }
 
 // One Markov chain run by the G lanes of one group on its own records st (tangent, length;
