@@ -107,10 +107,12 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restri
         ma.log10_abs = e.log10_abs;
         ma.lin = e.lin;
         const uint32_t chain = it.y + warp * CPW + q;
-        chain_body<G, SPL, EXACT, CLAMP, false, kModeForward, false, STEEP, !LUT_SMEM>(e.spec, e.kc, e.init_seg, tab, st,
-                                                                                       Lanes<G>::base_of(lane), j,
-                                                                            chain, chain < e.spec.n_chains,
-                                                                            out + e.out_offset, ma);
+        // the exact blend keeps PAIRS at 32 lanes here: after an item's split few warps are left to hide its loads
+        // (16 experiments of 2^14 paths, N = 512: 10.6 ms against 14.5 in XYZ, 1024: 35.6 against 51.7; 256 of
+        // them: 888 against 882, 1841 against 2013)
+        chain_body<G, SPL, EXACT, CLAMP, false, kModeForward, false, STEEP, !LUT_SMEM, false>(
+              e.spec, e.kc, e.init_seg, tab, st, Lanes<G>::base_of(lane), j, chain, chain < e.spec.n_chains,
+              out + e.out_offset, ma);
         __syncthreads();
     }
 }

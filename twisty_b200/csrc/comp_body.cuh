@@ -281,11 +281,13 @@ __device__ __forceinline__ F2 bins_of(F2 qq, const CompConsts &k, int32_t &L0, i
 // 701 +5 %, but 16 x 16 -5 % (more bank conflicts in the rotation, which that shape's
 // shared-memory pipe at 90 % of its wavefronts pays for) and 8 x 16 -8 % (spills); PLANES
 // at 4 lanes N = 64 +17 %, 66 +13 %, at one lane N = 16 +2 %, but under the 64 registers of the 4-lane
-// shapes below 12 segments per lane -4 to -7 % (N = 18, 30, 34).
+// shapes below 12 segments per lane -4 to -7 % (N = 18, 30, 34). ORDERED: a recompute that
+// walks its segments in order (the exact blend of single runs) would keep the later halves of PAIRS in registers, and
+// spills: N = 544 351 -> 324 us over 2^19 paths in XYZ, 768 371 -> 306, 1024 439 -> 330, receiver-shifted 669 -> 426.
 enum { kPairs = 0, kXyz = 1, kPlanes = 2 };
-__host__ __device__ constexpr int comp_layout(int G, int SPL)
+__host__ __device__ constexpr int comp_layout(int G, int SPL, bool ordered = false)
 {
-    return G == 32 ? kPairs : G == 1 || (G == 4 && SPL >= 12) ? kPlanes : kXyz;
+    return G == 32 ? (ordered ? kXyz : kPairs) : G == 1 || (G == 4 && SPL >= 12) ? kPlanes : kXyz;
 }
 // Whether the recompute works on pairs of segments with packed arithmetic.
 __host__ __device__ constexpr bool comp_packed(int G, int SPL) { return comp_layout(G, SPL) != kXyz; }
@@ -513,9 +515,9 @@ struct Slot {
 //  * PLANES: x, y and z in rows of 32 floats, the column rotated by the row: 4 consecutive
 //    segments of a 4-lane chain lie in the chain's own 4 banks where SPL = 1 mod 4 (and mostly so for
 //    other SPL), and every access of a one-lane chain in its own bank.
-template <int G, int SPL>
+template <int G, int SPL, bool ORDERED = false>
 struct Layout {
-    static constexpr int KIND = comp_layout(G, SPL);
+    static constexpr int KIND = comp_layout(G, SPL, ORDERED);
     static constexpr int H = (SPL + 1) / 2;
     static constexpr bool ODD = SPL & 1;
     static constexpr int CPW = 32 / G;
@@ -587,23 +589,23 @@ struct Planes {
 };
 
 // The tangents of lane j of the chain in slot q, for for_curvatures. SHIFT: the weights see the
-// receiver moved by `shift`: v_{N-2} = l t + shift, renormalised.
-template <int G, int SPL, bool SHIFT = false>
+// receiver moved by the spec's eval_shift: v_{N-2} = l t + shift, renormalised.
+template <int G, int SPL, bool SHIFT = false, bool ORDERED = false>
 struct SmemLoad {
-    using Lay = Layout<G, SPL>;
+    using Lay = Layout<G, SPL, ORDERED>;
     const Planes &st;
     uint32_t qb, j;
-    uint32_t moved;       // SHIFT: segment N - 2
-    const float *shift;
+    uint32_t N;
+    const ChainSpec *c;   // SHIFT (through a copy of its members the shifted passes ran up to 20 % slower)
     float kscale, inv_ks;
     __device__ __forceinline__ void one(int m, float &x, float &y, float &z) const
     {
         Lay::get(st.t, Lay::slot(j, m, qb), x, y, z);
-        if (SHIFT && j * SPL + m == moved) {
+        if (SHIFT && j * SPL + m == N - 2) {
             const float l = st.l[j * SPL + m] * inv_ks;
-            x = fmaf(l, x, shift[0]);
-            y = fmaf(l, y, shift[1]);
-            z = fmaf(l, z, shift[2]);
+            x = fmaf(l, x, c->eval_shift[0]);
+            y = fmaf(l, y, c->eval_shift[1]);
+            z = fmaf(l, z, c->eval_shift[2]);
             const float r = rsqrtf(fmaf(x, x, fmaf(y, y, z * z))) * kscale;
             x *= r; y *= r; z *= r;
         }
@@ -710,7 +712,7 @@ __device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j
 // STEEP: the fixed-point table has steep bins (NaN slopes); paths crossing one are re-weighed
 // through ma.lin. Without it a NaN slope cannot occur and a NaN total means a NaN curvature.
 template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INCR = false, bool STEEP = false,
-          bool TAB_GLOBAL = false>
+          bool TAB_GLOBAL = false, bool ORDERED = EXACT && MODE != kModeAdjoint>
 __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConsts &kc,
                                              const float *__restrict__ init_seg, const float2 *s_tab, Planes st,
                                              uint32_t qb, uint32_t j, uint32_t chain, bool real_chain,
@@ -719,7 +721,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
     constexpr bool FIX = !EXACT;
     constexpr bool ADJ = MODE == kModeAdjoint;
     const uint32_t N = c.n_segments;
-    using Lay = Layout<G, SPL>;
+    using Lay = Layout<G, SPL, ORDERED>;
     // segment record (tangent, length) of segment index s = owner*SPL + m
     // the tangents are stored at length kscale; records handed to export and the adjoint are unit
     const float inv_ks = 1.0f / kc.kscale;
@@ -803,7 +805,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
         return __float_as_uint(e.x) + (uint32_t)__float2int_rn(cor * kc.fscale);
     };
 
-    const SmemLoad<G, SPL, SHIFT> load_smem{st, qb, j, N - 2, c.eval_shift, kc.kscale, inv_ks};
+    const SmemLoad<G, SPL, SHIFT, ORDERED> load_smem{st, qb, j, N, &c, kc.kscale, inv_ks};
     const ShflNext<G> next_smem{};
     // adjoint with the fixed-point table: the reference as a path total, and the tangents and weight of the
     // step whose receiver gradient this lane works out
