@@ -171,7 +171,7 @@ cudaError_t batch_adjoint_t(const BatchShape &s, const BatchExp *exps, const Bat
 {
     if (s.warps * 32 > kAdjointThreads) return cudaErrorInvalidConfiguration;
     auto kern = batch_adjoint_kernel<G, SPL, EXACT, kAdjointThreads>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = grant_smem(kern, smem);
     if (e != cudaSuccess) return e;
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, s.warps * 32, smem);
     kern<<<grid, s.warps * 32, smem, st>>>(exps, adj, items, n_items, counter, grad, bins);
@@ -194,7 +194,7 @@ cudaError_t batch_t(const BatchShape &s, const BatchExp *exps, const uint2 *item
     constexpr int MAXT = batch_max_threads(G, SPL);
     if (s.warps * 32 > MAXT) return cudaErrorInvalidConfiguration;
     auto kern = batch_kernel<G, SPL, EXACT, LS, CL, SP, MAXT>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = grant_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, s.warps * 32, smem, st>>>(exps, items, n_items, counter, out, bins);
     return cudaGetLastError();
@@ -205,7 +205,7 @@ int batch_occ_t(const BatchShape &s, size_t smem)
 {
     constexpr int MAXT = batch_max_threads(G, SPL);
     auto kern = batch_kernel<G, SPL, EXACT, LS, CL, SP, MAXT>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    if (grant_smem(kern, smem) != cudaSuccess) return 0;
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, s.warps * 32, smem) != cudaSuccess) return 0;
     return nb;

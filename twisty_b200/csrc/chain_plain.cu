@@ -262,7 +262,7 @@ cudaError_t launch_plain_t(const ChainSpec &c, const float *init_pos, float *sta
     const size_t smem = SMEM ? sizeof(float) * (size_t)stride * per_block : 0;
     auto kern = plain_chain_kernel<G, SMEM>;
     if (SMEM) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = grant_smem(kern, smem);
         if (e != cudaSuccess) return e;
     }
     kern<<<blocks, kPlainThreads, smem, st>>>(c, init_pos, state, stride, lut, m, out, exp_pos, exp_w);

@@ -105,7 +105,7 @@ cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const 
     }
     if (warps * 32 > MAXT) return cudaErrorInvalidConfiguration;
     auto kern = comp_chain_kernel<G, SPL, EXACT, CLAMP, SHIFT, MAXT, MODE, INCR, STEEP, LUTG>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = grant_smem(kern, smem);
     if (e != cudaSuccess) return e;
     if (LUTG) {
         // the table is gathered through L1: ask for no more shared memory than the one CTA per SM

@@ -148,6 +148,20 @@ bool comp_tuning_supported(const CompTuning &t, uint32_t n_segments, uint32_t k_
 size_t comp_smem_bytes(const CompTuning &t, uint32_t bins);
 // Shared memory a CTA may use (B200: 227 KB).
 constexpr size_t kCompSmemCap = 227 * 1024;
+// Lets `kern` be launched with smem bytes of dynamic shared memory, by granting it all that a CTA may use beside
+// its static part: the limit belongs to the function on its device, so a launch on another thread, in another
+// context, may need more of it, or less, between this call and the launch.
+template <class Kernel>
+cudaError_t grant_smem(Kernel kern, size_t smem)
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return e;
+    const size_t most = kCompSmemCap - a.sharedSizeBytes;
+    if (smem > most) return cudaErrorInvalidValue;
+    if ((size_t)a.maxDynamicSharedSizeBytes == most) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 // Table placement of a forward pass of the full recompute: true when the table is gathered
 // through L1 at the shape's warps, because staging it would leave fewer than
 // comp_stage_min_warps(t) warps (or does not fit at all). may_shrink false: the warps were set
