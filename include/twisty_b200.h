@@ -224,7 +224,11 @@ twisty_status twisty_params_from_config(const char *text, int is_yaml, twisty_pa
 
 /* --------------------------------------------------------------- context */
 /* ExperimentRunner(ExperimentParameters&) ctor (Twisty/ExperimentRunner.cpp:180-192);
- * the params are copied. Selects and initialises the CUDA device. */
+ * the params are copied. Selects and initialises the CUDA device. A context keeps its device
+ * memory between calls: tables and chain results of its passes, the buffers of its batches (as
+ * large as its largest batch), up to 256 MB of buffers of the other calls (paths weighed or
+ * exported, gradients) and up to 512 MB of the M-segment estimator's (its columns of points); 4 MB
+ * of pinned host memory serve large uploads. twisty_destroy gives all of it back. */
 twisty_status twisty_create(const twisty_params *p, twisty_ctx **out);
 void twisty_destroy(twisty_ctx *ctx);
 const char *twisty_last_error(const twisty_ctx *ctx);

@@ -171,35 +171,44 @@ struct BatchBufs {
     }
 };
 
-// Device buffers of the calls that used to allocate and free theirs (a cudaMalloc or cudaFree waits for
-// the device: 0.1-0.3 ms each), kept by the context; the ones above kKeepBytes are given back when the
-// call ends.
-struct CallBufs {
-    static constexpr size_t kKeepBytes = 256ull << 20;
-    DevBuf a, b, c, d;
+// Device buffers that a context keeps between calls, because a cudaMalloc or cudaFree waits for the device
+// (0.1-0.3 ms each). When a call ends, the largest are given back until the rest fit `keep`, so a context's share
+// of the device stays bounded whatever it has run; the rest goes with the context.
+template <int N>
+struct KeptBufs {
+    DevBuf bufs[N];
     void release()
     {
-        for (DevBuf *x : {&a, &b, &c, &d}) x->release();
+        for (DevBuf &x : bufs) x.release();
     }
-    void trim()
+    void trim(size_t keep)
     {
-        for (DevBuf *x : {&a, &b, &c, &d})
-            if (x->bytes > kKeepBytes) x->release();
+        for (;;) {
+            size_t all = 0;
+            DevBuf *largest = bufs;
+            for (DevBuf &x : bufs) {
+                all += x.bytes;
+                if (x.bytes > largest->bytes) largest = &x;
+            }
+            if (all <= keep) return;
+            largest->release();
+        }
     }
 };
+struct CallBufs : KeptBufs<4> {
+    static constexpr size_t kKeep = 256ull << 20;
+    DevBuf &a = bufs[0], &b = bufs[1], &c = bufs[2], &d = bufs[3];
+};
+// Workspaces of the M-segment estimator: a column of points per thread of a launch (up to 384 MB,
+// msegment_threads), a sample per path of a launch (up to 64 MB), its slices.
+struct MSegBufs : KeptBufs<4> {
+    static constexpr size_t kKeep = 512ull << 20;
+    DevBuf &points = bufs[0], &samples = bufs[1], &red = bufs[2], &slices = bufs[3];
+};
+template <class Bufs>
 struct Trim {
-    CallBufs &b;
-    ~Trim() { b.trim(); }
-};
-
-// Workspaces of the M-segment estimator, kept by the context (a column of points per thread of a
-// launch, a sample per path of a launch, its slices).
-struct MSegBufs {
-    DevBuf points, samples, red, slices;
-    void release()
-    {
-        for (DevBuf *b : {&points, &samples, &red, &slices}) b->release();
-    }
+    Bufs &b;
+    ~Trim() { b.trim(Bufs::kKeep); }
 };
 
 // Outputs of the batched adjoint (twisty_adjoint_batch); every pointer nullable but grad.
@@ -1228,6 +1237,7 @@ twisty_status twisty_run_msegment(twisty_ctx *ctx, const twisty_bc *bc, twisty_r
         const uint64_t per_launch = std::min(std::min(chunk, kLaunch), std::max<uint64_t>(total, 1));
         const uint32_t threads = msegment_threads(N, per_launch);
         MSegBufs &B = ctx->mseg;
+        const Trim<MSegBufs> trim{B};
         ck(B.points.ensure(per_path * threads), "alloc points");
         ck(B.samples.ensure(sizeof(ChainOut) * per_launch), "alloc samples");
         ck(B.red.ensure(sizeof(ReduceOut) * std::max<size_t>(1, slices.size())), "alloc result");
@@ -1305,7 +1315,7 @@ twisty_status twisty_weight_paths(twisty_ctx *ctx, const twisty_bc *bc, const fl
         if (n_paths == 0) return;
         cudaStream_t st = ctx->stream;
         DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dv = ctx->call.c, &db = ctx->call.d;
-        const Trim trim{ctx->call};
+        const Trim<CallBufs> trim{ctx->call};
         const size_t np = 3 * (size_t)(N + 1) * n_paths;
         ck(dpos.ensure(sizeof(float) * np), "alloc paths");
         ck(dw.ensure(sizeof(double) * n_paths), "alloc weights");
@@ -2031,7 +2041,7 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
             const size_t npaths = (size_t)E * c.steps;
             cudaStream_t st = ctx->stream;
             DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dout = ctx->call.c;
-            const Trim trim{ctx->call};
+            const Trim<CallBufs> trim{ctx->call};
             struct Drain {   // before the buffers can go or serve another call
                 cudaStream_t s;
                 ~Drain()
@@ -2119,7 +2129,7 @@ twisty_status twisty_adjoint(twisty_ctx *ctx, const twisty_bc *bc, const twisty_
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
         DevBuf &dtab = ctx->call.a, &dg = ctx->call.b, &dout = ctx->call.c, &djob = ctx->call.d;
-        const Trim trim{ctx->call};
+        const Trim<CallBufs> trim{ctx->call};
         ck(dtab.ensure(sizeof(float4) * bins), "alloc");
         ck(dg.ensure(sizeof(double) * 6 * std::max<uint32_t>(c.n_chains, 1)), "alloc");
         ck(dout.ensure(sizeof(double) * 6), "alloc");
@@ -2162,7 +2172,7 @@ twisty_status twisty_weight_histogram(twisty_ctx *ctx, const twisty_bc *bc, doub
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
         DevBuf &dw = ctx->call.a, &dout = ctx->call.b, &dcnt = ctx->call.c;
-        const Trim trim{ctx->call};
+        const Trim<CallBufs> trim{ctx->call};
         ck(dcnt.ensure(sizeof(unsigned long long) * n_buckets), "alloc histogram");
         ck(cudaMemsetAsync(dcnt.p, 0, sizeof(unsigned long long) * n_buckets, st), "memset");
         if (c.n_chains) {
