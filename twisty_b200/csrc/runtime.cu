@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <functional>
 #include <limits>
+#include <map>
 #include <mutex>
 #include <new>
 #include <sstream>
@@ -247,7 +248,6 @@ struct twisty_ctx {
     twisty_params p{};
     int device = 0;
     int sm_count = 148;
-    std::string name;            // of the device, once the tuning cache needed it
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr; // an export's replay, beside the pass; made by the first one
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -348,13 +348,21 @@ struct TuneEntry {
 std::mutex g_tune_mu;
 std::vector<TuneEntry> g_tune;
 
-// The device's name, asked for only when the cache has entries to compare it with or to record
-// (cudaGetDeviceProperties takes 3.9 ms, which every context used to pay).
-std::string device_name(int device)
+// The device's name, asked for once per device, and only when the cache has entries to compare it with or to
+// record: cudaGetDeviceProperties takes 4 to 40 ms. It has a lock of its own, so that contexts on other threads
+// that need no name do not wait for the query.
+const std::string &device_name(int device)
 {
-    cudaDeviceProp prop{};
-    ck(cudaGetDeviceProperties(&prop, device), "device query");
-    return prop.name;
+    static std::mutex mu;
+    static std::map<int, std::string> names;   // its elements stay where they are
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = names.find(device);
+    if (it == names.end()) {
+        cudaDeviceProp prop{};
+        ck(cudaGetDeviceProperties(&prop, device), "device query");
+        it = names.emplace(device, prop.name).first;
+    }
+    return it->second;
 }
 
 void tune_record(const TuneEntry &e)
@@ -368,12 +376,16 @@ void tune_record(const TuneEntry &e)
     g_tune.push_back(e);
 }
 
-bool tune_lookup(twisty_ctx *ctx, uint32_t n, uint32_t bins, CompTuning &t)
+bool tune_lookup(const twisty_ctx *ctx, uint32_t n, uint32_t bins, CompTuning &t)
 {
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        if (std::none_of(g_tune.begin(), g_tune.end(), [&](const TuneEntry &x) { return x.n == n && x.bins == bins; })) return false;
+    }
+    const std::string &name = device_name(ctx->device);
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    if (!g_tune.empty() && ctx->name.empty()) ctx->name = device_name(ctx->device);
     for (const TuneEntry &x : g_tune)
-        if (x.n == n && x.bins == bins && x.device == ctx->name) {
+        if (x.n == n && x.bins == bins && x.device == name) {
             CompTuning c = t;
             c.group = (int)x.group;
             c.spl = (int)x.spl;
@@ -2307,8 +2319,7 @@ twisty_status twisty_autotune(twisty_ctx *ctx, const twisty_bc *bc, uint64_t tri
         ctx->p = saved;
         ctx->prepared = false;
         if (best_rate < 0) fail(TWISTY_ERR_UNSUPPORTED, "no shape ran: " + last_err);
-        if (ctx->name.empty()) ctx->name = device_name(ctx->device);
-        tune_record(TuneEntry{ctx->name, N, bins, (uint32_t)bestc.group, (uint32_t)bestc.spl,
+        tune_record(TuneEntry{device_name(ctx->device), N, bins, (uint32_t)bestc.group, (uint32_t)bestc.spl,
                               (uint32_t)bestc.warps, best_rate});
         best->num_segments = N;
         best->bins = bins;
