@@ -175,7 +175,7 @@ __device__ bool resolve_two(const PathPts &P, uint32_t l, uint32_t r, double ds,
 }
 
 // ResolveThreeSegments: the two points between l and l+3.
-__device__ bool resolve_three(const PathPts &P, uint32_t l, uint32_t r, double ds, Draws &g)
+__device__ __noinline__ bool resolve_three(const PathPts &P, uint32_t l, uint32_t r, double ds, Draws &g)
 {
     const F3 a = P.get(l), b = P.get(r);
     const float d = fmag(b - a);
@@ -272,19 +272,19 @@ struct MSegSpec {
     uint64_t n_paths;
 };
 
-// Places the points of one path; false when the reference would abort.
+// Places the points of one path; false when the reference would abort. N - 2 = LEAF << depth (the host validated N - 2 as
+// resolvable). LEAF, 4 or 6, is the kernel's, a leaf's two halves share their code, and resolve_three is called, not
+// inlined: with both kinds of leaves inlined twice in one kernel, compensated paths waited for their instructions
+// (2^26 path-segments, N = 66 2.04 -> 1.76 ms, 98 3.40 -> 2.49, 386 5.35 -> 3.30, 770 8.33 -> 5.05; plain 2.22 -> 2.15,
+// 3.13 -> 3.02, 4.11 -> 3.97, 6.57 -> 6.27; the same bits).
+template <uint32_t LEAF>
 __device__ bool build_path(const MSegSpec &s, const PathPts &P, uint64_t path)
 {
     const uint32_t N = s.n_segments;
     Draws g(s.seed, (uint32_t)path, (uint32_t)(path >> 32), s.experiment ^ 0x4D534547u);
     const double ds = s.ds, inv_ds = 1.0 / ds;
-    // N - 2 = leaf << depth, leaf 4 or 6 (the host validated N - 2 as resolvable)
-    const uint32_t M = N - 2;
-    uint32_t leaf = M, depth = 0;
-    while (leaf > 6) {
-        leaf >>= 1;
-        ++depth;
-    }
+    constexpr uint32_t leaf = LEAF;
+    const uint32_t depth = 31u - (uint32_t)__clz((int)((N - 2) / leaf));
     const double inv_leaf = 2.0 / (double)leaf;
     for (uint32_t t = 0; t < (1u << depth); ++t) {
         const uint32_t l = 1 + t * leaf;
@@ -295,10 +295,9 @@ __device__ bool build_path(const MSegSpec &s, const PathPts &P, uint64_t path)
             const double inv_h = __hiloint2double(__double2hiint(inv_leaf) - (k << 20), __double2loint(inv_leaf));
             if (!place_centre(P, (int)m, inv_h, l, l + m, ds, inv_ds, g)) return false;
         }
-        const uint32_t c = l + leaf / 2, r = l + leaf;
-        if (leaf == 4 ? !(resolve_two(P, l, c, ds, g) && resolve_two(P, c, r, ds, g))
-                      : !(resolve_three(P, l, c, ds, g) && resolve_three(P, c, r, ds, g)))
-            return false;
+#pragma unroll 1
+        for (uint32_t half = l; half < l + leaf; half += leaf / 2)
+            if (LEAF == 4 ? !resolve_two(P, half, half + 2, ds, g) : !resolve_three(P, half, half + 3, ds, g)) return false;
     }
     return true;
 }
@@ -392,7 +391,7 @@ constexpr int kMsegThreads = 128;
 
 // FORM 0: the plain weigher; 1: the compensated fixed-point table (a path through a steep bin, or with
 // a NaN curvature, again through the linear one); 2: the linear table. Writes one sample per path.
-template <int FORM>
+template <int FORM, uint32_t LEAF>
 __global__ void __launch_bounds__(kMsegThreads, 6)
 msegment_kernel(MSegSpec s, MSegWeigh wg, CompConsts kc, float *__restrict__ scratch, ChainOut *__restrict__ out)
 {
@@ -406,7 +405,7 @@ msegment_kernel(MSegSpec s, MSegWeigh wg, CompConsts kc, float *__restrict__ scr
     const dev::LutMeta m{wg.meta.min_k, wg.meta.max_k, wg.meta.step, wg.meta.bins};
     for (uint64_t i = tid; i < s.n_paths; i += threads) {
         double w = 0.0;
-        bool ok = build_path(s, P, s.path0 + i);
+        bool ok = build_path<LEAF>(s, P, s.path0 + i);
         if (ok) {
             if constexpr (FORM == 0) {
                 ok = weigh_plain(P, N, wg.inv_ds, wg.lut, m, wg.absorption_factor, w);
@@ -426,10 +425,20 @@ msegment_kernel(MSegSpec s, MSegWeigh wg, CompConsts kc, float *__restrict__ scr
     }
 }
 
+template <int FORM>
+void launch_form(const MSegSpec &s, const MSegWeigh &wg, const CompConsts &kc, unsigned blocks, float *scratch, ChainOut *out,
+                 cudaStream_t st)
+{
+    uint32_t leaf = s.n_segments - 2;
+    while (leaf > 6) leaf >>= 1;
+    if (leaf == 4) msegment_kernel<FORM, 4><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
+    else msegment_kernel<FORM, 6><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
+}
+
 }  // namespace
 
-// Threads of a launch: 768 per SM (N = 66, 2^21 paths: 4.03 ms at 768, 4.07 at 1024, 4.35 at 512; the step is
-// bound by issue, 40 k instructions per path, and instruction fetch), fewer while their columns
+// Threads of a launch: 768 per SM (N = 66, 2^21 paths, before a kernel had one kind of leaf: 4.03 ms at 768, 4.07 at
+// 1024, 4.35 at 512; the step is bound by issue, 40 k instructions per path, and instruction fetch), fewer while their columns
 // exceed 384 MB (the context keeps them), and no more than there are paths.
 uint32_t msegment_threads(uint32_t n_segments, uint64_t n_paths)
 {
@@ -459,9 +468,9 @@ cudaError_t launch_msegment(uint32_t n_segments, float ds, const float p0[3], co
     s.n_paths = n_paths;
     const CompConsts kc = make_consts(wg.inv_ds, wg.meta, n_segments, wg.lf);
     const unsigned blocks = threads / kMsegThreads;
-    if (wg.plain) msegment_kernel<0><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
-    else if (wg.exact || wg.lf.inv_scale == 0.0) msegment_kernel<2><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
-    else msegment_kernel<1><<<blocks, kMsegThreads, 0, st>>>(s, wg, kc, scratch, out);
+    if (wg.plain) launch_form<0>(s, wg, kc, blocks, scratch, out, st);
+    else if (wg.exact || wg.lf.inv_scale == 0.0) launch_form<2>(s, wg, kc, blocks, scratch, out, st);
+    else launch_form<1>(s, wg, kc, blocks, scratch, out, st);
     return cudaGetLastError();
 }
 
