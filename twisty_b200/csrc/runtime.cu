@@ -215,10 +215,17 @@ struct MSegBufs : KeptBufs<4> {
     static constexpr size_t kKeep = 512ull << 20;
     DevBuf &points = bufs[0], &samples = bufs[1], &red = bufs[2], &slices = bufs[3];
 };
+// At a call's end, whichever way it ends: waits for its work, which an error leaves behind with the caller's arrays and
+// these buffers in use (freeing its own buffers used to wait), then gives back what is above the limit.
 template <class Bufs>
-struct Trim {
+struct CallEnd {
     Bufs &b;
-    ~Trim() { b.trim(Bufs::kKeep); }
+    cudaStream_t st;
+    ~CallEnd()
+    {
+        cudaStreamSynchronize(st);
+        b.trim(Bufs::kKeep);
+    }
 };
 
 // Outputs of the batched adjoint (twisty_adjoint_batch); every pointer nullable but grad.
@@ -1258,7 +1265,7 @@ twisty_status twisty_run_msegment(twisty_ctx *ctx, const twisty_bc *bc, twisty_r
         const uint64_t per_launch = std::min(std::min(chunk, kLaunch), std::max<uint64_t>(total, 1));
         const uint32_t threads = msegment_threads(N, per_launch);
         MSegBufs &B = ctx->mseg;
-        const Trim<MSegBufs> trim{B};
+        const CallEnd<MSegBufs> end{B, st};
         ck(B.points.ensure(per_path * threads), "alloc points");
         ck(B.samples.ensure(sizeof(ChainOut) * per_launch), "alloc samples");
         ck(B.red.ensure(sizeof(ReduceOut) * std::max<size_t>(1, slices.size())), "alloc result");
@@ -1336,7 +1343,7 @@ twisty_status twisty_weight_paths(twisty_ctx *ctx, const twisty_bc *bc, const fl
         if (n_paths == 0) return;
         cudaStream_t st = ctx->stream;
         DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dv = ctx->call.c, &db = ctx->call.d;
-        const Trim<CallBufs> trim{ctx->call};
+        const CallEnd<CallBufs> end{ctx->call, st};
         const size_t np = 3 * (size_t)(N + 1) * n_paths;
         ck(dpos.ensure(sizeof(float) * np), "alloc paths");
         ck(dw.ensure(sizeof(double) * n_paths), "alloc weights");
@@ -2062,7 +2069,7 @@ twisty_status twisty_export_paths(twisty_ctx *ctx, const twisty_bc *bc, const ch
             const size_t npaths = (size_t)E * c.steps;
             cudaStream_t st = ctx->stream;
             DevBuf &dpos = ctx->call.a, &dw = ctx->call.b, &dout = ctx->call.c;
-            const Trim<CallBufs> trim{ctx->call};
+            const CallEnd<CallBufs> end{ctx->call, st};
             struct Drain {   // before the buffers can go or serve another call
                 cudaStream_t s;
                 ~Drain()
@@ -2166,7 +2173,7 @@ twisty_status twisty_adjoint(twisty_ctx *ctx, const twisty_bc *bc, const twisty_
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
         DevBuf &dtab = ctx->call.a, &dg = ctx->call.b, &dout = ctx->call.c, &djob = ctx->call.d;
-        const Trim<CallBufs> trim{ctx->call};
+        const CallEnd<CallBufs> end{ctx->call, st};
         ck(dtab.ensure(sizeof(float4) * bins), "alloc");
         ck(dg.ensure(sizeof(double) * 6 * std::max<uint32_t>(c.n_chains, 1)), "alloc");
         ck(dout.ensure(sizeof(double) * 6), "alloc");
@@ -2209,7 +2216,7 @@ twisty_status twisty_weight_histogram(twisty_ctx *ctx, const twisty_bc *bc, doub
         const ChainSpec &c = ctx->spec;
         cudaStream_t st = ctx->stream;
         DevBuf &dw = ctx->call.a, &dout = ctx->call.b, &dcnt = ctx->call.c;
-        const Trim<CallBufs> trim{ctx->call};
+        const CallEnd<CallBufs> end{ctx->call, st};
         ck(dcnt.ensure(sizeof(unsigned long long) * n_buckets), "alloc histogram");
         ck(cudaMemsetAsync(dcnt.p, 0, sizeof(unsigned long long) * n_buckets, st), "memset");
         if (c.n_chains) {
