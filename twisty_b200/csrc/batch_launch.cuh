@@ -72,6 +72,13 @@ bool batch_shapes_e_occ(const BatchShape &s, size_t smem, int &occ);
 
 namespace {
 
+// Whether a shape sums four weighted paths together (chain_body). In the batched kernels the experiment's constants take
+// registers that the single-run kernels read from the constant bank, and the sums in flight take more: up to 16 lanes
+// they spill. One sum per path there, and in 32 x 32: 256 experiments of 2^14 paths (2048 bins), N = 40 -4 %, 64 -4 %,
+// 180 -7 %, 350 -9 %, 400 -15 %, 1024 -8 %, 128 and 256 even; 24 of them, whose chains have few warps to hide a spill,
+// N = 180 -17 %, 350 -27 %, 400 -38 %. The other shapes of 32 lanes gain from the grouped sums: 512 -7 %, 640 -4 %, 896 -9 %.
+__host__ __device__ constexpr bool batch_grouped(int G, int SPL) { return G == 32 && SPL < 32; }
+
 template <int G, int SPL, bool EXACT, bool LUT_SMEM, bool CLAMP, bool STEEP, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restrict__ exps,
                                                         const uint2 *__restrict__ items, uint32_t n_items,
@@ -110,7 +117,7 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchExp *__restri
         // the exact blend keeps PAIRS at 32 lanes here: after an item's split few warps are left to hide its loads
         // (16 experiments of 2^14 paths, N = 512: 10.6 ms against 14.5 in XYZ, 1024: 35.6 against 51.7; 256 of
         // them: 888 against 882, 1841 against 2013)
-        chain_body<G, SPL, EXACT, CLAMP, false, kModeForward, false, STEEP, !LUT_SMEM, false>(
+        chain_body<G, SPL, EXACT, CLAMP, false, kModeForward, false, STEEP, !LUT_SMEM, false, batch_grouped(G, SPL)>(
               e.spec, e.kc, e.init_seg, tab, st, Lanes<G>::base_of(lane), j, chain, chain < e.spec.n_chains,
               out + e.out_offset, ma);
         __syncthreads();

@@ -712,7 +712,7 @@ __device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j
 // STEEP: the fixed-point table has steep bins (NaN slopes); paths crossing one are re-weighed
 // through ma.lin. Without it a NaN slope cannot occur and a NaN total means a NaN curvature.
 template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INCR = false, bool STEEP = false,
-          bool TAB_GLOBAL = false, bool ORDERED = EXACT && MODE != kModeAdjoint>
+          bool TAB_GLOBAL = false, bool ORDERED = EXACT && MODE != kModeAdjoint, bool GROUPED = true>
 __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConsts &kc,
                                              const float *__restrict__ init_seg, const float2 *s_tab, Planes st,
                                              uint32_t qb, uint32_t j, uint32_t chain, bool real_chain,
@@ -828,12 +828,13 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
         }
         kahan_add(lse_s, lse_c, term);
     };
-    // Forward passes of groups of 4 lanes and more sum the lanes' shares of four path totals together:
+    // Forward passes of groups of 4 lanes and more (GROUPED: in the batched kernels only some shapes, batch_grouped) sum the
+    // lanes' shares of four path totals together:
     // exchanges after every second and fourth weighted step leave one step's shares in each lane (step
     // j mod 4), the other levels add as a butterfly does, and each lane runs the log-sum-exp of
     // its own steps: 5 shuffles for four paths of 16 lanes instead of 16, and one log-sum-exp
     // update for four paths instead of one for each in every lane.
-    constexpr bool BATCH = FIX && MODE == kModeForward && !INCR && G >= 4;
+    constexpr bool BATCH = FIX && MODE == kModeForward && !INCR && G >= 4 && GROUPED;
     constexpr int LS = Lanes<G>::STRIDE;
     uint32_t even = 0, flags = 0;       // the even step's share; steps 0..3 met (bits 0..3) and weighed (bits 4..7)
     unsigned long long pair01 = 0;
