@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <filesystem>
 #include <fstream>
 #include <algorithm>
@@ -215,15 +216,17 @@ struct MSegBufs : KeptBufs<4> {
     static constexpr size_t kKeep = 512ull << 20;
     DevBuf &points = bufs[0], &samples = bufs[1], &red = bufs[2], &slices = bufs[3];
 };
-// At a call's end, whichever way it ends: waits for its work, which an error leaves behind with the caller's arrays and
-// these buffers in use (freeing its own buffers used to wait), then gives back what is above the limit.
+// At a call's end: an error leaves work behind with the caller's arrays and these buffers in use, which is waited for
+// (freeing its own buffers used to wait; a call that ends well has waited itself). Then what is above the limit is given
+// back.
 template <class Bufs>
 struct CallEnd {
     Bufs &b;
     cudaStream_t st;
+    int before = std::uncaught_exceptions();
     ~CallEnd()
     {
-        cudaStreamSynchronize(st);
+        if (std::uncaught_exceptions() > before) cudaStreamSynchronize(st);
         b.trim(Bufs::kKeep);
     }
 };
