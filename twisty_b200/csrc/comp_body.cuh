@@ -284,6 +284,8 @@ __device__ __forceinline__ F2 bins_of(F2 qq, const CompConsts &k, int32_t &L0, i
 // shapes below 12 segments per lane -4 to -7 % (N = 18, 30, 34). ORDERED: a recompute that
 // walks its segments in order (the exact blend of single runs) would keep the later halves of PAIRS in registers, and
 // spills: N = 544 351 -> 324 us over 2^19 paths in XYZ, 768 371 -> 306, 1024 439 -> 330, receiver-shifted 669 -> 426.
+// The incremental form, which reads single tangents more often than it recomputes, takes XYZ too (2^29 path-segments,
+// a recompute every 64 steps: N = 512 -11 %, 530 -13 %, 768 -10 %, 1024 -10 %).
 enum { kPairs = 0, kXyz = 1, kPlanes = 2 };
 __host__ __device__ constexpr int comp_layout(int G, int SPL, bool ordered = false)
 {
@@ -712,7 +714,7 @@ __device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j
 // STEEP: the fixed-point table has steep bins (NaN slopes); paths crossing one are re-weighed
 // through ma.lin. Without it a NaN slope cannot occur and a NaN total means a NaN curvature.
 template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INCR = false, bool STEEP = false,
-          bool TAB_GLOBAL = false, bool ORDERED = EXACT && MODE != kModeAdjoint, bool GROUPED = true>
+          bool TAB_GLOBAL = false, bool ORDERED = (EXACT && MODE != kModeAdjoint) || INCR, bool GROUPED = true>
 __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConsts &kc,
                                              const float *__restrict__ init_seg, const float2 *s_tab, Planes st,
                                              uint32_t qb, uint32_t j, uint32_t chain, bool real_chain,
