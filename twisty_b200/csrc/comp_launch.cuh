@@ -122,7 +122,8 @@ cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const 
 // Instantiated variants: forward (fixed/exact x clamp/no clamp, plus an exact+clamp+shift
 // variant for receiver-shifted evaluation), export (fixed/exact with clamp), adjoint (fixed without clamp,
 // exact with);
-// the fixed-point forward and incremental variants again with the steep-bin fallback, the fixed-point export with it only;
+// the fixed-point forward and incremental variants again with the steep-bin fallback, the fixed-point export
+// without it up to 17 segments per lane only;
 // with the table in global memory (lut_global), the forward variants only.
 template <int G, int SPL>
 cudaError_t launch_g(int mode, bool exact, bool clamp, bool shift, bool steep, const ChainSpec &c,
@@ -148,9 +149,12 @@ cudaError_t launch_g(int mode, bool exact, bool clamp, bool shift, bool steep, c
         return exact ? TWISTY_L(true, true, false, kModeAdjoint) : TWISTY_L(false, false, false, kModeAdjoint);
     if (mode == kModeExport) {
         if (exact) return TWISTY_L(true, true, false, kModeExport);
-        // the steep-bin form whatever the table: its fallback's call keeps the recompute's loads from being hoisted until
-        // they spill (400 bytes of stack at 32 x 24 without it; weights of 2^28 path-segments, the whole call: N = 384
-        // 531 -> 394 us, 700 755 -> 464, 896 518 -> 381; up to N = 36 even)
+        // mostly the steep-bin form whatever the table: its fallback's call keeps the recompute's loads from being hoisted
+        // until they spill (400 bytes of stack at 32 x 24 without it; weights of 2^28 path-segments, the whole call: N = 128
+        // -18 %, 384 531 -> 394 us, 700 755 -> 464, 896 518 -> 381; up to N = 36 even). Exports of points run few warps,
+        // for which hoisted loads are as well below 20 segments per lane (2000 paths, N = 128: 2 % faster without the call)
+        if constexpr (SPL < 20)
+            if (!steep && ma.exp_pos) return TWISTY_L(false, true, false, kModeExport);
         return TWISTY_S(true, kModeExport, false);
     }
     if (shift) return TWISTY_L(true, true, true, kModeForward);
