@@ -371,7 +371,6 @@ cudaError_t launch_comp_adjoint(const ChainSpec &c, const CompTuning &tuning, co
     ma.ref_log10 = ref_log10;
     ma.grad = grad_chains;
     CompTuning t = tuning;
-    t.warps_per_block = std::min(t.warps_per_block, kAdjointThreads / 32);
     t.exact_blend = comp_adjoint_fixed(lf, c.inv_ds, m) ? 0 : 1;
     cudaError_t e = launch_mode(kModeAdjoint, c, t, init_seg, fixtab, lintab, m, nullptr, nullptr, ma,
                                 t.exact_blend ? LogFixed{0.0, 0.0, 0, 0} : lf, st);

@@ -94,7 +94,7 @@ template <int G, int SPL, bool EXACT, int MODE>
 constexpr bool wide_registers() { return G == 32 && SPL >= 28 && MODE == kModeForward && !EXACT; }
 
 template <int G, int SPL, bool EXACT, bool CLAMP, bool SHIFT, int MODE, bool INCR = false, bool STEEP = false,
-          bool LUTG = false, int MAXT = MODE == kModeAdjoint ? kAdjointThreads : comp_max_threads(G, SPL)>
+          bool LUTG = false, int MAXT = comp_max_threads(G, SPL)>
 cudaError_t launch_t(const ChainSpec &c, const CompConsts &kc, int warps, const float *init_seg, const float2 *tab,
                      ChainOut *out, double2 *partials, const ModeArgs &ma, size_t smem, uint32_t blocks, cudaStream_t st)
 {
