@@ -194,29 +194,6 @@ __device__ __forceinline__ void cw_add(CombinedWeight &c, double v)
     c.n++;
 }
 
-__device__ __forceinline__ CombinedWeight cw_combine(CombinedWeight a, CombinedWeight b)
-{
-    if (a.n > 0 && b.n == 0) return a;
-    if (b.n > 0 && a.n == 0) return b;
-    if (b.max_log10 > a.max_log10) {
-        const CombinedWeight t = b;
-        b = a;
-        a = t;
-    }
-    CombinedWeight r;
-    cw_reset(r);
-    r.max_log10 = a.max_log10;
-    r.n = a.n + b.n;
-    r.offset = a.offset;
-    if (a.max_log10 == b.max_log10) {
-        r.total = a.total + b.total;
-        return r;
-    }
-    const double delta = a.offset - b.offset;
-    r.total = a.total + pow(10.0, log10(b.total) + delta);
-    return r;
-}
-
 // log10 of ExtractFinalValue (Twisty/CombinedWeightUtils.h:160-174).
 __device__ __forceinline__ double cw_log10(const CombinedWeight &c)
 {
