@@ -158,8 +158,12 @@ typedef struct twisty_result {
     uint32_t num_chains;
     uint32_t steps_per_chain;
     double total_ms;             /* totalExperimentMs */
-    double setup_ms;             /* setupExperimentMs: table, normaliser, initial curve */
-    double perturb_ms;           /* perturbExperimentMs: the chain kernel, device time */
+    double setup_ms;             /* setupExperimentMs: table, normaliser, initial curve; of twisty_run
+                                    and twisty_export_paths without the uploads' arrival, which the
+                                    pass's stream waits for */
+    double perturb_ms;           /* perturbExperimentMs: the chain kernel, device time; of a compensated
+                                    twisty_export_paths with the export's replay running beside it,
+                                    so up to the replay's time longer than twisty_run's */
     double weighting_ms;         /* weightingExperimentMs: final reduction */
     /* Compensated form only (no reference counterpart): which table the pass weighed with,
        TWISTY_TABLE_FIXED_NARROW / _FIXED_WIDE (fixed-point log tables, 32- or 64-bit path

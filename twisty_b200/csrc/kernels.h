@@ -88,9 +88,9 @@ struct TableInfo {
 cudaError_t launch_single_tables(uint32_t bins, float step, uint32_t n_segments, int finalize, double *lut64, float *lut32, float2 *lin,
                                  float2 *fix, TableInfo *info, cudaStream_t st);
 // Batches of n tables of `bins` entries, table x at offset x*bins: build (specs in device
-// memory, finalize (minmax + 3x), and the compensated-form tables (struct
-// LogFixed below; steps[x] = bin width, nsegs[x] = N of the paths the fixed point is scaled
-// for, ok[x] = 1 when the fixed-point form is usable).
+// memory), finalize (minmax + 3x: min, max and replacement), and the compensated-form tables
+// (struct LogFixed below; steps[x] = bin width, nsegs[x] = N of the paths the fixed point is
+// scaled for, ok[x] = 1 when the fixed-point form is usable).
 cudaError_t launch_lut_build_batch(const LutBuildSpec *d_specs, uint32_t n, uint32_t bins, double *out64,
                                    cudaStream_t st);
 cudaError_t launch_lut_finalize_batch(uint32_t n, uint32_t bins, double *lut64, float *out32, double *minmax,
