@@ -704,11 +704,11 @@ __device__ __forceinline__ void stage_table(float4 *smem4, const float2 *__restr
 // Exact-blend weight of the group's current path through the linear table, for paths of a
 // fixed-point table that cross a steep bin: in segment order, as every exact blend sums. Not
 // inlined: it runs rarely, and inlined its registers would count against the hot loop's.
-template <int G, int SPL, bool CLAMP>
+template <int G, int SPL, bool CLAMP, bool ORDERED>
 __device__ __noinline__ double steep_fallback(Planes st, uint32_t qb, uint32_t j, uint32_t N,
                                               const float2 *__restrict__ lin, CompConsts kc)
 {
-    const SmemLoad<G, SPL> load{st, qb, j, 0, nullptr, 0.f, 0.f};
+    const SmemLoad<G, SPL, false, ORDERED> load{st, qb, j, 0, nullptr, 0.f, 0.f};   // the chain's own layout
     uint32_t unused = 0;
     return path_log10<G, SPL, true, CLAMP, true, false>(j, N, lin, kc, load, ShflNext<G>{}, [](uint32_t, int32_t) {}, unused);
 }
@@ -1245,7 +1245,7 @@ __device__ __forceinline__ double chain_body(const ChainSpec &c, const CompConst
                     // table; only a NaN curvature leaves a path invalid
                     if constexpr (STEEP) {
                         if (__any_sync(FULL, bad)) {
-                            const double wx = steep_fallback<G, SPL, CLAMP>(st, qb, j, N, ma.lin, kc);
+                            const double wx = steep_fallback<G, SPL, CLAMP, ORDERED>(st, qb, j, N, ma.lin, kc);
                             if (bad && !isnan(wx)) {
                                 bad = false;
                                 // the total in shares of at most 32 bits, one per lane
