@@ -688,17 +688,12 @@ __device__ __forceinline__ void fill_lengths(float *s_len, const float *__restri
     }
 }
 
-// Stage a table of `bins` float2 entries into shared memory: two entries a load where the table starts on 16 bytes, one
-// where it does not (in a batch of tables of an odd number of bins every second one, and a caller's own table).
+// Stage a table of `bins` float2 entries into shared memory (float4 vector loads: the table starts on 16 bytes, which
+// table_pitch and the callers of single tables see to; a look at the address here cost 8 x 24 6 %).
 __device__ __forceinline__ void stage_table(float4 *smem4, const float2 *__restrict__ tab_g, int bins)
 {
-    float2 *const smem2 = reinterpret_cast<float2 *>(smem4);
-    if (reinterpret_cast<uintptr_t>(tab_g) & 15u) {
-        for (int i = threadIdx.x; i < bins; i += blockDim.x) smem2[i] = tab_g[i];
-        return;
-    }
     for (int i = threadIdx.x; i < bins / 2; i += blockDim.x) smem4[i] = reinterpret_cast<const float4 *>(tab_g)[i];
-    if ((bins & 1) && threadIdx.x == 0) smem2[bins - 1] = tab_g[bins - 1];
+    if ((bins & 1) && threadIdx.x == 0) reinterpret_cast<float2 *>(smem4)[bins - 1] = tab_g[bins - 1];
 }
 
 // Exact-blend weight of the group's current path through the linear table, for paths of a

@@ -89,13 +89,16 @@ cudaError_t launch_single_tables(uint32_t bins, float step, uint32_t n_segments,
                                  float2 *fix, TableInfo *info, cudaStream_t st);
 // Batches of n tables of `bins` entries, table x at offset x*bins: build (specs in device
 // memory), finalize (minmax + 3x: min, max and replacement), and the compensated-form tables
-// (struct LogFixed below; steps[x] = bin width, nsegs[x] = N of the paths the fixed point is
+// (struct LogFixed below; fix and lin of table x at x*table_pitch(bins); steps[x] = bin width, nsegs[x] = N of the paths the fixed point is
 // scaled for, ok[x] = 1 when the fixed-point form is usable).
 cudaError_t launch_lut_build_batch(const LutBuildSpec *d_specs, uint32_t n, uint32_t bins, double *out64,
                                    cudaStream_t st);
 cudaError_t launch_lut_finalize_batch(uint32_t n, uint32_t bins, double *lut64, float *out32, double *minmax,
                                       cudaStream_t st);
 struct LogFixed;
+// Entries from one fix or lin table of a batch to the next: an even number, so that every table starts on the 16 bytes
+// that the kernels stage it by.
+__host__ __device__ constexpr uint32_t table_pitch(uint32_t bins) { return (bins + 1u) & ~1u; }
 cudaError_t launch_comp_tables_batch(uint32_t n, uint32_t bins, const float *lut32, const float *steps,
                                      const uint32_t *nsegs, float2 *fix, float2 *lin, LogFixed *lf, int *ok,
                                      cudaStream_t st);

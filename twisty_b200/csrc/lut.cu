@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(1024) comp_tables_kernel(uint32_t bins, const 
     __shared__ int s_bad[32], s_steep[32];
     const uint32_t x = blockIdx.x;
     const float *L = lut32 + (size_t)x * bins;
-    fix += (size_t)x * bins;
-    lin += (size_t)x * bins;
+    fix += (size_t)x * table_pitch(bins);
+    lin += (size_t)x * table_pitch(bins);
     const double st = (double)steps[x];
     double lo = DBL_MAX, hi = -DBL_MAX, err = 0.0;
     int bad = 0, steep = 0;

@@ -106,7 +106,9 @@ extern "C" twisty_status twisty_run_noalloc(const twisty_noalloc_args *a, void *
     CompTuning t = comp_default_tuning(N, false, a->paths, a->burn_in);
     t.exact_blend = 1;  // the table is the linear (L_i, L_{i+1} - L_i) form
     if (!comp_tuning_supported(t, N, c.k_eff)) return bad("no compensated kernel shape for this N");
-    t.lut_global = comp_table_through_l1(t, a->bins, true) ? 1 : 0;
+    // a table that does not start on the 16 bytes it is staged by is gathered through L1 too
+    const bool unaligned = (reinterpret_cast<uintptr_t>(a->table) & 15u) != 0;
+    t.lut_global = unaligned || comp_table_through_l1(t, a->bins, true) ? 1 : 0;
     if (!comp_fit_smem(t, a->bins, true)) return bad("the chain state of this N does not fit in shared memory");
     const LutMetaF m{a->min_curvature, a->max_curvature, a->curvature_step, (int32_t)a->bins};
     cudaStream_t st = (cudaStream_t)stream;

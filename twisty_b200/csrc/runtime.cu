@@ -1614,8 +1614,8 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
     ck(B.specs.ensure(sizeof(LutBuildSpec) * n), "alloc batch");
     ck(B.lut64.ensure(sizeof(double) * (size_t)bins * n), "alloc batch tables");
     ck(B.lut32.ensure(sizeof(float) * (size_t)bins * n), "alloc batch tables");
-    ck(B.fix.ensure(sizeof(float2) * (size_t)bins * n), "alloc batch tables");
-    ck(B.lin.ensure(sizeof(float2) * (size_t)bins * n), "alloc batch tables");
+    ck(B.fix.ensure(sizeof(float2) * (size_t)table_pitch(bins) * n), "alloc batch tables");
+    ck(B.lin.ensure(sizeof(float2) * (size_t)table_pitch(bins) * n), "alloc batch tables");
     ck(B.steps.ensure(sizeof(float) * n), "alloc batch");
     ck(B.nsegs.ensure(sizeof(uint32_t) * n), "alloc batch");
     ck(B.lf.ensure(sizeof(LogFixed) * n), "alloc batch");
@@ -1712,8 +1712,8 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         b.spec = h.spec;
         b.meta = h.meta;
         b.lf = exact ? LogFixed{0.0, 0.0, 0, 0} : lf[e];
-        b.tab = (exact ? B.lin.as<float2>() : B.fix.as<float2>()) + (size_t)e * bins;
-        b.lin = B.lin.as<float2>() + (size_t)e * bins;
+        b.tab = (exact ? B.lin.as<float2>() : B.fix.as<float2>()) + (size_t)e * table_pitch(bins);
+        b.lin = B.lin.as<float2>() + (size_t)e * table_pitch(bins);
         b.init_seg = B.init_seg.as<float>() + h.seg_off;
         b.out_offset = h.chain_off;
         BatchShape sh{h.t.group, h.t.spl, h.t.warps_per_block, exact ? 1 : 0, 1,
@@ -1921,7 +1921,7 @@ void run_batch(twisty_ctx *ctx, const twisty_experiment *ex, uint32_t n, uint32_
         bx[e] = bh[e];
         const bool fixed = fixed_of(e);
         bx[e].lf = fixed ? lf[e] : LogFixed{0.0, 0.0, 0, 0};
-        bx[e].tab = (fixed ? B.fix.as<float2>() : B.lin.as<float2>()) + (size_t)e * bins;
+        bx[e].tab = (fixed ? B.fix.as<float2>() : B.lin.as<float2>()) + (size_t)e * table_pitch(bins);
         const double log10_abs = std::log10(h.spec.absorption_factor);
         const bool ok = red[e].valid > 0 && std::isfinite(red[e].log10_sum);
         ax[e] = BatchAdjHost{jobs[job_of[e]].out,
